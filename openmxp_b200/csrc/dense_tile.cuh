@@ -20,24 +20,19 @@ struct SmemGemm {
     float As[GBK][GBM];
     float Bs[GBK][GBN + 4];
 };
+struct __align__(16) PanelRows {  // getrf64: four pivot rows at a time, for every lane
+    float r[3][4][4][16];         // [warp][four-pivot step][row][column]
+};
 struct __align__(16) SmemTri {
-    union {
-        float t[kNB][kNB + 4];   // t[col][row] of a 64 x 64 block (16-byte rows)
-        float ub[kNB][kNB + 1];  // staging of 64 U-strip columns, ub[col][row] (t is dead by then)
-    };
+    float t[kNB][kNB + 4];   // t[col][row] of a 64 x 64 block (16-byte rows)
     float us[kNB][kNB];      // us[k][c] = U(k, k + 1 + c): row k of U right of the diagonal, zero past the block
     float ls[kNB][kNB];      // ls[k][c] = L(k + 1 + c, k): column k of L below the diagonal, zero past the block
     float dinv[kNB];
-    int ready[32];           // 64 x 64 factor: multipliers of pivot k published (getrf64)
-};
-struct __align__(16) SmemG64 {  // one 64 x 64 x 64 product staged whole
-    float As[kNB][kNB];       // As[k][row]
-    float Bs[kNB][kNB + 4];   // Bs[k][col]
+    PanelRows rows;          // getrf64: pivot rows in exchange
 };
 union __align__(16) Smem {
     SmemGemm g;
     SmemTri t;
-    SmemG64 g64;
 };
 
 // A 64 x 64 block (rows r < nb, columns c < nb; zero elsewhere) from global
@@ -360,242 +355,543 @@ __device__ void gemm_tile_v(SmemGV &sv, int m, int n, int kb, int ke, float alph
     __syncthreads();  // shared memory is reused by the caller's next item
 }
 
-// C[0:m, 0:n] += alpha * A(:, 0:k) B(0:k, :) for m, n <= 64 (one 64 x 64 tile,
-// 4 x 4 outputs per thread): the look-ahead update of the next diagonal block.
-// C is read together with the first operand slice (one L2 round trip for
-// all three).  to_smem: the result goes to sm.t.t[col][row] instead of C, for
-// getrf64(..., in_smem = true) to factor without a global round trip (the
-// caller then owns writing it back; getrf64 does).
-__device__ void gemm_tile64(Smem &sm, int m, int n, int k, float alpha, const float *__restrict__ A, int64_t lda,
-                            const float *__restrict__ B, int64_t ldb, float *C, int64_t ldc, bool to_smem = false) {
+// ---- 64 x 64 SIMT GEMM tiles staged by cp.async ------------------------------
+// The same sums as gemm_tile / gemm_tile_v (one fmaf chain over ascending k,
+// times alpha, plus C), in tiles a quarter the size: the trailing updates of a
+// diagonal block (rank 64, at most a few dozen 128 x 128 tiles for most
+// steps) and the doubling levels of its inverses then spread over all CTAs
+// instead of leaving most idle behind ~7 us tiles.  Operand slices (64 deep)
+// and the C tile arrive by 16-byte cp.async, double-buffered across slices and
+// across the CTA's tiles, so a tile's loads run under the previous one's
+// products (4 x 4 outputs per thread, ~75 % of the FMA rate).  Alignment as
+// gemm_tile_v_ok.
+struct __align__(16) SmemT64Buf {
+    float As[kNB][kNB];      // As[k][row]
+    float Bs[kNB][kNB + 4];  // Bs[col][k]
+    float Cs[kNB][kNB + 4];  // Cs[col][row]
+};
+struct __align__(16) SmemT64 {
+    SmemT64Buf buf[2];
+};
+
+// One tile: C[m0:m0+64, n0:n0+64] (clipped to m x n) over k in [kb, ke).
+struct Tile64 {
+    const float *A, *B;
+    float *C;
+    int64_t lda, ldb, ldc;
+    int m, n, m0, n0, kb, ke;
+    float alpha;
+};
+
+__device__ __forceinline__ void t64_load_slice(SmemT64Buf &b, const Tile64 &w, int k0, bool with_c) {
     const int t = threadIdx.x;
-    const int tx = t % 16, ty = t / 16;
-    float acc[4][4], cv[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int idx = t + kCT * q, i = idx >> 4, g = (idx & 15) * 4;
+        {  // A: k = i, rows g..g+3
+            const int gk = k0 + i, gr = w.m0 + g;
+            const int by = gk < w.ke ? grp_bytes(gr, w.m) : 0;
+            cp_async16(&b.As[i][g], by ? w.A + (int64_t)gk * w.lda + gr : w.A, by);
+        }
+        {  // B: column i, k = g..g+3
+            const int gc = w.n0 + i, gk = k0 + g;
+            const int by = gc < w.n ? grp_bytes(gk, w.ke) : 0;
+            cp_async16(&b.Bs[i][g], by ? w.B + (int64_t)gc * w.ldb + gk : w.B, by);
+        }
+        if (with_c) {  // C: column i, rows g..g+3
+            const int gc = w.n0 + i, gr = w.m0 + g;
+            const int by = gc < w.n ? grp_bytes(gr, w.m) : 0;
+            cp_async16(&b.Cs[i][g], by ? w.C + (int64_t)gc * w.ldc + gr : w.C, by);
+        }
+    }
+}
+
+// Tiles get(first), get(first + stride), ... < count.  get(i, w) fills w; every
+// tile has at least one k.  ACC: C += ..., else C = ...
+template <bool ACC, typename Get>
+__device__ __forceinline__ void run_tiles64(SmemT64 &sm, int first, int stride, int count, Get get) {
+    if (first >= count) return;
+    const int t = threadIdx.x, tx = t % 16, ty = t / 16;
+    Tile64 w, nw;
+    get(first, w);
+    nw = w;
+    int it = first, k0 = w.kb, buf = 0;
+    __syncthreads();  // the caller's previous use of this memory is over
+    t64_load_slice(sm.buf[0], w, k0, ACC && k0 + kNB >= w.ke);
+    cp_async_commit();
+    float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            acc[i][j] = 0.0f;
-            const int gr = tx * 4 + i, gc = ty * 4 + j;
-            cv[i][j] = (gr < m && gc < n) ? __ldcg(C + (int64_t)gc * ldc + gr) : 0.0f;
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    while (true) {
+        const bool last = k0 + kNB >= w.ke;  // last slice of the tile
+        int nk = k0 + kNB;
+        bool more = true;
+        if (last) {
+            more = it + stride < count;
+            if (more) {
+                get(it + stride, nw);
+                nk = nw.kb;
+            }
         }
-    for (int k0 = 0; k0 < k; k0 += kNB) {
-        // the whole 64-deep slice of both operands in one L2 round trip
-        const int kc = min(kNB, k - k0);
-        float va[16], vb[16];
-        load_block64(va, A + (int64_t)k0 * lda, lda, m, kc);  // va: A(r, k0 + c)
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {  // vb: B(k0 + kk, c), kk fastest
-            const int idx = t + kCT * q;
-            const int kk = idx % kNB, c = idx / kNB;
-            vb[q] = (kk < kc && c < n) ? __ldcg(B + (int64_t)c * ldb + k0 + kk) : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int idx = t + kCT * q;
-            sm.g64.As[idx / kNB][idx % kNB] = va[q];
-            sm.g64.Bs[idx % kNB][idx / kNB] = vb[q];
+        if (more) {
+            t64_load_slice(sm.buf[buf ^ 1], nw, nk, ACC && nk + kNB >= nw.ke);
+            cp_async_commit();
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
         }
         __syncthreads();
-#pragma unroll 16
-        for (int kk = 0; kk < kNB; ++kk) {
-            const float4 a = *reinterpret_cast<const float4 *>(&sm.g64.As[kk][tx * 4]);
-            const float4 b = *reinterpret_cast<const float4 *>(&sm.g64.Bs[kk][ty * 4]);
-            const float av[4] = {a.x, a.y, a.z, a.w};
-            const float bv[4] = {b.x, b.y, b.z, b.w};
+        const SmemT64Buf &b = sm.buf[buf];
+        const int nk4 = (min(kNB, w.ke - k0) + 3) / 4;
+#pragma unroll 4
+        for (int k4 = 0; k4 < nk4; ++k4) {
+            float4 bq[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; ++j) bq[j] = *reinterpret_cast<const float4 *>(&b.Bs[ty * 4 + j][4 * k4]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-    }
+            for (int s = 0; s < 4; ++s) {
+                const float4 a4 = *reinterpret_cast<const float4 *>(&b.As[4 * k4 + s][tx * 4]);
+                const float av[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int gc = ty * 4 + j;
+                for (int j = 0; j < 4; ++j) {
+                    const float bv = s == 0 ? bq[j].x : s == 1 ? bq[j].y : s == 2 ? bq[j].z : bq[j].w;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int gr = tx * 4 + i;
-            acc[i][j] *= alpha;
-            if (gr < m && gc < n) acc[i][j] += cv[i][j];
-        }
-    }
-    if (to_smem) __syncthreads();  // the operand slices share memory with t
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int gc = ty * 4 + j;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int gr = tx * 4 + i;
-            if (to_smem) sm.t.t[gc][gr] = acc[i][j];
-            else if (gr < m && gc < n) C[(int64_t)gc * ldc + gr] = acc[i][j];
-        }
-    }
-    __syncthreads();
-}
-
-// ---- 64 x 64 no-pivot LU of D (nb <= 64), warps 0 and 1 ---------------------
-// sgetrf_nopiv_naive order (sgetrf_nopiv.cpp:27-61): scale by the reciprocal
-// pivot, then the rank-1 update.  Lane l of each warp keeps rows l and l + 32;
-// warp 0 holds columns 0..31, warp 1 columns 32..63.
-//  pivots 0..31: warp 0 factors its columns, each row rotated (rot_axpy's
-//    scheme: at pivot k an active row holds A(r, k ..) from index 0), the
-//    pivot row by register shuffles, the next pivot's reciprocal
-//    (rcp_rn_f32, branch-free) issued as soon as that pivot is final; it
-//    publishes each pivot's multipliers (column k of L) in shared memory and
-//    raises ready[k].  Warp 1 follows pivot by pivot: it waits for ready[k]
-//    (bounded), takes the multipliers and the pivot row's right half (row k
-//    is in its own registers, by shuffles) and updates its columns;
-//  pivots 32..63: warp 1 alone on rows 32..63 of its columns, rotated.
-// Every element receives the same fmaf updates in the same order as in the
-// one-warp form, so the factors are bit-identical; splitting the columns
-// halves the shuffles on the pivot chain (~4 issue cycles each).  Rows stop
-// rotating at their own pivot, so at the end each lane holds its rows of U;
-// the factor goes through shared memory (T = t[col][row]) to one coalesced
-// store (scattered global stores stalled it under the L2 traffic of the
-// trailing update running beside it).  Warps 2..7 wait at the barriers.
-template <int W>
-__device__ __forceinline__ void getrf64_left(float (*T)[kNB + 4], volatile int *ready, float (&a0)[32],
-                                             float (&a1)[32], float &pv, float &rp, int k0, int k1, int nb,
-                                             DevStatus *dst, int pivot_base) {
-    const int ln = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu;
-#pragma unroll 1
-    for (int k = k0; k < k1; ++k) {
-        if (ln == 0 && (!(pv != 0.0f) || !isfinite(pv))) report(dst, MXP_ZERO_PIVOT, pivot_base + k + 1, 0);
-        const bool act0 = ln > k && ln < nb, act1 = ln + 32 < nb;
-        const float l0 = act0 ? a0[0] * rp : 0.0f;
-        const float l1 = act1 ? a1[0] * rp : 0.0f;
-        if (act0) T[k][ln] = l0;
-        if (act1) T[k][ln + 32] = l1;
-        __threadfence_block();
-        __syncwarp();
-        if (ln == 0) ready[k] = 1;
-        const float u0 = __shfl_sync(full, a0[1], k);
-        if (act0) a0[0] = fmaf(-u0, l0, a0[1]);
-        if (act1) a1[0] = fmaf(-u0, l1, a1[1]);
-        if (k + 1 < 32) {  // uniform: the next pivot is final now
-            pv = __shfl_sync(full, a0[0], k + 1);
-            rp = rcp_rn_f32(pv);
-        }
-#pragma unroll
-        for (int c = 1; c < W - 1; ++c) {
-            const float u = __shfl_sync(full, a0[c + 1], k);
-            if (act0) a0[c] = fmaf(-u, l0, a0[c + 1]);
-            if (act1) a1[c] = fmaf(-u, l1, a1[c + 1]);
-        }
-        if (act0) a0[W - 1] = 0.0f;
-        if (act1) a1[W - 1] = 0.0f;
-    }
-}
-
-template <int W>
-__device__ __forceinline__ void getrf64_lower_right(float (*T)[kNB + 4], float (&b1)[32], float &pv, float &rp,
-                                                    int k0, int k1, int nb, DevStatus *dst, int pivot_base) {
-    const int ln = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu;
-#pragma unroll 1
-    for (int k = k0; k < k1; ++k) {
-        if (ln == 0 && (!(pv != 0.0f) || !isfinite(pv))) report(dst, MXP_ZERO_PIVOT, pivot_base + k + 1, 0);
-        const int src = k - 32;  // row k: b1 of lane k - 32
-        const bool act1 = ln + 32 > k && ln + 32 < nb;
-        const float l1 = act1 ? b1[0] * rp : 0.0f;
-        const float u0 = __shfl_sync(full, b1[1], src);
-        if (act1) b1[0] = fmaf(-u0, l1, b1[1]);
-        {  // the next pivot (past the last one the value is not used)
-            pv = __shfl_sync(full, b1[0], (k + 1) & 31);
-            rp = rcp_rn_f32(pv);
-        }
-        if (act1) T[k][ln + 32] = l1;
-#pragma unroll
-        for (int c = 1; c < W - 1; ++c) {
-            const float u = __shfl_sync(full, b1[c + 1], src);
-            if (act1) b1[c] = fmaf(-u, l1, b1[c + 1]);
-        }
-        if (act1) b1[W - 1] = 0.0f;
-    }
-}
-
-// in_smem: the block to factor is already in sm.t.t[col][row] (gemm_tile64's
-// to_smem output), not read from D; either way the factors are written to D.
-__device__ __noinline__ void getrf64(Smem &sm, int nb, float *D, int64_t lda, DevStatus *dst, int pivot_base,
-                                     bool in_smem = false) {
-    float(*T)[kNB + 4] = sm.t.t;  // T[c][r]: the factored block, written out at the end
-    volatile int *ready = sm.t.ready;
-    if (threadIdx.x < 32) ready[threadIdx.x] = 0;
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu;
-    if (warp == 0) {
-        float a0[32], a1[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            a0[j] = (j < nb && ln < nb) ? (in_smem ? T[j][ln] : __ldcg(D + (int64_t)j * lda + ln)) : 0.0f;
-            a1[j] = (j < nb && ln + 32 < nb) ? (in_smem ? T[j][ln + 32] : __ldcg(D + (int64_t)j * lda + ln + 32))
-                                             : 0.0f;
-        }
-        float pv = __shfl_sync(full, a0[0], 0);
-        float rp = rcp_rn_f32(pv);
-        getrf64_left<32>(T, ready, a0, a1, pv, rp, 0, min(nb, 16), nb, dst, pivot_base);
-        getrf64_left<16>(T, ready, a0, a1, pv, rp, 16, min(nb, 32), nb, dst, pivot_base);
-        // rows 0..31 of U in columns 0..31: a0[c] = U(l, l + c)
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-            if (ln < nb && ln + c < min(nb, 32)) T[ln + c][ln] = a0[c];
-    } else if (warp == 1) {
-        float b0[32], b1[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            b0[j] = (32 + j < nb && ln < nb) ? (in_smem ? T[32 + j][ln] : __ldcg(D + (int64_t)(32 + j) * lda + ln))
-                                             : 0.0f;
-            b1[j] = (32 + j < nb && ln + 32 < nb)
-                        ? (in_smem ? T[32 + j][ln + 32] : __ldcg(D + (int64_t)(32 + j) * lda + ln + 32))
-                        : 0.0f;
-        }
-        if (nb > 32) {
-#pragma unroll 1
-            for (int k = 0; k < 32; ++k) {
-                // warp 0's multipliers of pivot k (bounded wait)
-                const unsigned long long t0 = globaltimer_ns();
-                while (ready[k] == 0) {
-                    if (globaltimer_ns() - t0 > kWaitTimeoutNs) {
-                        if (ln == 0) report(dst, MXP_TIMEOUT, 40, blockIdx.x);
-                        break;
-                    }
-                }
-                __threadfence_block();
-                const bool act0 = ln > k && ln < nb, act1 = ln + 32 < nb;
-                const float l0 = act0 ? T[k][ln] : 0.0f;
-                const float l1 = act1 ? T[k][ln + 32] : 0.0f;
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {  // row k's right half: b0 of lane k
-                    const float u = __shfl_sync(full, b0[c], k);
-                    if (act0) b0[c] = fmaf(-u, l0, b0[c]);
-                    if (act1) b1[c] = fmaf(-u, l1, b1[c]);
+                    for (int i = 0; i < 4; ++i) acc[i][j] = fmaf(av[i], bv, acc[i][j]);
                 }
             }
-            // rows 0..31 of U in columns 32..63
+        }
+        if (last) {
 #pragma unroll
-            for (int c = 0; c < 32; ++c)
-                if (ln < nb && 32 + c < nb) T[32 + c][ln] = b0[c];
-            float pv = __shfl_sync(full, b1[0], 0);
-            float rp = rcp_rn_f32(pv);
-            getrf64_lower_right<32>(T, b1, pv, rp, 32, min(nb, 48), nb, dst, pivot_base);
-            getrf64_lower_right<16>(T, b1, pv, rp, 48, nb, nb, dst, pivot_base);
+            for (int j = 0; j < 4; ++j) {
+                const int gc = w.n0 + ty * 4 + j, gr = w.m0 + tx * 4;
+                float v[4];
 #pragma unroll
-            for (int c = 0; c < 32; ++c)
-                if (ln + 32 < nb && ln + 32 + c < nb) T[ln + 32 + c][ln + 32] = b1[c];
+                for (int i = 0; i < 4; ++i) v[i] = acc[i][j] * w.alpha;
+                if (ACC) {
+                    const float4 c4 = *reinterpret_cast<const float4 *>(&b.Cs[ty * 4 + j][tx * 4]);
+                    v[0] += c4.x;
+                    v[1] += c4.y;
+                    v[2] += c4.z;
+                    v[3] += c4.w;
+                }
+                if (gc < w.n) {
+                    float *dst = w.C + (int64_t)gc * w.ldc + gr;
+                    if (gr + 3 < w.m) {
+                        *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (gr + i < w.m) dst[i] = v[i];
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i][j] = 0.0f;
+            }
+            it += stride;
+        }
+        __syncthreads();  // this buffer is refilled next
+        if (!more) break;
+        if (last) w = nw;
+        k0 = nk;
+        buf ^= 1;
+    }
+}
+
+// ---- 64-wide triangular pieces, blocked by 16 columns --------------------------
+// A block lives in shared memory as X[col][row] (pitch kNB + 4, or another that is 4 mod 32: 16-byte rows,
+// conflict-free 16-byte accesses down a column of threads).  A shared-memory
+// load returns at most 128 bytes per clock to the register file, broadcast or
+// not, so a thread-per-row elimination that reads one 16-byte group per four
+// FMAs is bound by those loads (a 64 x 64 strip solve: ~9.8 k cycles).  Here only
+// 16 columns at a time are eliminated that way; the rest of the work is
+// sub_gemm16, whose 4 x 4 outputs per thread use every loaded value four
+// times.  Every element still receives one fmaf per pivot in ascending order.
+typedef float (*Block64)[kNB + 4];
+
+// C[c][r] -= sum_{k = k0 .. k0+15} A[k][r] * B[c][k] for r in [r0, r0 + nr), c in
+// [c0, c0 + nc); nr and nc multiples of 4, at most 256 4 x 4 tiles.
+template <typename BA, typename BB, typename BC>
+__device__ __forceinline__ void sub_gemm16(BA A, BB B, BC C, int k0, int r0, int nr, int c0, int nc) {
+    const int tr = nr >> 2, tc = nc >> 2;
+    const int rg = threadIdx.x % tr, cg = threadIdx.x / tr;
+    if (cg >= tc) return;
+    const int r = r0 + 4 * rg, c = c0 + 4 * cg;
+    float x[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 v = *reinterpret_cast<const float4 *>(&C[c + j][r]);
+        x[j][0] = v.x;
+        x[j][1] = v.y;
+        x[j][2] = v.z;
+        x[j][3] = v.w;
+    }
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {
+        float4 bq[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bq[j] = *reinterpret_cast<const float4 *>(&B[c + j][k0 + 4 * k4]);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const float4 a = *reinterpret_cast<const float4 *>(&A[k0 + 4 * k4 + s][r]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float bv = s == 0 ? bq[j].x : s == 1 ? bq[j].y : s == 2 ? bq[j].z : bq[j].w;
+                x[j][0] = fmaf(-bv, a.x, x[j][0]);
+                x[j][1] = fmaf(-bv, a.y, x[j][1]);
+                x[j][2] = fmaf(-bv, a.z, x[j][2]);
+                x[j][3] = fmaf(-bv, a.w, x[j][3]);
+            }
         }
     }
-    __syncthreads();
-    // the whole block in one coalesced pass
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const int idx = threadIdx.x + kCT * q;
-        const int r = idx % kNB, c = idx / kNB;
-        if (r < nb && c < nb) D[(int64_t)c * lda + r] = T[c][r];
+    for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4 *>(&C[c + j][r]) = make_float4(x[j][0], x[j][1], x[j][2], x[j][3]);
+}
+
+// Rows k0 .. k0+15 of column X[c]: x_r -= l(r, k) x_k for r > k, L the unit lower
+// part of T's diagonal block at k0.
+__device__ __forceinline__ void sub_solve_lower(Block64 T, float *col, int k0) {
+    float u[16];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 v = *reinterpret_cast<const float4 *>(col + k0 + 4 * q);
+        u[4 * q + 0] = v.x;
+        u[4 * q + 1] = v.y;
+        u[4 * q + 2] = v.z;
+        u[4 * q + 3] = v.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 15; ++k) {
+        const float uk = u[k];
+#pragma unroll
+        for (int r4 = (k + 1) / 4; r4 < 4; ++r4) {
+            const float4 l = *reinterpret_cast<const float4 *>(&T[k0 + k][k0 + 4 * r4]);
+            if (4 * r4 + 0 > k) u[4 * r4 + 0] = fmaf(-l.x, uk, u[4 * r4 + 0]);
+            if (4 * r4 + 1 > k) u[4 * r4 + 1] = fmaf(-l.y, uk, u[4 * r4 + 1]);
+            if (4 * r4 + 2 > k) u[4 * r4 + 2] = fmaf(-l.z, uk, u[4 * r4 + 2]);
+            if (4 * r4 + 3 > k) u[4 * r4 + 3] = fmaf(-l.w, uk, u[4 * r4 + 3]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4 *>(col + k0 + 4 * q) = make_float4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+}
+
+// Columns k0 .. k0+15 of row r of X: x_c = (x_c - sum_{k<c} x_k u(k, c)) / u(c, c), U the
+// upper part of T's diagonal block at k0, dinv its reciprocal diagonal.
+template <typename BX>
+__device__ __forceinline__ void sub_solve_upper(Block64 T, const float *dinv, BX X, int r, int k0) {
+    float x[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) x[c] = X[k0 + c][r];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+#pragma unroll
+        for (int k4 = 0; 4 * k4 < c; ++k4) {
+            const float4 u = *reinterpret_cast<const float4 *>(&T[k0 + c][k0 + 4 * k4]);
+            x[c] = fmaf(-u.x, x[4 * k4], x[c]);
+            if (4 * k4 + 1 < c) x[c] = fmaf(-u.y, x[4 * k4 + 1], x[c]);
+            if (4 * k4 + 2 < c) x[c] = fmaf(-u.z, x[4 * k4 + 2], x[c]);
+            if (4 * k4 + 3 < c) x[c] = fmaf(-u.w, x[4 * k4 + 3], x[c]);
+        }
+        x[c] *= dinv[k0 + c];
+    }
+#pragma unroll
+    for (int c = 0; c < 16; ++c) X[k0 + c][r] = x[c];
+}
+
+// X (nr rows x 64, nr <= 64 and a multiple of 4, in shared memory) <- X U^{-1}, and X (64 x nc
+// columns, likewise) <- L^{-1} X, with the triangles of T.  All threads of the CTA.
+template <typename BX>
+__device__ __forceinline__ void block_solve_upper(Block64 T, const float *dinv, BX X, int nr) {
+#pragma unroll 1
+    for (int k0 = 0; k0 < kNB; k0 += 16) {
+        if (threadIdx.x < nr) sub_solve_upper(T, dinv, X, threadIdx.x, k0);
+        __syncthreads();
+        if (k0 + 16 < kNB) {
+            sub_gemm16(X, T, X, k0, 0, nr, k0 + 16, kNB - 16 - k0);
+            __syncthreads();
+        }
+    }
+}
+template <typename BX>
+__device__ __forceinline__ void block_solve_lower(Block64 T, BX X, int nc) {
+#pragma unroll 1
+    for (int k0 = 0; k0 < kNB; k0 += 16) {
+        if (threadIdx.x < nc) sub_solve_lower(T, &X[threadIdx.x][0], k0);
+        __syncthreads();
+        if (k0 + 16 < kNB) {
+            sub_gemm16(T, X, X, k0, k0 + 16, kNB - 16 - k0, 0, nc);
+            __syncthreads();
+        }
+    }
+}
+
+// A block D (nr x nc <= 64 x 64; zero, or the identity when `unit`, elsewhere)
+// from global memory into T[col][row], through L2: 16-byte cp.async when the
+// addresses allow (not waited for here), else through registers.
+__device__ __forceinline__ void request_block(Block64 T, const float *D, int64_t ld, int nr, int nc, bool unit) {
+    if (aligned16(D) && (ld & 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int idx = threadIdx.x + kCT * q;
+            const int c = idx >> 4, r = (idx & 15) * 4;
+            float *dst = &T[c][r];
+            if (c < nc && r + 4 <= nr) {
+                cp_async16(dst, D + (int64_t)c * ld + r, 16);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    dst[e] = c < nc && r + e < nr ? __ldcg(D + (int64_t)c * ld + r + e) : (unit && c == r + e) ? 1.0f : 0.0f;
+            }
+        }
+    } else {
+        float v[16];
+        load_block64(v, D, ld, nr, nc);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int idx = threadIdx.x + kCT * q;
+            const int c = idx / kNB, r = idx % kNB;
+            T[c][r] = c < nc && r < nr ? v[q] : (unit && c == r) ? 1.0f : 0.0f;
+        }
+    }
+}
+
+// ... and back (rows < nr, columns < nc).
+__device__ __forceinline__ void store_block(Block64 T, float *D, int64_t ld, int nr, int nc) {
+    if (aligned16(D) && (ld & 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int idx = threadIdx.x + kCT * q;
+            const int c = idx >> 4, r = (idx & 15) * 4;
+            if (c >= nc) continue;
+            if (r + 4 <= nr) {
+                *reinterpret_cast<float4 *>(D + (int64_t)c * ld + r) = *reinterpret_cast<const float4 *>(&T[c][r]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (r + e < nr) D[(int64_t)c * ld + r + e] = T[c][r + e];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int idx = threadIdx.x + kCT * q;
+            const int c = idx / kNB, r = idx % kNB;
+            if (c < nc && r < nr) D[(int64_t)c * ld + r] = T[c][r];
+        }
+    }
+}
+
+// ---- 64 x 64 no-pivot LU of D (nb <= 64) -------------------------------------
+// sgetrf_nopiv_naive order (sgetrf_nopiv.cpp:27-61): scale by the reciprocal
+// pivot, then the rank-1 update; every element receives its fmaf updates one
+// by one in ascending pivot order, whatever the blocking, so the factors are
+// those of the unblocked loop bit for bit.
+//
+// What bounds it is the chain of 64 pivots.  In blocks of 16 columns (the block
+// in shared memory, T = t[col][row]):
+//  * panel: warp w holds the 16 rows of the diagonal block in lanes 0..15 and
+//    16 of the rows below in lanes 16..31, 16 columns each in registers: the
+//    L panel is solved along with the diagonal block, which every warp
+//    factors for itself (no exchange between warps).  Four pivots at a
+//    time: the four pivot rows go through shared memory to every lane, and
+//    each lane eliminates the 4 x 4 block and the rest of those rows for
+//    itself, so the chain meets one exchange per four pivots (a shuffle per
+//    pivot and column took ~340 cycles per pivot);
+//  * then the 16 rows of U by sub_solve_lower and the rest by sub_gemm16.
+// Rows and columns past nb are those of the identity.
+// The 16 pivots of one panel on this warp's 32 rows (a: this lane's row).  kSafe:
+// reciprocals of pivots outside the fast form's range (subnormal, or 2^126 and
+// above).  Returns -1 or the first zero / non-finite pivot; extreme: set when
+// the fast form met a pivot outside its range (the caller runs it again).
+template <bool kSafe>
+__device__ __forceinline__ int getrf64_panel(float (&a)[16], float (*rows)[4][16], bool &extreme) {
+    const int ln = threadIdx.x & 31;
+    int bad = -1;
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {
+        const int kk = 4 * k4;
+        float(*p)[16] = rows[k4];
+        if (ln >= kk && ln < kk + 4) {
+#pragma unroll
+            for (int q = k4; q < 4; ++q)
+                *reinterpret_cast<float4 *>(&p[ln - kk][4 * q]) = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+        }
+        __syncwarp();
+        float r[4][16];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int q = k4; q < 4; ++q) {
+                const float4 v = *reinterpret_cast<const float4 *>(&p[i][4 * q]);
+                r[i][4 * q + 0] = v.x;
+                r[i][4 * q + 1] = v.y;
+                r[i][4 * q + 2] = v.z;
+                r[i][4 * q + 3] = v.w;
+            }
+        float rp[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float pv = r[i][kk + i];
+            rp[i] = kSafe ? rcp_rn_f32(pv) : rcp_rn_f32_fast(pv);
+            if (!kSafe) extreme |= !rcp_fast_range(pv);
+            const unsigned au = __float_as_uint(pv) & 0x7fffffffu;
+            if (bad < 0 && au - 1u >= 0x7f7fffffu) bad = kk + i;
+#pragma unroll
+            for (int j = i + 1; j < 4; ++j) {
+                const float l = r[j][kk + i] * rp[i];
+#pragma unroll
+                for (int c = kk + i + 1; c < 16; ++c) r[j][c] = fmaf(-r[i][c], l, r[j][c]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool act = ln > kk + i;
+            const float l = a[kk + i] * rp[i];
+            a[kk + i] = act ? l : a[kk + i];
+#pragma unroll
+            for (int c = kk + i + 1; c < 16; ++c) {
+                const float v = fmaf(-r[i][c], l, a[c]);
+                a[c] = act ? v : a[c];
+            }
+        }
+    }
+    return bad;
+}
+
+// in_smem: the block to factor is already in sm.t.t[col][row] (look_ahead), not
+// read from D; either way the factors are written to D.
+__device__ __noinline__ void getrf64(Smem &sm, int nb, float *D, int64_t lda, DevStatus *dst, int pivot_base,
+                                     bool in_smem = false) {
+    Block64 T = sm.t.t;  // T[c][r]: the block, written out at the end
+    const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
+    if (!in_smem) {
+        request_block(T, D, lda, nb, nb, true);
+        cp_async_commit();
+        cp_async_wait<0>();
+    } else if (threadIdx.x >= nb && threadIdx.x < kNB) {
+        T[threadIdx.x][threadIdx.x] = 1.0f;
     }
     __syncthreads();
+#pragma unroll 1
+    for (int k0 = 0; k0 < kNB; k0 += 16) {
+        const bool on = warp == 0 || 16 * warp + 16 < kNB - k0;
+        // lanes 16..31: 16 rows below the diagonal block (the last panel has
+        // none: those lanes follow the diagonal block's own rows)
+        const bool below = k0 + 16 < kNB;
+        const int row = k0 + (ln < 16 ? ln : below ? ln + 16 * warp : ln - 16);
+        float a[16];
+        int bad = -1;
+        if (on) {
+            bool extreme = false;
+#pragma unroll
+            for (int c = 0; c < 16; ++c) a[c] = T[k0 + c][row];
+            bad = getrf64_panel<false>(a, sm.t.rows.r[warp], extreme);
+            if (extreme) {  // the same in every warp: T still holds the panel
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < 16; ++c) a[c] = T[k0 + c][row];
+                bad = getrf64_panel<true>(a, sm.t.rows.r[warp], extreme);
+            }
+        }
+        __syncthreads();  // every warp has read the panel
+        if (on && (ln >= 16 ? below : warp == 0)) {
+#pragma unroll
+            for (int c = 0; c < 16; ++c) T[k0 + c][row] = a[c];
+        }
+        if (warp == 0 && ln == 0 && bad >= 0 && k0 + bad < nb) report(dst, MXP_ZERO_PIVOT, pivot_base + k0 + bad + 1, 0);
+        __syncthreads();
+        if (!below) break;
+        const int R = kNB - 16 - k0;
+        if (threadIdx.x < R) sub_solve_lower(T, &T[k0 + 16 + threadIdx.x][0], k0);
+        __syncthreads();
+        sub_gemm16(T, T, T, k0, k0 + 16, R, k0 + 16, R);
+        __syncthreads();
+    }
+    store_block(T, D, lda, nb, nb);
+    __syncthreads();
+}
+
+// Shared memory of the strip solves and of the look-ahead: the diagonal block (at
+// the place of Smem's t, where getrf64 expects it) and two more blocks.
+struct __align__(16) SmemStrip {
+    float t[kNB][kNB + 4], x[kNB][kNB + 4], y[kNB][kNB + 4];
+    float dinv[kNB];
+};
+
+// Look-ahead: T (in shared memory, for getrf64(..., in_smem = true)) = C - L U,
+// the next diagonal block (nb x nb) with the strips' first 64 rows and columns.
+// 8 x 4 outputs per thread of four warps; one fmaf chain over ascending k per
+// element, subtracted from C, as the other tiles of the update.
+__device__ __noinline__ void look_ahead(SmemStrip &s, int nb, const float *L, const float *U, const float *C,
+                                        int64_t ld) {
+    request_block(s.x, L, ld, nb, kNB, false);
+    request_block(s.y, U, ld, kNB, nb, false);
+    request_block(s.t, C, ld, nb, nb, false);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    if (threadIdx.x < 128) {
+        const int r = 4 * (threadIdx.x % 8), c = 4 * (threadIdx.x / 8);
+        float acc[4][8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[j][i] = 0.0f;
+#pragma unroll 4
+        for (int k4 = 0; k4 < kNB / 4; ++k4) {
+            float4 bq[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bq[j] = *reinterpret_cast<const float4 *>(&s.y[c + j][4 * k4]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 a0 = *reinterpret_cast<const float4 *>(&s.x[4 * k4 + e][r]);
+                const float4 a1 = *reinterpret_cast<const float4 *>(&s.x[4 * k4 + e][32 + r]);
+                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float bv = e == 0 ? bq[j].x : e == 1 ? bq[j].y : e == 2 ? bq[j].z : bq[j].w;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[j][i] = fmaf(av[i], bv, acc[j][i]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s.t[c + j][(i < 4 ? 0 : 28) + r + i] -= acc[j][i];
+    }
+    __syncthreads();
+}
+
+// Strip items of kStripW rows (L strip, X U = B) or columns (U strip, L X = B):
+// items 0 .. lit-1 are the L strip's, the rest the U strip's.  rem: rows of the
+// L strip (columns of the U strip); ld of both.
+constexpr int kStripW = 32;
+__device__ __noinline__ void strip_items(SmemStrip &s, int first, int stride, int lit, int rem, const float *D,
+                                         float *Ls, float *Us, int64_t ld) {
+    for (int it = first; it < 2 * lit; it += stride) {
+        const bool left = it < lit;
+        const int o = (left ? it : it - lit) * kStripW, w = min(kStripW, rem - o);
+        float *B = left ? Ls + o : Us + (int64_t)o * ld;
+        if (it == first) request_block(s.t, D, ld, kNB, kNB, false);
+        request_block(s.x, B, ld, left ? w : kNB, left ? kNB : w, false);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        if (left) {
+            if (threadIdx.x < kNB) s.dinv[threadIdx.x] = 1.0f / s.t[threadIdx.x][threadIdx.x];
+            __syncthreads();
+            block_solve_upper(s.t, s.dinv, s.x, kStripW);
+        } else {
+            block_solve_lower(s.t, s.x, kStripW);
+        }
+        store_block(s.x, B, ld, left ? w : kNB, left ? kNB : w);
+        __syncthreads();
+    }
 }
 
 // D (nb x nb, factored) into shared memory: t[col][row], the skewed rows of U
@@ -682,82 +978,27 @@ __device__ __forceinline__ void trsm_col(Smem &sm, float (&x)[kNB], int nb, floa
     trsm_col_phase<16>(sm, x, 48, nb, out);
 }
 
-// U strip columns [c0, c0 + 64) of B (nb x ncols): X = L^{-1} B, L = unit lower
-// part of the diagonal block (load_tri).  The 64 x 64 block moves through
-// shared memory (ub, over the dead t) with coalesced loads and stores;
-// threads 0..63 solve one column each.
-// v[0..15]: the block, already loaded by load_block64(v, B + c0 ldb, ldb, nb, ncols - c0)
-template <int N>
-__device__ void trsm_cols64_loaded(Smem &sm, const float (&v)[N], int ncols, int nb, float *B, int64_t ldb,
-                                   int c0) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const int idx = threadIdx.x + kCT * q;
-        sm.t.ub[idx / kNB][idx % kNB] = v[q];
-    }
-    __syncthreads();
-    if (threadIdx.x < kNB) {
-        const int j = threadIdx.x;
-        float x[kNB];
-#pragma unroll
-        for (int k = 0; k < kNB; ++k) x[k] = sm.t.ub[j][k];
-        trsm_col(sm, x, nb, &sm.t.ub[j][0]);
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < kNB * kNB; idx += kCT) {
-        const int k = idx % kNB, j = idx / kNB;
-        if (k < nb && c0 + j < ncols) B[(int64_t)(c0 + j) * ldb + k] = sm.t.ub[j][k];
-    }
-    __syncthreads();
-}
-
-__device__ void trsm_cols64(Smem &sm, int ncols, int nb, float *B, int64_t ldb, int c0) {
-    float v[16];
-    load_block64(v, B + (int64_t)c0 * ldb, ldb, nb, ncols - c0);
-    trsm_cols64_loaded(sm, v, ncols, nb, B, ldb, c0);
-}
-
 // Inverse of the 64 x 64 diagonal block `blk` of an upper non-unit (upper = true)
-// or unit-lower triangle; row i of the inverse solves x T = e_i.
-__device__ void inv_diag_block(Smem &sm, int n, const float *T, int64_t ldt, float *X, int64_t ldx,
-                               int blk, bool upper) {
+// or unit-lower triangle: the strip solves with the identity as right-hand
+// side (a fully unrolled substitution spent ~30 us per block fetching
+// instructions).
+__device__ __noinline__ void inv_diag_block(SmemStrip &s, int n, const float *T, int64_t ldt, float *X, int64_t ldx,
+                                            int blk, bool upper) {
     const int r0 = blk * kNB;
     const int nb = min(kNB, n - r0);
-    {
-        float v[16];
-        load_block64(v, T + r0 + (int64_t)r0 * ldt, ldt, nb, nb);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int idx = threadIdx.x + kCT * q;
-            sm.t.t[idx / kNB][idx % kNB] = v[q];
-        }
-    }
+    request_block(s.t, T + r0 + (int64_t)r0 * ldt, ldt, nb, nb, true);
+    request_block(s.x, nullptr, 0, 0, 0, true);  // the identity
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
-    const int i = threadIdx.x;
-    if (i < nb) {
-        float x[kNB];
-        if (upper) {
-#pragma unroll
-            for (int j = 0; j < kNB; ++j) {
-                float v = (j == i) ? 1.0f : 0.0f;
-#pragma unroll
-                for (int q = 0; q < j; ++q) v -= x[q] * sm.t.t[j][q];
-                x[j] = (j >= i && j < nb) ? v / sm.t.t[j][j] : 0.0f;
-            }
-        } else {
-#pragma unroll
-            for (int jj = 0; jj < kNB; ++jj) {
-                const int j = kNB - 1 - jj;
-                float v = (j == i) ? 1.0f : 0.0f;
-#pragma unroll
-                for (int q = j + 1; q < kNB; ++q) v -= x[q] * sm.t.t[j][q];
-                x[j] = (j <= i) ? v : 0.0f;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kNB; ++j)
-            if (j < nb) X[(int64_t)(r0 + j) * ldx + r0 + i] = x[j];
+    if (upper) {
+        if (threadIdx.x < kNB) s.dinv[threadIdx.x] = 1.0f / s.t[threadIdx.x][threadIdx.x];
+        __syncthreads();
+        block_solve_upper(s.t, s.dinv, s.x, kNB);
+    } else {
+        block_solve_lower(s.t, s.x, kNB);
     }
+    store_block(s.x, X + r0 + (int64_t)r0 * ldx, ldx, nb, nb);
     __syncthreads();
 }
 
@@ -774,33 +1015,53 @@ struct Job {
     int64_t ldc, sC;
 };
 
-// sv (when not null, with at least sizeof(SmemGV) bytes behind it): tiles
-// whose operands allow it run as gemm_tile_v.
-__device__ void run_jobs(Smem &sm, const Job *jobs, int njobs, int cta, int ncta, SmemGV *sv = nullptr) {
+// All tiles of the jobs, 64 x 64 (run_tiles64) when every job's operands allow
+// 16-byte copies, else 128 x 128 (gemm_tile).  st: memory for run_tiles64.
+__device__ void run_jobs(Smem &sm, const Job *jobs, int njobs, int cta, int ncta, SmemT64 &st) {
+    bool vec = true;
+    for (int q = 0; q < njobs; ++q) {
+        const Job &J = jobs[q];
+        vec = vec && gemm_tile_v_ok(J.A, J.lda, J.B, J.ldb, J.C, J.ldc, 0) && ((J.sA | J.sB | J.sC) & 3) == 0;
+    }
+    const int TS = vec ? kNB : GBM;
     int tiles[4] = {0, 0, 0, 0}, total = 0;
     for (int q = 0; q < njobs; ++q) {
-        tiles[q] = ((jobs[q].m + GBM - 1) / GBM) * ((jobs[q].n + GBN - 1) / GBN) * jobs[q].batch;
+        tiles[q] = ((jobs[q].m + TS - 1) / TS) * ((jobs[q].n + TS - 1) / TS) * jobs[q].batch;
         total += tiles[q];
     }
-    for (int it = cta; it < total; it += ncta) {
+    auto get = [&](int it, Tile64 &w) {
         int q = 0, r = it;
         while (r >= tiles[q]) r -= tiles[q++];
         const Job &J = jobs[q];
-        const int tm = (J.m + GBM - 1) / GBM, tn = (J.n + GBN - 1) / GBN;
+        const int tm = (J.m + TS - 1) / TS, tn = (J.n + TS - 1) / TS;
         const int z = r / (tm * tn);
         const int rt = r % (tm * tn);
-        const int m0 = (rt % tm) * GBM, n0 = (rt / tm) * GBN;
-        int kb = 0, ke = J.K;
-        if (J.tri == 1) kb = m0;
-        if (J.tri == 2) ke = min(J.K, m0 + GBM);
-        if (J.tri == 3) ke = min(J.K, n0 + GBN);
-        if (J.tri == 4) kb = n0;
-        const float *Az = J.A + J.sA * z, *Bz = J.B + J.sB * z;
-        float *Cz = J.C + J.sC * z;
-        if (sv && gemm_tile_v_ok(Az, J.lda, Bz, J.ldb, Cz, J.ldc, kb))
-            gemm_tile_v(*sv, J.m, J.n, kb, ke, J.alpha, Az, J.lda, Bz, J.ldb, false, Cz, J.ldc, m0, n0);
-        else
-            gemm_tile(sm, J.m, J.n, kb, ke, J.alpha, Az, J.lda, Bz, J.ldb, false, Cz, J.ldc, m0, n0);
+        w.m0 = (rt % tm) * TS;
+        w.n0 = (rt / tm) * TS;
+        w.kb = 0;
+        w.ke = J.K;
+        if (J.tri == 1) w.kb = w.m0;
+        if (J.tri == 2) w.ke = min(J.K, w.m0 + TS);
+        if (J.tri == 3) w.ke = min(J.K, w.n0 + TS);
+        if (J.tri == 4) w.kb = w.n0;
+        w.m = J.m;
+        w.n = J.n;
+        w.A = J.A + J.sA * z;
+        w.B = J.B + J.sB * z;
+        w.C = J.C + J.sC * z;
+        w.lda = J.lda;
+        w.ldb = J.ldb;
+        w.ldc = J.ldc;
+        w.alpha = J.alpha;
+    };
+    if (vec) {
+        run_tiles64<false>(st, cta, ncta, total, get);
+        return;
+    }
+    for (int it = cta; it < total; it += ncta) {
+        Tile64 w;
+        get(it, w);
+        gemm_tile(sm, w.m, w.n, w.kb, w.ke, w.alpha, w.A, w.lda, w.B, w.ldb, false, w.C, w.ldc, w.m0, w.n0);
     }
 }
 
@@ -815,13 +1076,12 @@ __device__ void run_jobs(Smem &sm, const Job *jobs, int njobs, int cta, int ncta
 // blocks of size s_stop (the caller finishes those levels elsewhere).
 template <typename Sync>
 __device__ bool tri_inverses(Smem &sm, int n, const float *A, int64_t lda, float *XU, float *XL, int64_t ldx,
-                             float *tmpU, float *tmpL, int cta, int G, Sync sync, int s_stop = 0,
-                             SmemGV *sv = nullptr) {
+                             float *tmpU, float *tmpL, int cta, int G, Sync sync, int s_stop, SmemT64 &st, SmemStrip &ss) {
     const int nsteps = (n + kNB - 1) / kNB;
     // invert the diagonal 64 x 64 blocks and zero the opposite block-triangle
     const int nblk = nsteps;
     for (int it = cta; it < 2 * nblk; it += G)
-        inv_diag_block(sm, n, A, lda, it < nblk ? XU : XL, ldx, it % nblk, it < nblk);
+        inv_diag_block(ss, n, A, lda, it < nblk ? XU : XL, ldx, it % nblk, it < nblk);
     {   // zero the opposite block-triangles: a column per warp, rows by lanes
         // (a flat index split by 64-bit division cost ~30 us per 2560 block)
         constexpr int W = kCT / 32;
@@ -861,7 +1121,7 @@ __device__ bool tri_inverses(Smem &sm, int n, const float *A, int64_t lda, float
             jb[nj++] = Job{c, S, S, 1, 4, 1.0f, L + (r0 + S) + r0 * ldl, ldl, 0, XL + r0 + r0 * ldx, ldx, 0,
                            tmpL + np * SS, c, 0};
         }
-        run_jobs(sm, jb, nj, cta, G, sv);
+        run_jobs(sm, jb, nj, cta, G, st);
         if (!sync(24)) return false;
         // phase b:  X12 = -inv(U11) T_U;  X21 = -inv(L22) T_L
         nj = 0;
@@ -876,7 +1136,7 @@ __device__ bool tri_inverses(Smem &sm, int n, const float *A, int64_t lda, float
             jb[nj++] = Job{c, S, c, 1, 2, -1.0f, XL + (r0 + S) + (r0 + S) * ldx, ldx, 0, tmpL + np * SS, c, 0,
                            XL + (r0 + S) + r0 * ldx, ldx, 0};
         }
-        run_jobs(sm, jb, nj, cta, G, sv);
+        run_jobs(sm, jb, nj, cta, G, st);
         if (!sync(25)) return false;
     }
     return true;

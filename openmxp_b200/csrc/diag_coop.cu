@@ -12,14 +12,12 @@
 // grid barriers:
 //
 //   LU, for each 64-column step j (D_j = diagonal 64 x 64 block):
-//     strips : L strip rows (thread per row, X = B U_jj^{-1}) and U strip
-//              columns (thread per column, X = L_jj^{-1} B, staged through
-//              shared memory), 64 per item, right-looking against D_j held in
-//              shared memory, items spread over all CTAs;
-//     update : trailing rank-64 update in 128 x 128 SIMT tiles.  CTA 0
-//              updates only D_{j+1} (64 x 64) and factors it right away
-//              (look-ahead), so the 64-step serial factor overlaps the rest of
-//              the update; the CTA owning tile 0 skips that corner.
+//     strips : L strip rows (X = B U_jj^{-1}) and U strip columns (X =
+//              L_jj^{-1} B), 32 per item, against D_j, all in shared memory,
+//              items spread over all CTAs;
+//     update : trailing rank-64 update in 64 x 64 SIMT tiles.  CTA 0
+//              updates only D_{j+1} and factors it right away (look-ahead),
+//              so the serial factor overlaps the rest of the update.
 //   inverses: 64 x 64 diagonal blocks of inv(U) and inv(L) one per item,
 //             then recursive doubling: for adjacent S-blocks the off-diagonal
 //             block of the inverse is -inv(A) B inv(C), two GEMM phases per
@@ -31,6 +29,10 @@
 // kWaitTimeoutNs, after which the CTA records MXP_TIMEOUT, raises the shared
 // abort word so the others leave at their next barrier, and returns.
 // All reads of data written by other CTAs go through L2 (ld.global.cg).
+#include <stddef.h>
+
+#include <algorithm>
+
 #include "dense_tile.cuh"
 #include "mxp_internal.cuh"
 
@@ -66,10 +68,14 @@ __device__ bool grid_sync(const Ctl &c, unsigned int &epoch, int where) {
     epoch += gridDim.x;
     if (threadIdx.x == 0) {
         int ok = 1;
-        __threadfence();
-        atomicAdd(c.count, 1u);
+        // release: every write of the CTA (ordered before this thread by the
+        // CTA barrier) is visible to whoever acquires the count
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c.count) : "memory");
         const unsigned long long t0 = globaltimer_ns();
-        while (ld_acquire_u32(c.count) < epoch) {
+        // back-to-back polls; the abort word and the clock (each a round trip
+        // of its own) only every 64th
+        for (unsigned it = 1; ld_acquire_u32(c.count) < epoch; ++it) {
+            if (it & 63u) continue;
             if (ld_relaxed_i32(c.abort)) {
                 ok = 0;
                 break;
@@ -80,7 +86,6 @@ __device__ bool grid_sync(const Ctl &c, unsigned int &epoch, int where) {
                 report(c.dst, MXP_TIMEOUT, where, blockIdx.x);
                 break;
             }
-            __nanosleep(64);
         }
         ok_sh = ok;
     }
@@ -88,22 +93,19 @@ __device__ bool grid_sync(const Ctl &c, unsigned int &epoch, int where) {
     return ok_sh != 0;
 }
 
-// Dynamic shared memory.  kStaged: the 128 x 128 update tiles are
-// gemm_tile_v's (the Smem union and its two 64-deep slices share ~132 KB);
-// otherwise gemm_tile's, in the ~50 KB of the Smem union.  Blocks below
-// kStagedMinN have few update tiles per step, none on the step's critical
-// path, and run ~2 % faster with the smaller allocation.
-constexpr size_t kSmemPlain = sizeof(Smem);
-constexpr size_t kSmemStaged = sizeof(Smem) > sizeof(SmemGV) ? sizeof(Smem) : sizeof(SmemGV);
-constexpr int kStagedMinN = 2048;
+// Dynamic shared memory: the SIMT pieces' union and the two tile buffers of
+// run_tiles64 share it.
+constexpr size_t kCoopSmem = sizeof(Smem) > sizeof(SmemT64) ? sizeof(Smem) : sizeof(SmemT64);
+static_assert(sizeof(SmemStrip) <= kCoopSmem && offsetof(SmemStrip, t) == 0 && offsetof(SmemTri, t) == 0,
+              "the look-ahead leaves its block where getrf64 reads it");
 
-template <bool kStaged>
 __global__ void __launch_bounds__(kCT, 1)
 diag_factor_kernel(int n, float *A, int64_t lda, float *XU, float *XL, int64_t ldx, float *tmpU,
                    float *tmpL, Ctl ctl, int pivot_base, int inv_stop) {
     extern __shared__ __align__(16) unsigned char coop_smem[];
     Smem &sm = *reinterpret_cast<Smem *>(coop_smem);
-    SmemGV &sv = *reinterpret_cast<SmemGV *>(coop_smem);  // the same memory, for gemm_tile_v (kStaged)
+    SmemT64 &st = *reinterpret_cast<SmemT64 *>(coop_smem);  // the same memory
+    SmemStrip &ss = *reinterpret_cast<SmemStrip *>(coop_smem);
     const int G = gridDim.x, cta = blockIdx.x;
     unsigned int epoch = 0;
     const int nsteps = (n + kNB - 1) / kNB;
@@ -120,46 +122,26 @@ diag_factor_kernel(int n, float *A, int64_t lda, float *XU, float *XL, int64_t l
         float *Lstrip = Djj + nbk;
         float *Ustrip = Djj + (int64_t)nbk * lda;
         // strips
-        const int lit = (rem + kNB - 1) / kNB, uit = (rem + kNB - 1) / kNB;  // 64-row / 64-column items
-        if (cta < lit + uit) {
-            // the first item's operands are requested before the diagonal
-            // block, so the two L2 round trips overlap
-            // (a row of the L strip in x, or the U strip block in x[0..15])
-            float x[kNB];
-            const int it0 = cta;
-            if (it0 < lit) trsm_rows_load(x, rem, nbk, Lstrip, lda, it0 * kNB, kNB);
-            else load_block64(x, Ustrip + (int64_t)(it0 - lit) * kNB * lda, lda, nbk, rem - (it0 - lit) * kNB);
-            load_tri(sm, nbk, Djj, lda);
-            if (it0 < lit) trsm_rows_solve(sm, x, rem, nbk, Lstrip, lda, it0 * kNB, kNB);
-            else trsm_cols64_loaded(sm, x, rem, nbk, Ustrip, lda, (it0 - lit) * kNB);
-            for (int it = cta + G; it < lit + uit; it += G) {
-                if (it < lit) trsm_rows(sm, rem, nbk, Lstrip, lda, it * kNB, kNB);
-                else trsm_cols64(sm, rem, nbk, Ustrip, lda, (it - lit) * kNB);
-            }
-        }
+        strip_items(ss, cta, G, (rem + kStripW - 1) / kStripW, rem, Djj, Lstrip, Ustrip, lda);
         if (!grid_sync(ctl, epoch, 21)) return;
         // trailing rank-nbk update.  CTA 0 updates only the next diagonal block
-        // (64 x 64) and factors it at once (look-ahead); the CTA owning tile 0
-        // leaves that corner alone.
+        // (64 x 64) and factors it at once (look-ahead); the others leave that
+        // corner alone.
         float *C = Ustrip + nbk;
-        const int tm = (rem + GBM - 1) / GBM;
-        const int ntiles = tm * tm;
         const int dn = min(kNB, rem);
         if (cta == 0) {  // the updated block stays in shared memory for the factor
-            gemm_tile64(sm, dn, dn, nbk, -1.0f, Lstrip, lda, Ustrip, lda, C, lda, /*to_smem=*/true);
+            look_ahead(ss, dn, Lstrip, Ustrip, C, lda);
             getrf64(sm, dn, C, lda, ctl.dst, pivot_base + jb + nbk, /*in_smem=*/true);
-        }
-        if (G == 1 || cta > 0) {
-            const int first = G == 1 ? 0 : cta - 1, stride = G == 1 ? 1 : G - 1;
-            const bool vec = kStaged && gemm_tile_v_ok(Lstrip, lda, Ustrip, lda, C, lda, 0);
-            for (int t = first; t < ntiles; t += stride) {
-                if (vec)
-                    gemm_tile_v(sv, rem, rem, 0, nbk, -1.0f, Lstrip, lda, Ustrip, lda, true, C, lda,
-                                (t % tm) * GBM, (t / tm) * GBN, t == 0 ? kNB : 0);
-                else
-                    gemm_tile(sm, rem, rem, 0, nbk, -1.0f, Lstrip, lda, Ustrip, lda, true, C, lda,
-                              (t % tm) * GBM, (t / tm) * GBN, t == 0 ? kNB : 0);
-            }
+        } else if (gemm_tile_v_ok(Lstrip, lda, Ustrip, lda, C, lda, 0)) {
+            const int tm = (rem + kNB - 1) / kNB;
+            run_tiles64<true>(st, cta, G - 1, tm * tm, [&](int t, Tile64 &w) {  // tile 0 is CTA 0's
+                w = Tile64{Lstrip, Ustrip, C, lda, lda, lda, rem, rem, (t % tm) * kNB, (t / tm) * kNB, 0, nbk, -1.0f};
+            });
+        } else {
+            const int tm = (rem + GBM - 1) / GBM;
+            for (int t = cta - 1; t < tm * tm; t += G - 1)
+                gemm_tile(sm, rem, rem, 0, nbk, -1.0f, Lstrip, lda, Ustrip, lda, true, C, lda, (t % tm) * GBM,
+                          (t / tm) * GBN, t == 0 ? kNB : 0);
         }
         if (!grid_sync(ctl, epoch, 22)) return;
     }
@@ -167,19 +149,17 @@ diag_factor_kernel(int n, float *A, int64_t lda, float *XU, float *XL, int64_t l
 
     // ---------------- triangular inverses ----------------
     auto gsync = [&](int where) { return grid_sync(ctl, epoch, where); };
-    tri_inverses(sm, n, A, lda, XU, XL, ldx, tmpU, tmpL, cta, G, gsync, inv_stop, kStaged ? &sv : nullptr);
+    tri_inverses(sm, n, A, lda, XU, XL, ldx, tmpU, tmpL, cta, G, gsync, inv_stop, st, ss);
 }
 
-template <bool kStaged>
 int coop_grid(int device) {
     static int cached[64] = {0};
     if (device < 0 || device >= 64) return 0;
     if (!cached[device]) {
-        const size_t smem = kStaged ? kSmemStaged : kSmemPlain;
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        cudaFuncSetAttribute(diag_factor_kernel<kStaged>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, diag_factor_kernel<kStaged>, kCT, smem);
+        cudaFuncSetAttribute(diag_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoopSmem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, diag_factor_kernel, kCT, kCoopSmem);
         cached[device] = per_sm > 0 ? sms : -1;
     }
     return cached[device];
@@ -236,21 +216,17 @@ mxp_status launch_diag_factor(int n, float *A, int64_t lda, float *XU, float *XL
     if (XU && (!tmpU || !tmpL)) return fail(MXP_INVALID_ARG, "diag_factor: inverse scratch missing");
     int dev = 0;
     MXP_CUDA(cudaGetDevice(&dev));
-    const bool staged = n >= kStagedMinN;
-    const int sms = staged ? coop_grid<true>(dev) : coop_grid<false>(dev);
+    const int sms = coop_grid(dev);
     if (sms <= 0) return fail(MXP_UNSUPPORTED, "diag_factor: kernel cannot be made resident");
-    const int tm = (n + GBM - 1) / GBM;
-    int grid = min(sms, max(2, tm * tm));
+    // a CTA per 64 x 64 tile of the first update, at least two (CTA 0 only
+    // updates and factors the next diagonal block)
+    const int tm = (n + kNB - 1) / kNB;
+    int grid = (int)imin64(sms, std::max<int64_t>(2, (int64_t)tm * tm));
     if (max_grid > 0) grid = min(grid, max(2, max_grid));
     MXP_CUDA(cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), st));
     Ctl ctl{sync_words, reinterpret_cast<int *>(sync_words + 1), dst};
     void *args[] = {&n, &A, &lda, &XU, &XL, &ldx, &tmpU, &tmpL, &ctl, &pivot_base, &inv_stop};
-    if (staged)
-        MXP_CUDA(cudaLaunchCooperativeKernel((const void *)diag_factor_kernel<true>, dim3(grid), dim3(kCT), args,
-                                             kSmemStaged, st));
-    else
-        MXP_CUDA(cudaLaunchCooperativeKernel((const void *)diag_factor_kernel<false>, dim3(grid), dim3(kCT), args,
-                                             kSmemPlain, st));
+    MXP_CUDA(cudaLaunchCooperativeKernel((const void *)diag_factor_kernel, dim3(grid), dim3(kCT), args, kCoopSmem, st));
     MXP_LAUNCHED();
     return MXP_OK;
 }

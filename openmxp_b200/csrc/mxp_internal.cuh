@@ -58,19 +58,36 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
-// Round-to-nearest FP32 reciprocal without a branch: the hardware FP64
-// approximation (rcp.approx.ftz.f64) refined by two Newton-Raphson steps
-// r += r (1 - x r) in FP64, then rounded once to FP32.  For a normal FP32 x,
-// 1/x is never exactly halfway between two FP32 values and never closer to
-// such a point than about 2^-49 (relative), while the refined FP64 value is
-// within about 2^-52 of 1/x, so the single rounding gives the correctly
-// rounded reciprocal.  It serves where the reciprocal is
-// on a latency chain: the IEEE reciprocal of the CUDA runtime takes a
-// data-dependent branch that keeps later independent instructions from being
-// issued ahead of it.  Checked bit for bit against that reciprocal by
-// mxp_check_reciprocal.  Zero, infinite and NaN inputs give NaN (callers
-// report such pivots as errors).
+// Round-to-nearest FP32 reciprocal for a latency chain (the pivots of the 64 x
+// 64 factor).  The IEEE reciprocal of the CUDA runtime takes a data-dependent
+// branch that keeps later independent instructions from being issued ahead of
+// it.  Two forms, both checked bit for bit against that reciprocal by
+// mxp_check_reciprocal:
+//  * rcp_rn_f32_fast, normal |x| < 2^126 (rcp_fast_range; the result is then
+//    normal too): the hardware approximation (rcp.approx.ftz.f32, at most one
+//    ulp off) and one Newton-Raphson step with a fused residual, r + r (1 - x
+//    r): 1 - x r is exact in the fma, so the step's one rounding is that of a
+//    value within ~2^-46 (relative) of 1/x (Markstein, "Computation of
+//    elementary functions on the IBM RISC System/6000 processor", 1990);
+//  * rcp_rn_f32, any x: outside that range the FP64 approximation
+//    (rcp.approx.ftz.f64) refined by two Newton-Raphson steps in FP64, then
+//    rounded once to FP32.  For a normal FP32 x, 1/x is never exactly halfway
+//    between two FP32 values and never closer to such a point than about
+//    2^-49 (relative), while the refined FP64 value is within about 2^-52.
+// Zero, infinite and NaN inputs give NaN (callers report such pivots as
+// errors).
+__device__ __forceinline__ bool rcp_fast_range(float x) {
+    return ((__float_as_uint(x) >> 23) & 0xffu) - 1u < 252u;
+}
+
+__device__ __forceinline__ float rcp_rn_f32_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+
 __device__ __forceinline__ float rcp_rn_f32(float x) {
+    if (rcp_fast_range(x)) return rcp_rn_f32_fast(x);
     const double d = (double)x;
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
