@@ -49,13 +49,7 @@ constexpr int kRowTile = 128;                // MMA M
 constexpr uint32_t kBlockBytes = 16384;      // 128 rows x 64 FP16, swizzled
 constexpr int kMaxStages = 4;
 
-struct BatchSys {
-    int n;          // order (multiple of 128)
-    int pad;
-    uint64_t seed;  // generator seed
-    int64_t a_off;  // first element of the matrix in the packed FP32 array
-    int64_t v_off;  // first element of the vectors in the packed FP64 arrays
-};
+using BatchSys = GenSys;  // n: a multiple of 128
 
 struct BatchOut {
     int iterations;  // refinement steps taken
@@ -1069,12 +1063,7 @@ extern "C" mxp_status mxp_batch_layout(const mxp_batch *bt, int64_t *matrix_floa
 extern "C" mxp_status mxp_batch_matgen(mxp_batch *bt, float *d_A, double *d_d, double *d_rhs, void *stream) {
     if (!bt || !d_A || !d_d || !d_rhs) return fail(MXP_INVALID_ARG, "batch_matgen: NULL argument");
     cudaStream_t st = as_stream(stream);
-    for (int i = 0; i < bt->count; ++i) {
-        mxp_status s = launch_matgen(bt->n[i], bt->seed[i], MXP_DIAG_ROWSUM, d_A + bt->a_off[i], bt->n[i],
-                                     d_d + bt->v_off[i], nullptr, d_rhs + bt->v_off[i], st);
-        if (s != MXP_OK) return s;
-    }
-    return MXP_OK;
+    return launch_matgen_batch(bt->count, bt->d_sys, bt->nmax, d_A, d_d, d_rhs, st);
 }
 
 extern "C" mxp_status mxp_batch_set_config(mxp_batch *bt, int b, int tile_n, int stages) {

@@ -181,6 +181,19 @@ mxp_status launch_matgen_f64(int n, uint64_t seed, int diag_rule, double *A, int
 mxp_status launch_matgen(int n, uint64_t seed, int diag_rule, float *A, int64_t lda, double *d,
                          double *rowsum, double *rhs, cudaStream_t st);
 
+// One system of a batch: order, generator seed, first element of its matrix in
+// the packed FP32 array and of its vectors in the packed FP64 ones.
+struct GenSys {
+    int n;
+    int pad;
+    uint64_t seed;
+    int64_t a_off, v_off;
+};
+// The matrices (diagonal: row sums), diagonals and right-hand sides of count
+// systems (sys: device array, orders at most nmax) in one launch.
+mxp_status launch_matgen_batch(int count, const GenSys *sys, int nmax, float *A, double *d, double *rhs,
+                               cudaStream_t st);
+
 mxp_status launch_getrf_blocked(int n, float *A, int64_t lda, DevStatus *dst, int pivot_base,
                                 cudaStream_t st);
 mxp_status launch_trsm_runn(int m, int n, const float *U, int64_t ldu, float *B, int64_t ldb,
