@@ -392,41 +392,4 @@ mxp_status launch_getrf_blocked(int n, float *A, int64_t lda, DevStatus *dst, in
     return MXP_OK;
 }
 
-mxp_status launch_trsm_runn(int m, int n, const float *U, int64_t ldu, float *B, int64_t ldb,
-                            cudaStream_t st) {
-    if (m <= 0 || n <= 0) return MXP_OK;
-    if (ldu < n || ldb < m) return fail(MXP_INVALID_ARG, "trsm_right_upper: bad leading dimension");
-    for (int jb = 0; jb < n; jb += kNB) {
-        const int nbk = n - jb < kNB ? n - jb : kNB;
-        const float *Ujj = U + jb + (int64_t)jb * ldu;
-        float *Bj = B + (int64_t)jb * ldb;
-        trsm_runn_small_kernel<<<(unsigned)cdiv(m, 128), 128, 0, st>>>(m, nbk, Ujj, ldu, Bj, ldb);
-        MXP_LAUNCHED();
-        const int rem = n - jb - nbk;
-        if (rem <= 0) continue;
-        mxp_status s = launch_sgemm_sub(m, rem, nbk, Bj, ldb, Ujj + (int64_t)nbk * ldu, ldu,
-                                        Bj + (int64_t)nbk * ldb, ldb, st);
-        if (s != MXP_OK) return s;
-    }
-    return MXP_OK;
-}
-
-mxp_status launch_trsm_llnu(int m, int n, const float *L, int64_t ldl, float *B, int64_t ldb,
-                            cudaStream_t st) {
-    if (m <= 0 || n <= 0) return MXP_OK;
-    if (ldl < m || ldb < m) return fail(MXP_INVALID_ARG, "trsm_left_lower_unit: bad leading dimension");
-    for (int jb = 0; jb < m; jb += kNB) {
-        const int nbk = m - jb < kNB ? m - jb : kNB;
-        const float *Ljj = L + jb + (int64_t)jb * ldl;
-        trsm_llnu_small_kernel<<<(unsigned)cdiv(n, 64), 256, 0, st>>>(n, nbk, Ljj, ldl, B + jb, ldb);
-        MXP_LAUNCHED();
-        const int rem = m - jb - nbk;
-        if (rem <= 0) continue;
-        mxp_status s = launch_sgemm_sub(rem, n, nbk, Ljj + nbk, ldl, B + jb, ldb, B + jb + nbk,
-                                        ldb, st);
-        if (s != MXP_OK) return s;
-    }
-    return MXP_OK;
-}
-
 }  // namespace mxp
