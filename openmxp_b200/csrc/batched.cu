@@ -25,6 +25,7 @@
 //    r in shared memory).
 // Every wait is bounded; a timeout records MXP_TIMEOUT, stops all roles, frees
 // TMEM and returns.
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -66,6 +67,7 @@ struct BatchArgs {
     int count;
     int b;                 // block size (multiple of 64, <= 256)
     int stages;            // smem ring depth
+    int ncbuf;             // slots of the epilogue's C staging (1 or 2)
     int maxit;
     float *A;
     const double *d;
@@ -75,6 +77,7 @@ struct BatchArgs {
     uint8_t *staging;      // per-CTA FP16 operand staging
     int64_t staging_stride;  // bytes per CTA
     int64_t rstage_off;    // offset of the R staging inside a CTA's area
+    int64_t wstage_off;    // offset of the strips' triangle images
     unsigned int *ticket;
     DevStatus *dst;
 };
@@ -91,81 +94,8 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// Cast one operand row (bk values, v(k) for k in [0, bk)) into the staging area:
-// slice s = k / 64 of row-block rt lives at base + (s * nblk + rt) * 16 KB.
-template <typename Get>
-__device__ __forceinline__ void stage_row(uint8_t *base, int nblk, int row, int bk, Get v) {
-    const int rt = row >> 7, r = row & 127;
-    for (int s = 0; s < bk / kSliceK; ++s) {
-        uint8_t *blk = base + ((int64_t)s * nblk + rt) * kBlockBytes;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const int k = s * kSliceK + c * 8;
-            uint4 q;
-            q.x = pack_h2(v(k + 0), v(k + 1));
-            q.y = pack_h2(v(k + 2), v(k + 3));
-            q.z = pack_h2(v(k + 4), v(k + 5));
-            q.w = pack_h2(v(k + 6), v(k + 7));
-            *reinterpret_cast<uint4 *>(blk + sw128_offset(r, c)) = q;
-        }
-    }
-}
-
-// The same for a row whose bk values are contiguous and 16-byte aligned in
-// memory (a column of the U strip, i.e. a row of R = U^T): eight values per
-// chunk as two 16-byte loads (a whole 32-byte sector per thread; the scalar
-// form read 4 bytes of a sector per load across 32 columns per warp).
-__device__ __forceinline__ void stage_row_contig(uint8_t *base, int nblk, int row, int bk, const float *src) {
-    const int rt = row >> 7, r = row & 127;
-    for (int s = 0; s < bk / kSliceK; ++s) {
-        uint8_t *blk = base + ((int64_t)s * nblk + rt) * kBlockBytes;
-        float4 lo[8], hi[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const float4 *p4 = reinterpret_cast<const float4 *>(src + s * kSliceK + c * 8);
-            lo[c] = __ldcg(p4);
-            hi[c] = __ldcg(p4 + 1);
-        }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            uint4 q;
-            q.x = pack_h2(lo[c].x, lo[c].y);
-            q.y = pack_h2(lo[c].z, lo[c].w);
-            q.z = pack_h2(hi[c].x, hi[c].y);
-            q.w = pack_h2(hi[c].z, hi[c].w);
-            *reinterpret_cast<uint4 *>(blk + sw128_offset(r, c)) = q;
-        }
-    }
-}
-
-// Four consecutive rows r4 .. r4 + 3 of a column-major panel (row i, value k at
-// src[(i - r4) + k * ld], src 16-byte aligned, ld % 4 == 0): each k read as one
-// 16-byte load of the four rows (a warp covers 128 consecutive rows, 512
-// contiguous bytes), instead of a 4-byte load per row.  Not inlined (the
-// persistent kernel around it is at the register limit).
-__device__ __noinline__ void stage_rows4(uint8_t *base, int nblk, int r4, int bk, const float *src, int64_t ld) {
-    const int rt = r4 >> 7, r = r4 & 127;
-    for (int s = 0; s < bk / kSliceK; ++s) {
-        uint8_t *blk = base + ((int64_t)s * nblk + rt) * kBlockBytes;
-#pragma unroll 2
-        for (int c = 0; c < 8; ++c) {
-            const int k = s * kSliceK + c * 8;
-            float4 v[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = __ldcg(reinterpret_cast<const float4 *>(src + (int64_t)(k + e) * ld));
-            uint4 q0, q1, q2, q3;
-            q0.x = pack_h2(v[0].x, v[1].x); q0.y = pack_h2(v[2].x, v[3].x); q0.z = pack_h2(v[4].x, v[5].x); q0.w = pack_h2(v[6].x, v[7].x);
-            q1.x = pack_h2(v[0].y, v[1].y); q1.y = pack_h2(v[2].y, v[3].y); q1.z = pack_h2(v[4].y, v[5].y); q1.w = pack_h2(v[6].y, v[7].y);
-            q2.x = pack_h2(v[0].z, v[1].z); q2.y = pack_h2(v[2].z, v[3].z); q2.z = pack_h2(v[4].z, v[5].z); q2.w = pack_h2(v[6].z, v[7].z);
-            q3.x = pack_h2(v[0].w, v[1].w); q3.y = pack_h2(v[2].w, v[3].w); q3.z = pack_h2(v[4].w, v[5].w); q3.w = pack_h2(v[6].w, v[7].w);
-            *reinterpret_cast<uint4 *>(blk + sw128_offset(r + 0, c)) = q0;
-            *reinterpret_cast<uint4 *>(blk + sw128_offset(r + 1, c)) = q1;
-            *reinterpret_cast<uint4 *>(blk + sw128_offset(r + 2, c)) = q2;
-            *reinterpret_cast<uint4 *>(blk + sw128_offset(r + 3, c)) = q3;
-        }
-    }
-}
-
+// A zero row of the staging area: slice s = k / 64 of row-block rt lives at
+// base + (s * nblk + rt) * 16 KB.
 __device__ __forceinline__ void stage_zero_row(uint8_t *base, int nblk, int row, int bk) {
     const int rt = row >> 7, r = row & 127;
     for (int s = 0; s < bk / kSliceK; ++s) {
@@ -252,10 +182,9 @@ __device__ __noinline__ void panel_tile_v(SmemGV &sv, int m, int n, const float 
     gemm_tile_v<MI, NJ>(sv, m, n, 0, kNB, -1.0f, A, ld, B, ld, true, C, ld, m0, n0);
 }
 
-// ---- panel factorisation of one block step (SIMT FP32, whole CTA) -----------
-// D = A(k0, k0) (bk x bk), L strip = A(k0+bk.., k0..) (m x bk), U strip =
-// A(k0.., k0+bk..) (bk x m); lda = n.
-__device__ void factor_step(Smem &sm, float *stage, float *A, int n, int k0, int bk, DevStatus *dst) {
+// ---- diagonal block of one block step (SIMT FP32, whole CTA) -----------------
+// D = A(k0, k0) (bk x bk), lda = n.
+__device__ void factor_diag(Smem &sm, float *stage, float *A, int n, int k0, int bk, DevStatus *dst) {
     const int64_t lda = n;
     // the rank-64 updates as cp.async-staged tiles when the system allows
     // 16-byte copies (its base 16-byte aligned, n a multiple of 4)
@@ -272,8 +201,7 @@ __device__ void factor_step(Smem &sm, float *stage, float *A, int n, int k0, int
         else gemm_tile(sm, tm_, tn_, 0, kNB, -1.0f, Ap, lda, Bp, lda, true, Cp, lda, m0, n0);
     };
     float *D = A + k0 + (int64_t)k0 * lda;
-    const int m = n - k0 - bk;
-    // diagonal block: blocked by 64, whole CTA
+    // blocked by 64
     for (int jb = 0; jb < bk; jb += kNB) {
         float *Dj = D + jb + (int64_t)jb * lda;
         getrf64(sm, kNB, Dj, lda, dst, k0 + jb);
@@ -288,62 +216,272 @@ __device__ void factor_step(Smem &sm, float *stage, float *A, int n, int k0, int
             tile(rem, rem, Dj + kNB, Dj + (int64_t)kNB * lda, Dj + kNB + (int64_t)kNB * lda, (t % tm) * GBM,
                  (t / tm) * GBN);
     }
-    if (m <= 0) return;
-    float *Ls = D + bk;                     // m x bk
-    float *Us = D + (int64_t)bk * lda;      // bk x m
-    // L strip: X U = B, one 64-column block at a time
-    for (int c = 0; c < bk; c += kNB) {
-        load_tri(sm, kNB, D + c + (int64_t)c * lda, lda);
-        for (int r0 = 0; r0 < m; r0 += kCT) trsm_rows(sm, m, kNB, Ls + (int64_t)c * lda, lda, r0);
-        __syncthreads();
-        const int rest = bk - c - kNB;
-        if (rest > 0) {
-            const int tm = (m + GBM - 1) / GBM, tn = (rest + GBN - 1) / GBN;
-            for (int t = 0; t < tm * tn; ++t)
-                tile(m, rest, Ls + (int64_t)c * lda, D + c + (int64_t)(c + kNB) * lda, Ls + (int64_t)(c + kNB) * lda,
-                     (t % tm) * GBM, (t / tm) * GBN);
-        }
-    }
-    // U strip: L X = B, one 64-row block at a time, one group of 256 columns
-    // after another.  Its columns are independent, so every element receives
-    // the same operations in the same order as with the row blocks outermost;
-    // but a column's 64-row slices (256 bytes each) are then read while the
-    // group is still in L2, instead of four passes over the whole strip from
-    // DRAM (2048 systems of orders 256..4096: U strip 163 -> 135 ms per CTA;
-    // the diagonal triangle reloaded per group costs little).
-    for (int g0 = 0; g0 < m; g0 += kCT) {
-        const int ge = min(m, g0 + kCT);
-        for (int c = 0; c < bk; c += kNB) {
-            load_tri(sm, kNB, D + c + (int64_t)c * lda, lda);
-            trsm_cols_staged(sm, stage, m, kNB, Us + c, lda, g0);
-            __syncthreads();
-            const int rest = bk - c - kNB;
-            if (rest > 0) {
-                const int tm = (rest + GBM - 1) / GBM, tn = (ge - g0 + GBN - 1) / GBN;
-                for (int t = 0; t < tm * tn; ++t)
-                    tile(rest, ge, D + c + kNB + (int64_t)c * lda, Us + c, Us + c + kNB, (t % tm) * GBM,
-                         g0 + (t / tm) * GBN);
-            }
-        }
-    }
 }
 
-// ---- tcgen05 trailing update of one block step --------------------------------
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+// ---- panel strips of one block step: substitution with the products on tcgen05 --
+// L strip: X U = B (rows of A(k0+bk.., k0..)), U strip: L X = B (columns of A(k0..,
+// k0+bk..)).  Both are the same work on m independent vectors of length bk (a
+// row of the L strip, a column of the U strip): x_c = (b_c - sum_{k<c} x_k
+// W(k, c)) / w_c with W(k, c) = U(k, c), or L(c, k) and w = 1.
+//
+// As rank-64 SIMT updates the strips were 42 % of a batch, at half the FP32 FMA
+// rate and bound by shared-memory operand loads.  Here a thread owns a
+// vector and a group of four warps 128 of them, one per TMEM lane; the sums of
+// all bk columns stay in TMEM.  Per 16 columns: b minus the sums, a 16-wide
+// substitution in registers, then sums += X W on the tensor core for every
+// column to the right (N = what is left, K = 16).  The operands stay FP32 in
+// value: each is split exactly into three BF16 terms (8 + 8 + 8 bits), and all
+// products of them above 2^-25 of the whole are taken (eight MMAs; FP32
+// accumulation).  B is read once and X written once, in FP32 and, for the
+// trailing update, rounded to FP16 in the staging area (rounding the strips
+// in a pass of their own took another 5 % of the batch).  The two groups of
+// warps work on tiles of their own, so one's substitution runs under the
+// other's products.
+constexpr int kSB = 16;                              // columns per substitution block
+constexpr int kMaxBk = 256;
+constexpr uint32_t kWImgBytes = kMaxBk * 128;        // W(16 columns k, all c): kMaxBk rows of 128 bytes
+constexpr int64_t kWBytes = (int64_t)(kMaxBk / kSB) * kWImgBytes;  // one side's images
+struct StripSmem {                                   // 1024-byte aligned
+    uint8_t a[2][kBlockBytes];                       // per group: X, 128 rows x (3 x 16 BF16), swizzled
+    uint8_t b[2][2][kWImgBytes];                     // per group, two buffers: W
+    float wd[kMaxBk / kSB][kSB][kSB];                // diagonal blocks, wd[.][c][k] = W(k, c)
+    float dinv[kMaxBk];
+};
+struct StripBars {
+    uint64_t *mma;      // per group: the products of one block are done
+    uint64_t *b;        // per group and buffer: W has landed
+    uint32_t tmem;
+    int *abort_flag;
+};
+struct StripState {  // barrier positions, carried across tiles, steps and systems
+    uint32_t mma_phase = 0, nb = 0;  // nb: W loads of the group so far
+};
 
+// x split into three BF16 terms: x = t0 + t1 + t2 exactly (24 bits), each term's
+// bits in the low half.
+__device__ __forceinline__ void split3(float x, uint32_t (&t)[3]) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(x);
+        t[p] = (uint32_t)__bfloat16_as_ushort(h);
+        x -= __bfloat162float(h);
+    }
+}
+
+// Row r of a 128-byte-swizzled image: 16 values as [t0 | t1 | t2 | unused], 32 bytes each.
+__device__ __forceinline__ void store_split_row(uint8_t *img, int r, const float (&x)[kSB]) {
+    uint8_t *blk = img + (r >> 7) * kBlockBytes;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t t[8][3];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) split3(x[8 * h + e], t[e]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            uint4 q;
+            q.x = t[0][p] | t[1][p] << 16;
+            q.y = t[2][p] | t[3][p] << 16;
+            q.z = t[4][p] | t[5][p] << 16;
+            q.w = t[6][p] | t[7][p] << 16;
+            *reinterpret_cast<uint4 *>(blk + sw128_offset(r & 127, 2 * p + h)) = q;
+        }
+    }
+}
+
+// W's images (global, image kb at wimg + kb * kWImgBytes: rows c > the block) and
+// diagonal blocks, from the factored diagonal block.  All threads.
+template <bool LEFT>
+__device__ __noinline__ void prepare_w(StripSmem &s, const float *D, int64_t lda, int bk, uint8_t *wimg) {
+    for (int id = threadIdx.x; id < bk * (bk / kSB); id += kBatchThreads) {
+        const int c = id % bk, kb = id / bk, k0 = kb * kSB;
+        if (c < k0) continue;
+        float w[kSB];
+#pragma unroll
+        for (int k = 0; k < kSB; ++k)
+            w[k] = LEFT ? __ldcg(D + (k0 + k) + (int64_t)c * lda) : __ldcg(D + c + (int64_t)(k0 + k) * lda);
+        if (c >= k0 + kSB) {
+            store_split_row(wimg + (int64_t)kb * kWImgBytes, c, w);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kSB; ++k) s.wd[kb][c - k0][k] = k < c - k0 ? w[k] : 0.0f;
+        }
+    }
+    if (LEFT)
+        for (int c = threadIdx.x; c < bk; c += kBatchThreads) s.dinv[c] = 1.0f / __ldcg(D + (int64_t)c * (lda + 1));
+}
+
+// The vectors of one strip (S: its first element), tiles of 128 shared out to the
+// two groups.  stage: the FP16 staging area of the strip, nblk 128-row blocks.
+template <bool LEFT>
+__device__ __noinline__ void strip_tiles(StripSmem &s, const StripBars &bars, StripState &ss, float *S, int64_t lda,
+                                         int m, int bk, const uint8_t *wimg, uint8_t *stage, int nblk,
+                                         DevStatus *dst) {
+    const int warp = threadIdx.x >> 5, g = warp >> 2, tg = threadIdx.x & 127;
+    const int nkb = bk / kSB, ntiles = (m + kRowTile - 1) / kRowTile;
+    const uint32_t mma_bar = smem_u32(bars.mma + g);
+    const uint32_t tacc = bars.tmem + (uint32_t)(g * kMaxBk);
+    const uint32_t tlane = tacc + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool lead = tg == 0, vec = aligned16(S) && (lda & 3) == 0;
+    uint8_t *abuf = s.a[g];
+    volatile int *ab = bars.abort_flag;
+    bool ok = true;
+    auto load_w = [&](int kb) {  // rows kSB (kb + 1) .. bk of image kb (one contiguous range), by the lead thread
+        const uint32_t off = (uint32_t)(kb + 1) * kSB * 128, bytes = (uint32_t)bk * 128 - off;
+        const uint32_t buf = ss.nb & 1, bar = smem_u32(bars.b + 2 * g + buf);
+        mbar_expect_tx(bar, bytes);
+        bulk_copy_g2s(smem_u32(s.b[g][buf] + off), wimg + (int64_t)kb * kWImgBytes + off, bytes, bar);
+    };
+    for (int rt = g; rt < ntiles; rt += 2) {
+        const int v = rt * kRowTile + tg;
+        const bool act = v < m;
+        float *vp = LEFT ? S + v : S + (int64_t)v * lda;
+        float b[kSB];
+        auto load_b = [&](int kb) {
+            if (LEFT) {
+#pragma unroll
+                for (int k = 0; k < kSB; ++k) b[k] = act ? __ldcg(vp + (int64_t)(kb * kSB + k) * lda) : 0.0f;
+            } else if (vec) {
+#pragma unroll
+                for (int q = 0; q < kSB / 4; ++q) {
+                    const float4 f = act ? __ldcg(reinterpret_cast<const float4 *>(vp + kb * kSB) + q)
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+                    b[4 * q] = f.x;
+                    b[4 * q + 1] = f.y;
+                    b[4 * q + 2] = f.z;
+                    b[4 * q + 3] = f.w;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kSB; ++k) b[k] = act ? __ldcg(vp + kb * kSB + k) : 0.0f;
+            }
+        };
+        if (lead && nkb > 1) load_w(0);
+        load_b(0);
+#pragma unroll 1
+        for (int kb = 0; kb < nkb; ++kb) {
+            float x[kSB];
+#pragma unroll
+            for (int k = 0; k < kSB; ++k) x[k] = b[k];
+            if (kb + 1 < nkb) load_b(kb + 1);
+            if (kb > 0) {
+                if (!mbar_wait(mma_bar, ss.mma_phase, ab)) {  // raised at once: later waits then return
+                    ok = false;
+                    *ab = 1;
+                }
+                ss.mma_phase ^= 1u;
+                __syncwarp();
+                tc_fence_after();
+                uint32_t acc[kSB];
+                tmem_ld_32x32b_x16(tlane + (uint32_t)(kb * kSB), acc);
+#pragma unroll
+                for (int k = 0; k < kSB; ++k) x[k] -= __uint_as_float(acc[k]);
+            }
+            const float(*w)[kSB] = s.wd[kb];
+#pragma unroll
+            for (int c = 0; c < kSB; ++c) {
+#pragma unroll
+                for (int k4 = 0; 4 * k4 < c; ++k4) {
+                    const float4 u = *reinterpret_cast<const float4 *>(&w[c][4 * k4]);
+                    x[c] = fmaf(-u.x, x[4 * k4], x[c]);
+                    if (4 * k4 + 1 < c) x[c] = fmaf(-u.y, x[4 * k4 + 1], x[c]);
+                    if (4 * k4 + 2 < c) x[c] = fmaf(-u.z, x[4 * k4 + 2], x[c]);
+                    if (4 * k4 + 3 < c) x[c] = fmaf(-u.w, x[4 * k4 + 3], x[c]);
+                }
+                if (LEFT) x[c] *= s.dinv[kb * kSB + c];
+            }
+            if (kb + 1 < nkb) {
+                store_split_row(abuf, tg, x);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                tc_fence_before();
+                asm volatile("barrier.cta.sync %0, 128;" ::"r"(2 + g) : "memory");
+                const uint32_t buf = ss.nb & 1, bphase = (ss.nb >> 1) & 1u;
+                ++ss.nb;
+                if (lead) {
+                    // the other buffer's products (two blocks ago) were waited for above
+                    if (kb + 2 < nkb) load_w(kb + 1);
+                    if (!mbar_wait(smem_u32(bars.b + 2 * g + buf), bphase, ab)) {
+                        ok = false;
+                        *ab = 1;
+                    }
+                    tc_fence_after();
+                    if (ok) {
+                        const uint32_t left = (uint32_t)(bk - (kb + 1) * kSB);
+                        const uint32_t idesc = idesc_f16_mn(1u, kRowTile, (int)left);
+                        const uint32_t a0 = smem_u32(abuf), b0 = smem_u32(s.b[g][buf]) + (uint32_t)(kb + 1) * kSB * 128;
+                        const uint32_t d = tacc + (uint32_t)((kb + 1) * kSB);
+                        // the small products first: they meet the smallest sums
+                        constexpr int pa[8] = {2, 1, 2, 0, 1, 1, 0, 0}, pb[8] = {1, 2, 0, 2, 1, 0, 1, 0};
+#pragma unroll
+                        for (int p = 0; p < 8; ++p)
+                            tc_mma_f16(d, smem_desc_sw128(a0 + 32 * pa[p]), smem_desc_sw128(b0 + 32 * pb[p]), idesc,
+                                       (kb > 0 || p > 0) ? 1u : 0u);
+                        tc_commit(mma_bar);
+                    }
+                }
+                __syncwarp();
+            }
+            // X in FP32 and its FP16 rounding (padding vectors: zero rows), under the products
+            if (act) {
+                if (LEFT) {
+#pragma unroll
+                    for (int k = 0; k < kSB; ++k) vp[(int64_t)(kb * kSB + k) * lda] = x[k];
+                } else if (vec) {
+#pragma unroll
+                    for (int q = 0; q < kSB / 4; ++q)
+                        reinterpret_cast<float4 *>(vp + kb * kSB)[q] =
+                            make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kSB; ++k) vp[kb * kSB + k] = x[k];
+                }
+            }
+            uint8_t *blk = stage + ((int64_t)(kb >> 2) * nblk + rt) * kBlockBytes;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint4 q;
+                q.x = pack_h2(x[8 * h + 0], x[8 * h + 1]);
+                q.y = pack_h2(x[8 * h + 2], x[8 * h + 3]);
+                q.z = pack_h2(x[8 * h + 4], x[8 * h + 5]);
+                q.w = pack_h2(x[8 * h + 6], x[8 * h + 7]);
+                *reinterpret_cast<uint4 *>(blk + sw128_offset(tg, (kb & 3) * 2 + h)) = q;
+            }
+        }
+    }
+    if (!ok && lead) report(dst, MXP_TIMEOUT, 34, blockIdx.x);
+    __syncthreads();
+}
+
+// ---- tcgen05 trailing update of one block step --------------------------------
 struct Ring {
-    float *cbuf;            // epilogue staging of C: 128 columns x 128 rows
+    float *cbuf;            // epilogue staging of C: ncbuf slots of 128 columns x 128 rows
     uint8_t *sA;            // stages x 16 KB
     uint8_t *sB;            // stages x TN x 128 B
     uint64_t *full, *empty; // per stage
     uint64_t *tfull, *tempty;  // per accumulator
     uint32_t tmem;
     int stages;
+    int ncbuf;
 };
+
+// Barrier among the four epilogue warps, and the same with a vote.
+__device__ __forceinline__ void epi_sync() { asm volatile("barrier.cta.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ bool epi_all(bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)v)
+        : "memory");
+    return r != 0;
+}
 
 // Barrier positions carried across steps and systems (each role owns its own).
 struct RoleState {
@@ -424,58 +562,88 @@ __device__ bool schur_step(const Ring &rg, RoleState &rs, volatile int *abort_fl
             if (!ok) report(dst, MXP_TIMEOUT, 32, blockIdx.x);
         }
     } else if (warp >= 4) {  // ---- epilogue: TMEM lane quarter = warp % 4 ----
-        const int quarter = warp & 3;
-        for (int t = 0; t < ntiles && ok; ++t) {
-            const int rt = t / tiles_n, ct = t % tiles_n;
-            if (!mbar_wait(smem_u32(&rg.tfull[rs.acc]), rs.acc_phase, abort_flag)) {
-                ok = false;
-                break;
+        // What bounds it is C's read and write (a tile's products take a sixth
+        // of that time at K = 256), so C is requested ahead: 128 columns of a
+        // tile at a time go to a slot of shared memory by cp.async (16 bytes:
+        // a warp instruction is a whole column), ncbuf slots deep, and the
+        // slot of one tile fills while the products and stores of the tiles
+        // before it run.
+        constexpr int H = TN / 128;
+        const int quarter = warp & 3, nseq = ntiles * H;
+        const bool vec = aligned16(C) && (ldc & 3) == 0 && (m & 3) == 0;
+        auto request = [&](int q) {  // C of 128-column piece q; always one copy group
+            if (q < nseq) {
+                const int t = q / H, row0 = (t / tiles_n) * kRowTile, col0 = (t % tiles_n) * TN + (q % H) * 128;
+                float *slot = rg.cbuf + (q % rg.ncbuf) * (128 * 128);
+                if (vec) {
+                    const int r = 4 * lane;
+                    if (row0 + r < m) {
+                        const float *cp = C + (int64_t)(col0 + quarter * 32) * ldc + row0 + r;
+#pragma unroll 8
+                        for (int j = 0; j < 32; ++j)
+                            if (col0 + quarter * 32 + j < m)
+                                cp_async16(slot + (quarter * 32 + j) * 128 + r, cp + (int64_t)j * ldc, 16);
+                    }
+                } else {
+                    const int r = quarter * 32 + lane;
+                    if (row0 + r < m) {
+                        const float *cp = C + (int64_t)col0 * ldc + row0 + r;
+#pragma unroll 8
+                        for (int j = 0; j < 128; ++j)
+                            if (col0 + j < m)
+                                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(slot + j * 128 + r)),
+                                             "l"(cp + (int64_t)j * ldc)
+                                             : "memory");
+                    }
+                }
             }
-            __syncwarp();
-            tc_fence_after();
+            cp_async_commit();
+        };
+        for (int q = 0; q < rg.ncbuf; ++q) request(q);
+        for (int q = 0; q < nseq; ++q) {
+            const int t = q / H, h = q % H;
+            const int rt = t / tiles_n, ct = t % tiles_n;
+            if (h == 0) {
+                // the four warps leave together or not at all: they meet at barriers below
+                ok = epi_all(mbar_wait(smem_u32(&rg.tfull[rs.acc]), rs.acc_phase, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+            }
+            if (rg.ncbuf == 2) cp_async_wait<1>();
+            else cp_async_wait<0>();
+            epi_sync();  // every warp's copies of this piece have landed
             const int r = quarter * 32 + lane;  // row within the tile
             const int row = rt * kRowTile + r;
             const uint32_t tbase = rg.tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(rs.acc * TN);
+            const int colh = ct * TN + h * 128;
+            const float *slot = rg.cbuf + (q % rg.ncbuf) * (128 * 128) + r;
 #pragma unroll 1
-            for (int h = 0; h < TN / 128; ++h) {
-                // C for 128 columns of this row -> shared memory with async copies (the
-                // bytes in flight are not bounded by registers), then subtract the
-                // accumulator column by column and store
-                const int colh = ct * TN + h * 128;
-                if (row < m) {
-                    const float *cp = C + (int64_t)colh * ldc + row;
-#pragma unroll 8
-                    for (int j = 0; j < 128; ++j)
-                        if (colh + j < m)
-                            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(rg.cbuf + j * 128 + r)),
-                                         "l"(cp + (int64_t)j * ldc)
-                                         : "memory");
+            for (int c = 0; c < 4; ++c) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(tbase + h * 128 + c * 32, v);
+                if (h == H - 1 && c == 3) {  // accumulator drained: the next tile may use it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&rg.tempty[rs.acc]));
                 }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-#pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t v[32];
-                    tmem_ld_32x32b_x32(tbase + h * 128 + c * 32, v);
-                    if (h == TN / 128 - 1 && c == 3) {  // accumulator drained: the next tile may use it
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&rg.tempty[rs.acc]));
-                    }
-                    if (row < m) {
-                        float *cp = C + (int64_t)(colh + c * 32) * ldc + row;
+                if (row < m) {
+                    float *cp = C + (int64_t)(colh + c * 32) * ldc + row;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (colh + c * 32 + j < m)
-                                __stcs(cp + (int64_t)j * ldc, rg.cbuf[(c * 32 + j) * 128 + r] - __uint_as_float(v[j]));
-                    }
+                    for (int j = 0; j < 32; ++j)
+                        if (colh + c * 32 + j < m)
+                            __stcs(cp + (int64_t)j * ldc, slot[(c * 32 + j) * 128] - __uint_as_float(v[j]));
                 }
             }
-            if (++rs.acc == 2) {
-                rs.acc = 0;
-                rs.acc_phase ^= 1u;
+            epi_sync();  // the slot is free
+            request(q + rg.ncbuf);
+            if (h == H - 1) {
+                if (++rs.acc == 2) {
+                    rs.acc = 0;
+                    rs.acc_phase ^= 1u;
+                }
             }
         }
+        cp_async_wait<0>();
         if (!ok && lane == 0) report(dst, MXP_TIMEOUT, 33, blockIdx.x);
     }
     if (!ok) *abort_flag = 1;
@@ -686,11 +854,12 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(BatchKernelAr
     extern __shared__ uint8_t batch_smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(batch_smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) uint64_t bar_full[kMaxStages], bar_empty[kMaxStages], bar_tfull[2], bar_tempty[2];
+    __shared__ __align__(8) uint64_t bar_smma[2], bar_sw[4];
     __shared__ uint32_t tmem_holder;
     __shared__ int abort_flag;
     __shared__ int s_ticket;
     __shared__ double red[kBatchThreads / 32];
-    constexpr uint32_t kTmemCols = 2 * TN;
+    constexpr uint32_t kTmemCols = 512;  // the strips' sums: 2 groups x 256 columns (the trailing update uses 2 x TN)
     const int warp = threadIdx.x >> 5;
 
     if (threadIdx.x == 0) {
@@ -703,6 +872,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(BatchKernelAr
             mbar_init(smem_u32(&bar_tfull[c]), 1);
             mbar_init(smem_u32(&bar_tempty[c]), 4);  // the four epilogue warps
         }
+        for (int c = 0; c < 2; ++c) mbar_init(smem_u32(&bar_smma[c]), 1);
+        for (int c = 0; c < 4; ++c) mbar_init(smem_u32(&bar_sw[c]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -726,12 +897,17 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(BatchKernelAr
     rg.tempty = bar_tempty;
     rg.tmem = tmem_holder;
     rg.stages = a.stages;
+    rg.ncbuf = a.ncbuf;
     RoleState rs;
     Smem &sm = *reinterpret_cast<Smem *>(smem);  // SIMT phases reuse the ring's memory
     float *colstage = reinterpret_cast<float *>(smem + kColStageOff);
     static_assert(sizeof(Smem) <= kColStageOff, "column stage overlaps the SIMT scratch");
     uint8_t *Lst = a.staging + (int64_t)blockIdx.x * a.staging_stride;
     uint8_t *Rst = Lst + a.rstage_off;
+    uint8_t *Wst = Lst + a.wstage_off;
+    StripSmem &ssm = *reinterpret_cast<StripSmem *>(smem);
+    const StripBars sbars{bar_smma, bar_sw, tmem_holder, &abort_flag};
+    StripState sst8;
 
     while (true) {
         if (threadIdx.x == 0) s_ticket = (int)atomicAdd(a.ticket, 1u);
@@ -747,46 +923,26 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(BatchKernelAr
         // ---------------- LU ----------------
         for (int k0 = 0; k0 < n && !abort_flag; k0 += a.b) {
             const int bk = min(a.b, n - k0);
-            factor_step(sm, colstage, A, n, k0, bk, sst);
+            factor_diag(sm, colstage, A, n, k0, bk, sst);
             const int m = n - k0 - bk;
             if (m <= 0) break;
             const int mp = (m + kRowTile - 1) / kRowTile * kRowTile;
             const int np = (m + TN - 1) / TN * TN;
-            const float *Ls = A + (k0 + bk) + (int64_t)k0 * lda;
-            const float *Us = A + k0 + (int64_t)(k0 + bk) * lda;
-            const bool lvec = ((reinterpret_cast<uintptr_t>(Ls) & 15) == 0) && (lda & 3) == 0;
-            if (lvec) {
-                for (int r4 = 4 * threadIdx.x; r4 < mp; r4 += 4 * kBatchThreads) {
-                    if (r4 + 4 <= m) {
-                        stage_rows4(Lst, mp / 128, r4, bk, Ls + r4, lda);
-                    } else {
-                        for (int row = r4; row < r4 + 4 && row < mp; ++row) {
-                            if (row < m)
-                                stage_row(Lst, mp / 128, row, bk,
-                                          [&](int k) { return __ldcg(Ls + row + (int64_t)k * lda); });
-                            else
-                                stage_zero_row(Lst, mp / 128, row, bk);
-                        }
-                    }
-                }
-            } else {
-                for (int row = threadIdx.x; row < mp; row += kBatchThreads) {
-                    if (row < m)
-                        stage_row(Lst, mp / 128, row, bk, [&](int k) { return __ldcg(Ls + row + (int64_t)k * lda); });
-                    else
-                        stage_zero_row(Lst, mp / 128, row, bk);
-                }
-            }
-            const bool rvec = ((reinterpret_cast<uintptr_t>(Us) & 15) == 0) && (lda & 3) == 0;
-            for (int j = threadIdx.x; j < np; j += kBatchThreads) {
-                if (j < m && rvec)
-                    stage_row_contig(Rst, np / 128, j, bk, Us + (int64_t)j * lda);
-                else if (j < m)
-                    stage_row(Rst, np / 128, j, bk, [&](int k) { return __ldcg(Us + k + (int64_t)j * lda); });
-                else
-                    stage_zero_row(Rst, np / 128, j, bk);
-            }
-            asm volatile("fence.proxy.async.global;" ::: "memory");  // staging -> bulk copies
+            const float *D = A + k0 + (int64_t)k0 * lda;
+            float *Ls = A + (k0 + bk) + (int64_t)k0 * lda;
+            float *Us = A + k0 + (int64_t)(k0 + bk) * lda;
+            // L strip, then U strip: W's images in memory, then the tiles
+            prepare_w<true>(ssm, D, lda, bk, Wst);
+            asm volatile("fence.proxy.async;" ::: "memory");  // images and shared memory -> bulk copies
+            __syncthreads();
+            strip_tiles<true>(ssm, sbars, sst8, Ls, lda, m, bk, Wst, Lst, mp / 128, a.dst);
+            prepare_w<false>(ssm, D, lda, bk, Wst + kWBytes);
+            asm volatile("fence.proxy.async;" ::: "memory");
+            __syncthreads();
+            strip_tiles<false>(ssm, sbars, sst8, Us, lda, m, bk, Wst + kWBytes, Rst, np / 128, a.dst);
+            if (abort_flag) break;
+            for (int j = mp + threadIdx.x; j < np; j += kBatchThreads) stage_zero_row(Rst, np / 128, j, bk);
+            asm volatile("fence.proxy.async;" ::: "memory");  // staging and shared memory -> bulk copies
             __syncthreads();
             schur_step<TN>(rg, rs, &abort_flag, A + (k0 + bk) + (int64_t)(k0 + bk) * lda, lda, m, bk, Lst, mp / 128,
                            Rst, np / 128, a.dst);
@@ -843,7 +999,7 @@ struct mxp_batch {
     DevStatus *d_status = nullptr;
     unsigned int *d_ticket = nullptr;
     uint8_t *d_staging = nullptr;
-    int64_t staging_stride = 0, rstage_off = 0;
+    int64_t staging_stride = 0, rstage_off = 0, wstage_off = 0;
     BatchConfig cfg;
     int autotuned = 0;
     // captured launch (captured on a private stream, replayed on the caller's)
@@ -860,13 +1016,20 @@ constexpr int kBatchMaxN = 8192;
 
 size_t ring_bytes(int tile_n, int stages) { return (size_t)stages * (kBlockBytes + (size_t)tile_n * 128); }
 
-constexpr size_t kCbufBytes = 128 * 128 * 4;  // epilogue staging of C
+constexpr size_t kCbufBytes = 128 * 128 * 4;  // one slot of the epilogue's C staging
+constexpr size_t kBatchMaxSmem = 227 * 1024;
+
+// Slots of the C staging: two where they fit beside the operand ring.
+int c_slots(const BatchConfig &c) {
+    return ring_bytes(c.tile_n, c.stages) + 2 * kCbufBytes + 1024 <= kBatchMaxSmem ? 2 : 1;
+}
 
 size_t smem_bytes(const mxp_batch *bt, const BatchConfig &c) {
-    size_t s = ring_bytes(c.tile_n, c.stages) + kCbufBytes;
+    size_t s = ring_bytes(c.tile_n, c.stages) + c_slots(c) * kCbufBytes;
     s = std::max(s, (size_t)16 * bt->nmax + sizeof(float) * kNB * (kNB + 1));  // x, r (FP64) + a 64 x 64 block
     s = std::max(s, kColStageOff + kColStageBytes);
-    s = std::max(s, sizeof(SmemGV));  // the panel's cp.async-staged update tiles
+    s = std::max(s, sizeof(SmemGV));     // the diagonal block's cp.async-staged update tiles
+    s = std::max(s, sizeof(StripSmem));  // the panel strips
     return s + 1024;                          // 1024-byte alignment of the ring
 }
 
@@ -874,7 +1037,7 @@ bool config_ok(const mxp_batch *bt, const BatchConfig &c) {
     if (c.b != 64 && c.b != 128 && c.b != 256) return false;
     if (c.tile_n != 128 && c.tile_n != 256) return false;
     if (c.stages < 2 || c.stages > kMaxStages) return false;
-    return smem_bytes(bt, c) <= 227 * 1024;
+    return smem_bytes(bt, c) <= kBatchMaxSmem;
 }
 
 mxp_status launch_batch(mxp_batch *bt, const BatchConfig &c, int count, const int *d_order, float *A,
@@ -885,6 +1048,7 @@ mxp_status launch_batch(mxp_batch *bt, const BatchConfig &c, int count, const in
     ka.a.count = count;
     ka.a.b = c.b;
     ka.a.stages = c.stages;
+    ka.a.ncbuf = c_slots(c);
     ka.a.maxit = maxit;
     ka.a.A = A;
     ka.a.d = d;
@@ -894,6 +1058,7 @@ mxp_status launch_batch(mxp_batch *bt, const BatchConfig &c, int count, const in
     ka.a.staging = bt->d_staging;
     ka.a.staging_stride = bt->staging_stride;
     ka.a.rstage_off = bt->rstage_off;
+    ka.a.wstage_off = bt->wstage_off;
     ka.a.ticket = bt->d_ticket;
     ka.a.dst = bt->d_status;
     ka.sys_status = bt->d_sys_status;
@@ -1008,7 +1173,8 @@ extern "C" mxp_status mxp_batch_create(int count, const int *h_n, const uint64_t
     // 128, R rows to 256, 256 FP16 per row
     const int64_t lrows = ((int64_t)bt->nmax + 127) / 128 * 128, rrows = ((int64_t)bt->nmax + 255) / 256 * 256;
     bt->rstage_off = lrows * 256 * 2;
-    bt->staging_stride = (bt->rstage_off + rrows * 256 * 2 + 1023) / 1024 * 1024;
+    bt->wstage_off = (bt->rstage_off + rrows * 256 * 2 + 1023) / 1024 * 1024;
+    bt->staging_stride = bt->wstage_off + 2 * kWBytes;
     std::vector<BatchSys> hs(count);
     for (int i = 0; i < count; ++i) hs[i] = BatchSys{h_n[i], 0, h_seed[i], bt->a_off[i], bt->v_off[i]};
     bool ok = cudaMalloc(&bt->d_sys, sizeof(BatchSys) * count) == cudaSuccess &&
