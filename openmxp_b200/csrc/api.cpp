@@ -129,14 +129,13 @@ struct mxp_workspace {
     int inv_blocks = 0;
     float *inv_store = nullptr;
     double *trsv_t = nullptr;             // 4 b doubles
-    cudaEvent_t ev_trsv[4] = {nullptr, nullptr, nullptr, nullptr};  // two-stream refinement solves
     const float *inv_lu = nullptr;        // factor the stored inverses belong to (nullptr: none)
     int inv_n = 0;
     int64_t inv_lda = 0;
     // cooperative diagonal-block factorisation (LU + inverses in one launch)
     int coop = 1;
     float *coop_tmp = nullptr;          // 2 x diag_factor_tmp_floats(b)
-    unsigned int *coop_sync = nullptr;  // grid-barrier counter + abort word
+    unsigned int *coop_sync = nullptr;  // grid-barrier counter + abort word: [0, 2) diagonal block, [8, 10) triangular solves
     void *split_big = nullptr, *split_u = nullptr, *split_l = nullptr;
     // GMRES-IR: basis V ((m+1) x n), Hessenberg H ((m+1) x m), rotations, scalars
     int gm_m = 30;
@@ -207,8 +206,6 @@ extern "C" mxp_status mxp_workspace_destroy(mxp_workspace *ws) {
     if (ws->h_scal) cudaFreeHost(ws->h_scal);
     if (ws->ev_fork) cudaEventDestroy(ws->ev_fork);
     if (ws->ev_join) cudaEventDestroy(ws->ev_join);
-    for (cudaEvent_t e : ws->ev_trsv)
-        if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ws->ev_inv)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ws->ev_ir)
@@ -277,8 +274,6 @@ extern "C" mxp_status mxp_workspace_create(int n, int b, int form, int device, m
              cudaStreamCreateWithPriority(&ws->side, cudaStreamNonBlocking, greatest) == cudaSuccess &&
              cudaEventCreateWithFlags(&ws->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&ws->ev_join, cudaEventDisableTiming) == cudaSuccess;
-        for (int e = 0; e < 4 && ok; ++e)
-            ok = cudaEventCreateWithFlags(&ws->ev_trsv[e], cudaEventDisableTiming) == cudaSuccess;
         for (int e = 0; e < 2 && ok; ++e)
             ok = cudaEventCreateWithFlags(&ws->ev_inv[e], cudaEventDisableTiming) == cudaSuccess;
         for (int e = 0; e < 6 && ok; ++e) ok = cudaEventCreate(&ws->ev_ir[e]) == cudaSuccess;
@@ -940,8 +935,8 @@ static mxp_status lu_solve_ws(mxp_workspace *ws, int n, const float *LU, int64_t
     if (withhold < 0 && ws->trsv_inv && ws->inv_lu && LU == ws->inv_lu && n == ws->inv_n &&
         lda == ws->inv_lda && lu_solve_inv_supported(n, ws->b, LU, lda)) {
         const int64_t bb = (int64_t)ws->b * ws->b;
-        return launch_lu_solve_inv(n, ws->b, LU, lda, ws->inv_store, ws->inv_store + bb, 2 * bb, x, ws->trsv_t, st,
-                                   ws->side, ws->ev_trsv);
+        return launch_lu_solve_inv(n, ws->b, LU, lda, ws->inv_store, ws->inv_store + bb, 2 * bb, x, ws->trsv_t,
+                                   ws->coop_sync + 8, ws->status, st);
     }
     return launch_lu_solve(n, LU, lda, x, ws->flags, ws->status, st, withhold);
 }

@@ -382,108 +382,257 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
 // The diagonal-block products are load-latency bound (a 13 MB triangle at
 // b = 2560): small row tiles give many CTAs, each staging only the part of v
 // its rows use; the trailing products stream the factor at HBM bandwidth.
-constexpr int kIvThreads = 256;
+//
+// All steps of both triangles run in one cooperative launch, separated by grid
+// barriers: a launch per product (four per step on the chain, two streams)
+// spent ~23 us per step at b = 256 on launch gaps.  Per step:
+//   1: t1 = X x_k   2: s = x_k - T t1   3: t2 = t1 + X s
+//   4: x_i -= M(i,k) t2 for the rows of the next block (x_k = t2 with it)
+// and the update of all rows beyond the next block, which only step k+2
+// needs, is done in the barriers' shadow: a CTA that has arrived at barrier
+// 4, 1 and 2 works off a third of its share before it waits, so for a large
+// factor the chain hides behind that stream (HBM-bound) and for a small one
+// the barriers are all there is.  Every row is summed by one CTA in a fixed
+// order and receives its updates in step order.
+constexpr int kIvThreads = 512;
+constexpr int kIvWarps = kIvThreads / 32;
+constexpr int kIvRowsUpd = 32;   // rows per tile of the trailing products (a column: one 128-byte line)
+constexpr int kIvRowsDiag = 8;   // rows per tile on the chain (many CTAs, whole 32-byte sectors)
+constexpr int kIvDepth = 4;      // 16-byte loads in flight per thread, two CTAs per SM
 
-// One CTA: ROWS rows (ROWS/4 quads of four rows, one float4 per column) x
-// 256 / (ROWS/4) column groups (ROWS >= 8: a warp reads whole 32-byte
+// chain vector, bulk vector, the warps' row sums
+size_t trsv_inv_smem(int b) { return (2 * (size_t)b + kIvWarps * kIvRowsUpd) * sizeof(double); }
+
+struct InvSolve {
+    int n, b;
+    const float *LU;
+    int64_t lda;
+    const float *X[2];   // inv(U_00), inv(L_00)
+    int64_t xstride;
+    double *x, *t;       // t: 4 b doubles
+    unsigned int *count; // grid-barrier arrivals (zero at launch)
+    int *abort;
+    DevStatus *dst;
+};
+
+// Grid barrier in two halves.  The waiter gives up after kWaitTimeoutNs, or
+// when another CTA did.
+__device__ __forceinline__ void iv_arrive(const InvSolve &a) {
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.count) : "memory");
+}
+__device__ __forceinline__ bool iv_wait(const InvSolve &a, unsigned &epoch, int where) {
+    __shared__ int ok_sh;
+    epoch += gridDim.x;
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        const unsigned long long t0 = globaltimer_ns();
+        for (unsigned it = 1; (unsigned)ld_acquire(reinterpret_cast<const int *>(a.count)) < epoch; ++it) {
+            if (it & 63u) continue;
+            if (ld_acquire(a.abort)) {
+                ok = 0;
+                break;
+            }
+            if (globaltimer_ns() - t0 > kWaitTimeoutNs) {
+                ok = 0;
+                atomicExch(a.abort, 1);
+                report(a.dst, MXP_TIMEOUT, where, blockIdx.x);
+                break;
+            }
+        }
+        ok_sh = ok;
+    }
+    __syncthreads();
+    return ok_sh != 0;
+}
+
+// One tile: ROWS rows (ROWS/4 quads of four rows, one float4 per column) x
+// kIvThreads / (ROWS/4) column groups (ROWS >= 8: a warp reads whole 32-byte
 // sectors).  M: column-major FP32, ldm % 4 == 0, 16-byte
-// aligned.  v: cols doubles, staged in shared memory.  With sum_i over the
-// mode's entries of row i:
+// aligned.  vs: cols doubles in shared memory, which fill() provides (called
+// when the first loads of M are under way).  With sum_i over the mode's
+// entries of row i:
 //   MODE 0: out[i] = base[i] - sum_j M(i,j) v_j                 (all columns)
 //   MODE 1: out[i] = [base[i] +] v_i + sum_{j<i} M(i,j) v_j      (unit lower inverse)
 //   MODE 2: out[i] = [base[i] +] v_i / T(i,i) + sum_{j>i} M(i,j) v_j  (upper inverse)
 //   MODE 3: out[i] = base[i] - v_i - sum_{j<i} M(i,j) v_j        (v - T v, T unit lower)
 //   MODE 4: out[i] = base[i] - sum_{j>=i} M(i,j) v_j             (v - T v, T upper)
-// T(i,i) is read from tdiag (ld ldt).  CTA 0 also writes copy_dst[0..cols) = v.
-template <int MODE, int ROWS>
-__global__ void __launch_bounds__(kIvThreads)
-trsv_inv_kernel(int rows, int cols, const float *__restrict__ M, int64_t ldm, const double *v,
-                const float *__restrict__ tdiag, int64_t ldt, const double *base, double *out,
-                double *copy_dst) {
+// T(i,i) is read from tdiag (ld ldt).  base and out are data other CTAs write.
+template <int MODE, int ROWS, typename Fill>
+__device__ __forceinline__ void iv_tile(double (*red)[kIvRowsUpd], int cols, const float *__restrict__ M,
+                                        int64_t ldm, int r0, const double *vs,
+                                        Fill fill, const float *__restrict__ tdiag, int64_t ldt, const double *base,
+                                        double *out) {
     constexpr int QUADS = ROWS / 4;
     constexpr int GROUPS = kIvThreads / QUADS;
-    extern __shared__ __align__(16) unsigned char iv_smem[];
-    double *vs = reinterpret_cast<double *>(iv_smem);
-    double(*red)[ROWS + 1] = reinterpret_cast<double(*)[ROWS + 1]>(vs + cols);
-    const int tid = threadIdx.x;
-    const int r0 = blockIdx.x * ROWS;
+    const int tid = threadIdx.x, lane = tid & 31;
     constexpr bool kLow = MODE == 1 || MODE == 3;   // strictly lower entries
     constexpr bool kUpS = MODE == 2;                // strictly upper
     constexpr bool kUpD = MODE == 4;                // upper with the diagonal
-    // the part of v this CTA reads: its rows and the columns they need
-    int s0 = 0, s1 = cols;
-    if (MODE != 0 && r0 < rows) {
-        if (kLow) s1 = min(cols, r0 + ROWS);
-        else s0 = r0;
-    }
-    for (int j = s0 + tid; j < s1; j += kIvThreads) vs[j] = v[j];
-    __syncthreads();
-    if (copy_dst && blockIdx.x == 0)
-        for (int j = tid; j < cols; j += kIvThreads) copy_dst[j] = vs[j];
-    if (r0 >= rows) return;  // a CTA launched only for the copy
     const int q = tid % QUADS, g = tid / QUADS;
     const int ri = r0 + 4 * q;  // first of this thread's four rows
-    // column range the CTA's rows need
+    // column range the tile's rows need
     int jb = 0, je = cols;
     if (kLow) je = min(cols, r0 + ROWS - 1);
     if (kUpS) jb = r0 + 1;
     if (kUpD) jb = r0;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
     const float *mp = M + ri;
-    auto fma4 = [&](float4 m, int j) {
-        const double vj = vs[j];
-        if (MODE == 0) {
-            a0 = __fma_rn((double)m.x, vj, a0);
-            a1 = __fma_rn((double)m.y, vj, a1);
-            a2 = __fma_rn((double)m.z, vj, a2);
-            a3 = __fma_rn((double)m.w, vj, a3);
-        } else {
-            const bool k0 = kLow ? j < ri : (kUpS ? j > ri : j >= ri);
-            const bool k1 = kLow ? j < ri + 1 : (kUpS ? j > ri + 1 : j >= ri + 1);
-            const bool k2 = kLow ? j < ri + 2 : (kUpS ? j > ri + 2 : j >= ri + 2);
-            const bool k3 = kLow ? j < ri + 3 : (kUpS ? j > ri + 3 : j >= ri + 3);
-            a0 = __fma_rn(k0 ? (double)m.x : 0.0, vj, a0);
-            a1 = __fma_rn(k1 ? (double)m.y : 0.0, vj, a1);
-            a2 = __fma_rn(k2 ? (double)m.z : 0.0, vj, a2);
-            a3 = __fma_rn(k3 ? (double)m.w : 0.0, vj, a3);
-        }
+    float4 m[kIvDepth];
+    auto load = [&](int j) {
+#pragma unroll
+        for (int u = 0; u < kIvDepth; ++u)
+            m[u] = j + GROUPS * u < je ? __ldcs(reinterpret_cast<const float4 *>(mp + (int64_t)(j + GROUPS * u) * ldm))
+                                       : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     int j = jb + g;
-    // eight 16-byte loads in flight per thread
-    for (; j + 7 * GROUPS < je; j += 8 * GROUPS) {
-        float4 m[8];
+    load(j);
+    fill();
+    for (; j < je; j += kIvDepth * GROUPS) {
+        float4 c[kIvDepth];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            m[u] = __ldcs(reinterpret_cast<const float4 *>(mp + (int64_t)(j + GROUPS * u) * ldm));
+        for (int u = 0; u < kIvDepth; ++u) c[u] = m[u];
+        const int jn = j + kIvDepth * GROUPS;
+        if (jn < je) load(jn);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) fma4(m[u], j + GROUPS * u);
+        for (int u = 0; u < kIvDepth; ++u) {
+            const int jj = j + GROUPS * u;
+            if (jj >= je) break;
+            const double vj = vs[jj];
+            if (MODE == 0) {
+                a0 = __fma_rn((double)c[u].x, vj, a0);
+                a1 = __fma_rn((double)c[u].y, vj, a1);
+                a2 = __fma_rn((double)c[u].z, vj, a2);
+                a3 = __fma_rn((double)c[u].w, vj, a3);
+            } else {
+                const bool k0 = kLow ? jj < ri : (kUpS ? jj > ri : jj >= ri);
+                const bool k1 = kLow ? jj < ri + 1 : (kUpS ? jj > ri + 1 : jj >= ri + 1);
+                const bool k2 = kLow ? jj < ri + 2 : (kUpS ? jj > ri + 2 : jj >= ri + 2);
+                const bool k3 = kLow ? jj < ri + 3 : (kUpS ? jj > ri + 3 : jj >= ri + 3);
+                a0 = __fma_rn(k0 ? (double)c[u].x : 0.0, vj, a0);
+                a1 = __fma_rn(k1 ? (double)c[u].y : 0.0, vj, a1);
+                a2 = __fma_rn(k2 ? (double)c[u].z : 0.0, vj, a2);
+                a3 = __fma_rn(k3 ? (double)c[u].w : 0.0, vj, a3);
+            }
+        }
     }
-    for (; j < je; j += GROUPS) fma4(__ldcs(reinterpret_cast<const float4 *>(mp + (int64_t)j * ldm)), j);
-    red[g][4 * q + 0] = a0;
-    red[g][4 * q + 1] = a1;
-    red[g][4 * q + 2] = a2;
-    red[g][4 * q + 3] = a3;
+    // sum over the column groups: the warp's by shuffles, the warps' in order
+#pragma unroll
+    for (int o = QUADS; o < 32; o <<= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+        a3 += __shfl_xor_sync(0xffffffffu, a3, o);
+    }
+    __syncthreads();  // the previous tile's sums have been read
+    if (lane < QUADS) {
+        double *rd = &red[tid >> 5][4 * lane];
+        rd[0] = a0;
+        rd[1] = a1;
+        rd[2] = a2;
+        rd[3] = a3;
+    }
     __syncthreads();
     if (tid < ROWS) {
         double s = 0.0;
-#pragma unroll 8
-        for (int c = 0; c < GROUPS; ++c) s += red[c][tid];
+#pragma unroll
+        for (int c = 0; c < kIvWarps; ++c) s += red[c][tid];
         const int i = r0 + tid;
         double y;
-        if (MODE == 0) y = base[i] - s;
+        if (MODE == 0) y = __ldcg(base + i) - s;
         else if (MODE == 1) y = vs[i] + s;
         else if (MODE == 2) y = vs[i] / (double)tdiag[(int64_t)i * (ldt + 1)] + s;
-        else if (MODE == 3) y = base[i] - vs[i] - s;
-        else y = base[i] - s;
-        if ((MODE == 1 || MODE == 2) && base) y += base[i];
+        else if (MODE == 3) y = __ldcg(base + i) - vs[i] - s;
+        else y = __ldcg(base + i) - s;
+        if ((MODE == 1 || MODE == 2) && base) y += __ldcg(base + i);
         out[i] = y;
     }
 }
 
-constexpr int kIvRowsUpd = 32;   // rows per CTA of the trailing products
-constexpr int kIvRowsDiag = 8;   // rows per CTA of the diagonal-block products (b / 8 CTAs)
+// A product with a triangle of the diagonal block: out = ... over b rows, v in
+// global memory (staged in vs: the part the tile's rows use).
+template <int MODE>
+__device__ __forceinline__ void iv_chain(double (*red)[kIvRowsUpd], int b, const float *M, int64_t ldm, const double *v, double *vs,
+                                         const float *tdiag, int64_t ldt, const double *base, double *out) {
+    for (int t = blockIdx.x; t * kIvRowsDiag < b; t += gridDim.x) {
+        const int r0 = t * kIvRowsDiag;
+        auto fill = [&] {
+            constexpr bool low = MODE == 1 || MODE == 3;
+            const int s0 = low ? 0 : r0, s1 = low ? r0 + kIvRowsDiag : b;
+            __syncthreads();  // vs is free
+            for (int j = s0 + threadIdx.x; j < s1; j += kIvThreads) vs[j] = __ldcg(v + j);
+            __syncthreads();
+        };
+        iv_tile<MODE, kIvRowsDiag>(red, b, M, ldm, r0, vs, fill, tdiag, ldt, base, out);
+    }
+}
 
-size_t trsv_inv_smem(int b) { return (size_t)b * sizeof(double) + sizeof(double) * 64 * (kIvRowsUpd + 1); }
+template <bool LOWER>
+__device__ bool iv_triangle(const InvSolve &a, double *vc, double *vb, double (*red)[kIvRowsUpd], unsigned &epoch) {
+    const int n = a.n, b = a.b, nb = n / b;
+    double *t1 = a.t, *sv = a.t + b;
+    const double *none = nullptr;
+    // rows beyond the next block, updated with the last step's t2 (in vb)
+    const float *bulk_m = nullptr;
+    double *bulk_x = nullptr;
+    int bulk_next = 0, bulk_tiles = 0;
+    auto bulk = [&](int parts) {  // 1/parts of what this CTA still has to do
+        const int left = bulk_next < bulk_tiles ? (bulk_tiles - bulk_next + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+        for (int i = (left + parts - 1) / parts; i > 0; --i, bulk_next += gridDim.x)
+            iv_tile<0, kIvRowsUpd>(red, b, bulk_m, a.lda, bulk_next * kIvRowsUpd, vb, [] {}, nullptr, 0, bulk_x, bulk_x);
+    };
+    for (int s = 0; s < nb; ++s) {
+        const int k = LOWER ? s : nb - 1 - s;
+        const int64_t kk = (int64_t)k * b;
+        const float *X = a.X[LOWER ? 1 : 0] + k * a.xstride, *T = a.LU + kk + kk * a.lda;
+        double *xk = a.x + kk, *t2 = a.t + (2 + (s & 1)) * (int64_t)b;
+        iv_chain<LOWER ? 1 : 2>(red, b, X, b, xk, vc, T, a.lda, none, t1);
+        iv_arrive(a);
+        bulk(2);
+        if (!iv_wait(a, epoch, 50)) return false;
+        iv_chain<LOWER ? 3 : 4>(red, b, T, a.lda, t1, vc, T, a.lda, xk, sv);
+        iv_arrive(a);
+        bulk(1);
+        if (!iv_wait(a, epoch, 51)) return false;
+        iv_chain<LOWER ? 1 : 2>(red, b, X, b, sv, vc, T, a.lda, t1, t2);
+        iv_arrive(a);
+        if (!iv_wait(a, epoch, 52)) return false;
+        // t2 for this step's updates, and x_k
+        __syncthreads();
+        for (int j = threadIdx.x; j < b; j += kIvThreads) {
+            const double v = __ldcg(t2 + j);
+            vb[j] = v;
+            if (blockIdx.x == 0) xk[j] = v;
+        }
+        __syncthreads();
+        if (s + 1 < nb) {  // the next block's rows, on the chain
+            const int64_t nx = LOWER ? kk + b : kk - b;
+            for (int t = blockIdx.x; t * kIvRowsDiag < b; t += gridDim.x)
+                iv_tile<0, kIvRowsDiag>(red, b, a.LU + nx + kk * a.lda, a.lda, t * kIvRowsDiag, vb, [] {}, nullptr, 0,
+                                        a.x + nx, a.x + nx);
+        }
+        const int64_t r0 = LOWER ? kk + 2 * (int64_t)b : 0;
+        const int64_t rows = LOWER ? n - r0 : kk - b;
+        bulk_m = a.LU + r0 + kk * a.lda;
+        bulk_x = a.x + r0;
+        bulk_tiles = rows > 0 ? (int)(rows / kIvRowsUpd) : 0;
+        // the CTAs that had no tile on the chain take theirs first
+        bulk_next = (int)gridDim.x - 1 - (int)blockIdx.x;
+        iv_arrive(a);
+        bulk(3);
+        if (!iv_wait(a, epoch, 53)) return false;
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(kIvThreads, 2) trsv_inv_kernel(InvSolve a) {
+    extern __shared__ __align__(16) unsigned char iv_smem[];
+    double *vc = reinterpret_cast<double *>(iv_smem), *vb = vc + a.b;
+    double(*red)[kIvRowsUpd] = reinterpret_cast<double(*)[kIvRowsUpd]>(vb + a.b);
+    unsigned epoch = 0;
+    if (!iv_triangle<true>(a, vc, vb, red, epoch)) return;
+    iv_triangle<false>(a, vc, vb, red, epoch);
+}
 
 // ---------------------------------------------------------------------------
 // norms and vector ops
@@ -589,90 +738,25 @@ bool lu_solve_inv_supported(int n, int b, const float *LU, int64_t lda) {
 }
 
 mxp_status launch_lu_solve_inv(int n, int b, const float *LU, int64_t lda, const float *XU,
-                               const float *XL, int64_t xstride, double *x, double *t, cudaStream_t st,
-                               cudaStream_t side, cudaEvent_t *ev) {
+                               const float *XL, int64_t xstride, double *x, double *t, unsigned int *sync_words,
+                               DevStatus *dst, cudaStream_t st) {
     if (n <= 0) return MXP_OK;
     if (!lu_solve_inv_supported(n, b, LU, lda) || xstride % 4 != 0 ||
         ((reinterpret_cast<uintptr_t>(XU) | reinterpret_cast<uintptr_t>(XL)) & 15u))
         return fail(MXP_INVALID_ARG, "lu_solve_inv: shape or alignment not supported");
-    const int nb = n / b;
     const size_t smem = trsv_inv_smem(b);
-    if (smem > 48 * 1024) {
-        MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel<0, kIvRowsUpd>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel<1, kIvRowsDiag>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel<2, kIvRowsDiag>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel<3, kIvRowsDiag>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel<4, kIvRowsDiag>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel<0, kIvRowsDiag>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
-    double *t1 = t, *sv = t + b, *t2 = t + 2 * (int64_t)b;  // 4 b doubles (t2 double-buffered)
-    const unsigned dg = (unsigned)(b / kIvRowsDiag);
-    auto upd_grid = [](int rows) { return (unsigned)std::max(1, rows / kIvRowsUpd); };
-    if (!side || !ev) return fail(MXP_INVALID_ARG, "lu_solve_inv: needs a second stream and four events");
-    {
-        // Two streams.  The chain that bounds the solve -- the three
-        // diagonal-block products of step s and the update of the next
-        // block's rows -- runs on `side` (high priority); the update of all
-        // rows beyond the next block, which only step s+2 needs, runs on `st`
-        // and overlaps the chain of step s+1.  Every row still receives its
-        // updates in step order (the next-block update of step s waits for
-        // the bulk update of step s-1, which covered that block), so the
-        // result is the same, bit for bit, as with every launch on one stream.
-        // ev[0]: fork / join, ev[1]: t2 of the step ready, ev[2 + s % 2]: bulk update of step s done.
-        for (int tri = 0; tri < 2; ++tri) {
-            const bool lower = tri == 0;
-            MXP_CUDA(cudaEventRecord(ev[0], st));
-            MXP_CUDA(cudaStreamWaitEvent(side, ev[0], 0));
-            int bulk_step[2] = {-1, -1};
-            for (int s = 0; s < nb; ++s) {
-                const int k = lower ? s : nb - 1 - s;
-                const int64_t kk = (int64_t)k * b;
-                const float *X = (lower ? XL : XU) + k * xstride, *T = LU + kk + kk * lda;
-                double *xk = x + kk;
-                double *t2s = t2 + (int64_t)(s & 1) * b;
-                if (s >= 2 && bulk_step[s & 1] == s - 2) MXP_CUDA(cudaStreamWaitEvent(side, ev[2 + (s & 1)], 0));
-                if (lower) {
-                    trsv_inv_kernel<1, kIvRowsDiag><<<dg, kIvThreads, smem, side>>>(b, b, X, b, xk, nullptr, 0, nullptr, t1, nullptr);
-                    MXP_LAUNCHED();
-                    trsv_inv_kernel<3, kIvRowsDiag><<<dg, kIvThreads, smem, side>>>(b, b, T, lda, t1, nullptr, 0, xk, sv, nullptr);
-                    MXP_LAUNCHED();
-                    trsv_inv_kernel<1, kIvRowsDiag><<<dg, kIvThreads, smem, side>>>(b, b, X, b, sv, nullptr, 0, t1, t2s, nullptr);
-                    MXP_LAUNCHED();
-                } else {
-                    trsv_inv_kernel<2, kIvRowsDiag><<<dg, kIvThreads, smem, side>>>(b, b, X, b, xk, T, lda, nullptr, t1, nullptr);
-                    MXP_LAUNCHED();
-                    trsv_inv_kernel<4, kIvRowsDiag><<<dg, kIvThreads, smem, side>>>(b, b, T, lda, t1, nullptr, 0, xk, sv, nullptr);
-                    MXP_LAUNCHED();
-                    trsv_inv_kernel<2, kIvRowsDiag><<<dg, kIvThreads, smem, side>>>(b, b, X, b, sv, T, lda, t1, t2s, nullptr);
-                    MXP_LAUNCHED();
-                }
-                MXP_CUDA(cudaEventRecord(ev[1], side));
-                // rows of the next block (and x_k = t2) on the chain, after the bulk update of step s-1
-                if (s >= 1 && bulk_step[(s - 1) & 1] == s - 1)
-                    MXP_CUDA(cudaStreamWaitEvent(side, ev[2 + ((s - 1) & 1)], 0));
-                const bool has_next = s + 1 < nb;
-                const int64_t nx = lower ? kk + b : kk - b;  // first row of the next block
-                // (on the chain: small row tiles, many CTAs)
-                trsv_inv_kernel<0, kIvRowsDiag><<<has_next ? dg : 1, kIvThreads, smem, side>>>(
-                    has_next ? b : 0, b, LU + (has_next ? nx : 0) + kk * lda, lda, t2s, nullptr, 0,
-                    x + (has_next ? nx : 0), x + (has_next ? nx : 0), xk);
-                MXP_LAUNCHED();
-                // rows beyond the next block
-                const int64_t r0 = lower ? kk + 2 * (int64_t)b : 0;
-                const int rows = (int)(lower ? n - kk - 2 * (int64_t)b : kk - b);
-                if (rows > 0) {
-                    MXP_CUDA(cudaStreamWaitEvent(st, ev[1], 0));
-                    trsv_inv_kernel<0, kIvRowsUpd><<<upd_grid(rows), kIvThreads, smem, st>>>(
-                        rows, b, LU + r0 + kk * lda, lda, t2s, nullptr, 0, x + r0, x + r0, nullptr);
-                    MXP_LAUNCHED();
-                    MXP_CUDA(cudaEventRecord(ev[2 + (s & 1)], st));
-                    bulk_step[s & 1] = s;
-                }
-            }
-            MXP_CUDA(cudaEventRecord(ev[0], side));
-            MXP_CUDA(cudaStreamWaitEvent(st, ev[0], 0));
-        }
-    }
+    MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    MXP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trsv_inv_kernel, kIvThreads, smem));
+    if (per_sm < 1) return fail(MXP_UNSUPPORTED, "lu_solve_inv: kernel cannot be made resident");
+    // as many CTAs as a step has tiles (fewer make the barriers cheaper), all co-resident
+    const int64_t tiles = std::max<int64_t>(b / kIvRowsDiag, n / kIvRowsUpd);
+    const int grid = (int)imin64(tiles, (int64_t)num_sms() * std::min(per_sm, 2));
+    MXP_CUDA(cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), st));
+    InvSolve a{n, b, LU, lda, {XU, XL}, xstride, x, t, sync_words, reinterpret_cast<int *>(sync_words + 1), dst};
+    void *args[] = {&a};
+    MXP_CUDA(cudaLaunchCooperativeKernel((const void *)trsv_inv_kernel, dim3(grid), dim3(kIvThreads), args, smem, st));
+    MXP_LAUNCHED();
     return MXP_OK;
 }
 
