@@ -11,12 +11,14 @@
 // contiguous bytes per column) and keeps the rows' t-th partials, and the CTA
 // reduces them, writes A(i,i) = float(d_i) over the generator's value, and
 // fills its rows of the right-hand side (stream column n).
-// What bounds it is the store of the matrix (n = 61440: 15.1 GB) and, when
-// only d is asked for, the FP64 and conversion pipes.  Separate passes for
-// the elements and for d generated everything twice (n = 61440: 7.1 ms).
-// ROWS = 16 amortises the jump-ahead of a thread's first state and writes 64
-// bytes per column; up to kSmallN, where that would leave SMs without a CTA,
-// ROWS = 4.
+// What bounds it is the store of the matrix (n = 61440: 15.1 GB) and the FP64 and
+// conversion pipes.  Separate passes for the elements and for d generated
+// everything twice.  A thread's ROWS elements of a column are contiguous, but a
+// warp's are 32 columns apart, so a warp exchanges its 32 columns x ROWS rows
+// through shared memory and stores whole sectors, several columns per
+// instruction (16-byte stores to 32 different columns each: n = 61440 7.2 ms).
+// ROWS = 8: whole 32-byte sectors, a CTA per SM from n ~ 1200 on, and 64
+// registers, so that two CTAs share an SM (16 rows spill there).
 #include <algorithm>
 
 #include "mxp_internal.cuh"
@@ -26,7 +28,7 @@ namespace mxp {
 namespace {
 
 constexpr int kGenThreads = 512;   // MATGEM_THREADS of matgen.hpp:7, pinned by the reduction order
-constexpr int kSmallN = 148 * 16 * 2;
+constexpr int kGenRows = 8;
 constexpr int kRedRows = 4;        // rows reduced together in shared memory
 
 template <typename T>
@@ -39,50 +41,71 @@ struct GenArgs {
     double *d, *rowsum, *rhs;
 };
 
+// Dynamic shared memory: a tile per warp, 32 columns of ROWS values (pitch ROWS +
+// 16 bytes: 16-byte accesses without conflicts), and the reduction after them.
+template <typename T, int ROWS>
+constexpr size_t gen_smem() {
+    const size_t tiles = (size_t)kGenThreads * (ROWS * sizeof(T) + 16), red = sizeof(double) * kRedRows * kGenThreads;
+    return tiles > red ? tiles : red;
+}
+
 template <typename T, int ROWS>
 __device__ __forceinline__ void gen_rows(const GenArgs<T> &g, int64_t row0) {
     static_assert(ROWS % kRedRows == 0, "whole reduction groups");
-    __shared__ double sh[kRedRows][kGenThreads];
-    const int t = threadIdx.x, n = g.n;
+    extern __shared__ __align__(16) unsigned char gen_mem[];
+    double(*sh)[kGenThreads] = reinterpret_cast<double(*)[kGenThreads]>(gen_mem);
+    constexpr int V = 16 / sizeof(T), P = ROWS + V;  // values per 16 bytes, tile pitch
+    const int t = threadIdx.x, lane = t & 31, n = g.n;
+    T *tile = reinterpret_cast<T *>(gen_mem) + (size_t)(t - lane) * P;
     const int rows = (int)imin64(ROWS, n - row0);
     const Aff inc1 = lcg_inc1();
     double acc[ROWS];
 #pragma unroll
     for (int q = 0; q < ROWS; ++q) acc[q] = 0.0;
     const bool elements = g.A || g.d || g.rowsum;
-    if (t < n && elements) {
+    if (elements && t - lane < n) {
         // element (row0, t): INC1^(row0 + n*t) = J_n^t o INC1^row0
-        uint64_t s[ROWS];
-        s[0] = aff_apply(aff_pow(g.jn, (uint64_t)t), aff_apply(aff_pow(inc1, (uint64_t)row0), g.s00));
-#pragma unroll
-        for (int q = 1; q < ROWS; ++q) s[q] = aff_apply(inc1, s[q - 1]);
-        constexpr int V = 16 / sizeof(T);
+        uint64_t s0 = aff_apply(aff_pow(g.jn, (uint64_t)t), aff_apply(aff_pow(inc1, (uint64_t)row0), g.s00));
         const bool vec = rows == ROWS && ((reinterpret_cast<uintptr_t>(g.A) | (uintptr_t)(g.lda * sizeof(T))) & 15) == 0;
-        for (int64_t j = t; j < n; j += kGenThreads) {
+        for (int64_t jb = t - lane; jb < n; jb += kGenThreads) {  // the warp's 32 columns
+            const int64_t j = jb + lane;
             const int dq = (int)(j - row0);  // row of the diagonal element, when in 0 .. ROWS - 1
-            T v[ROWS];
+            uint64_t s = s0;
 #pragma unroll
-            for (int q = 0; q < ROWS; ++q) {
-                const double x = lcg_to_double(s[q]);
-                v[q] = static_cast<T>(x);  // float: round to nearest (RandStat::operator float)
-                acc[q] += q == dq ? 0.0 : fabs(x);
-                s[q] = aff_apply(g.j512, s[q]);
-            }
-            if (!g.A) continue;
-            T *col = g.A + j * g.lda + row0;
-            if (vec) {
+            for (int q0 = 0; q0 < ROWS; q0 += V) {
+                T v[V];
 #pragma unroll
-                for (int q = 0; q < ROWS; q += V) {
-                    if constexpr (sizeof(T) == 4)
-                        *reinterpret_cast<float4 *>(col + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-                    else
-                        *reinterpret_cast<double2 *>(col + q) = make_double2(v[q], v[q + 1]);
+                for (int e = 0; e < V; ++e) {
+                    const double x = lcg_to_double(s);
+                    v[e] = static_cast<T>(x);  // float: round to nearest (RandStat::operator float)
+                    // (columns past n add nothing)
+                    acc[q0 + e] += q0 + e == dq || j >= n ? 0.0 : fabs(x);
+                    s = aff_apply(inc1, s);
                 }
-            } else {
-#pragma unroll
-                for (int q = 0; q < ROWS; ++q)
-                    if (q < rows) col[q] = v[q];
+                if (g.A) {
+                    if constexpr (sizeof(T) == 4)
+                        *reinterpret_cast<float4 *>(tile + lane * P + q0) = make_float4(v[0], v[1], v[2], v[3]);
+                    else
+                        *reinterpret_cast<double2 *>(tile + lane * P + q0) = make_double2(v[0], v[1]);
+                }
             }
+            s0 = aff_apply(g.j512, s0);
+            if (!g.A) continue;
+            __syncwarp();
+            constexpr int L = ROWS / V;  // lanes per column
+            if (vec) {
+                const int r = (lane % L) * V;
+#pragma unroll
+                for (int c = lane / L; c < 32; c += 32 / L)
+                    if (jb + c < n)
+                        *reinterpret_cast<float4 *>(g.A + (jb + c) * g.lda + row0 + r) =
+                            *reinterpret_cast<const float4 *>(tile + c * P + r);
+            } else {
+                const int r = lane % ROWS;
+                for (int c = lane / ROWS; c < 32; c += 32 / ROWS)
+                    if (jb + c < n && r < rows) g.A[(jb + c) * g.lda + row0 + r] = tile[c * P + r];
+            }
+            __syncwarp();
         }
     }
     if (g.rhs && t < rows) {
@@ -113,14 +136,14 @@ __device__ __forceinline__ void gen_rows(const GenArgs<T> &g, int64_t row0) {
 }
 
 template <typename T, int ROWS>
-__global__ void __launch_bounds__(kGenThreads) gen_kernel(GenArgs<T> g) {
+__global__ void __launch_bounds__(kGenThreads, 2) gen_kernel(GenArgs<T> g) {
     gen_rows<T, ROWS>(g, (int64_t)blockIdx.x * ROWS);
 }
 
 // Many systems in one launch: blockIdx.y walks the systems, blockIdx.x a system's
 // row bands (those past its order leave).
 template <int ROWS>
-__global__ void __launch_bounds__(kGenThreads)
+__global__ void __launch_bounds__(kGenThreads, 2)
 gen_batch_kernel(const GenSys *sys, int count, float *A, double *d, double *rhs) {
     for (int i = blockIdx.y; i < count; i += gridDim.y) {
         const GenSys S = sys[i];
@@ -142,6 +165,15 @@ gen_batch_kernel(const GenSys *sys, int count, float *A, double *d, double *rhs)
     }
 }
 
+template <typename T, int ROWS>
+mxp_status launch_gen_rows(const GenArgs<T> &g, cudaStream_t st) {
+    const size_t smem = gen_smem<T, ROWS>();
+    MXP_CUDA(cudaFuncSetAttribute(gen_kernel<T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gen_kernel<T, ROWS><<<(unsigned)cdiv(g.n, ROWS), kGenThreads, smem, st>>>(g);
+    MXP_LAUNCHED();
+    return MXP_OK;
+}
+
 template <typename T>
 mxp_status launch_gen(int n, uint64_t seed, int diag_rule, T *A, int64_t lda, double *d, double *rowsum,
                       double *rhs, cudaStream_t st) {
@@ -157,10 +189,7 @@ mxp_status launch_gen(int n, uint64_t seed, int diag_rule, T *A, int64_t lda, do
     g.d = d;
     g.rowsum = rowsum;
     g.rhs = rhs;
-    if (n <= kSmallN) gen_kernel<T, 4><<<(unsigned)cdiv(n, 4), kGenThreads, 0, st>>>(g);
-    else gen_kernel<T, 16><<<(unsigned)cdiv(n, 16), kGenThreads, 0, st>>>(g);
-    MXP_LAUNCHED();
-    return MXP_OK;
+    return launch_gen_rows<T, kGenRows>(g, st);
 }
 
 }  // namespace
@@ -177,8 +206,10 @@ mxp_status launch_matgen(int n, uint64_t seed, int diag_rule, float *A, int64_t 
 mxp_status launch_matgen_batch(int count, const GenSys *sys, int nmax, float *A, double *d, double *rhs,
                                cudaStream_t st) {
     if (count <= 0) return MXP_OK;
-    const dim3 grid((unsigned)cdiv(nmax, 16), (unsigned)std::min(count, 65535));
-    gen_batch_kernel<16><<<grid, kGenThreads, 0, st>>>(sys, count, A, d, rhs);
+    const dim3 grid((unsigned)cdiv(nmax, kGenRows), (unsigned)std::min(count, 65535));
+    const size_t smem = gen_smem<float, kGenRows>();
+    MXP_CUDA(cudaFuncSetAttribute(gen_batch_kernel<kGenRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gen_batch_kernel<kGenRows><<<grid, kGenThreads, smem, st>>>(sys, count, A, d, rhs);
     MXP_LAUNCHED();
     return MXP_OK;
 }
