@@ -666,33 +666,63 @@ __device__ double block_max(double v, double *red) {
 
 // r = b - A x with a_ij regenerated in FP64 from the LCG (otf_gemv,
 // panel_gemv.hpp:13-81) and the diagonal taken from d; x and r in shared memory.
-// Rows are processed two per thread; the sum over j runs in increasing j.
+// The sum over j runs in increasing j.  R rows per thread, 256 apart: their
+// independent chains (LCG step, one subtraction, two FMAs per element) are
+// what hides latency with two warps per scheduler.  The element as in
+// otf_gemv_kernel: both 32-bit halves of the state in the mantissas of
+// biased doubles, the low half's bias (2^52 x_j) and the diagonal's
+// generator value taken out at the end.
+template <int R>
+__device__ __noinline__ void otf_rows(int n, uint64_t s00, Aff jn, const double *__restrict__ d,
+                                      const double *__restrict__ b, const double *xs, double *rs, int i0) {
+    constexpr double kScale = 0x1.fffffffffffffP-65;
+    constexpr double kHiBias = 0x1p84 + 0x1p63;
+    const Aff inc1 = lcg_inc1(), step = aff_pow(inc1, (uint64_t)kBatchThreads);
+    uint64_t s[R];
+    double acc[R], sum = 0.0;
+    s[0] = aff_apply(aff_pow(inc1, (uint64_t)i0), s00);  // element (i0, 0)
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        if (q) s[q] = aff_apply(step, s[q - 1]);
+        acc[q] = 0.0;
+    }
+#pragma unroll 2
+    for (int j = 0; j < n; ++j) {
+        const double xj = xs[j] * kScale;
+        sum += xj;
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const double h = __hiloint2double(0x45300000, (int)((uint32_t)(s[q] >> 32) ^ 0x80000000u)) - kHiBias;
+            acc[q] = __fma_rn(h, xj, acc[q]);
+            acc[q] = __fma_rn(__hiloint2double(0x43300000, (int)(uint32_t)s[q]), xj, acc[q]);
+            s[q] = aff_apply(jn, s[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int i = i0 + q * kBatchThreads;
+        if (i >= n) break;
+        const uint64_t sd = aff_apply(aff_pow(inc1, (uint64_t)i * (uint64_t)(n + 1)), s00);
+        double v = __fma_rn(-0x1p52, sum, acc[q]);
+        v = __fma_rn(-i64_to_double_rn(sd), xs[i] * kScale, v);
+        rs[i] = b[i] - (v + d[i] * xs[i]);
+    }
+}
+
 __device__ void otf_residual(int n, uint64_t seed, const double *__restrict__ d, const double *__restrict__ b,
                              const double *xs, double *rs) {
     const uint64_t s00 = lcg_stat00(seed);
-    const Aff inc1 = lcg_inc1();
-    const Aff jn = aff_pow(inc1, (uint64_t)n);
-    const Aff step2 = aff_pow(inc1, (uint64_t)kBatchThreads);
-    constexpr double kScale = 0x1.fffffffffffffP-65;
-    for (int i0 = threadIdx.x; i0 < n; i0 += 2 * kBatchThreads) {
-        const int i1 = i0 + kBatchThreads;
-        uint64_t s0 = aff_apply(aff_pow(inc1, (uint64_t)i0), s00);  // element (i0, 0)
-        uint64_t s1 = aff_apply(step2, s0);                          // element (i1, 0)
-        double acc0 = 0.0, acc1 = 0.0;
-#pragma unroll 4
-        for (int j = 0; j < n; ++j) {
-            const double xj = xs[j];
-            double v0 = i64_to_double_rn(s0) * kScale;
-            double v1 = i64_to_double_rn(s1) * kScale;
-            v0 = (j == i0) ? 0.0 : v0;
-            v1 = (j == i1) ? 0.0 : v1;
-            acc0 = __fma_rn(v0, xj, acc0);
-            acc1 = __fma_rn(v1, xj, acc1);
-            s0 = aff_apply(jn, s0);
-            s1 = aff_apply(jn, s1);
-        }
-        rs[i0] = b[i0] - (acc0 + d[i0] * xs[i0]);
-        if (i1 < n) rs[i1] = b[i1] - (acc1 + d[i1] * xs[i1]);
+    const Aff jn = aff_pow(lcg_inc1(), (uint64_t)n);
+    // groups of 256 rows in even passes of at most four
+    int left = (n + kBatchThreads - 1) / kBatchThreads, i0 = threadIdx.x;
+    for (int passes = (left + 3) / 4; passes > 0; --passes) {
+        const int r = (left + passes - 1) / passes;
+        if (r == 4) otf_rows<4>(n, s00, jn, d, b, xs, rs, i0);
+        else if (r == 3) otf_rows<3>(n, s00, jn, d, b, xs, rs, i0);
+        else if (r == 2) otf_rows<2>(n, s00, jn, d, b, xs, rs, i0);
+        else otf_rows<1>(n, s00, jn, d, b, xs, rs, i0);
+        left -= r;
+        i0 += r * kBatchThreads;
     }
     __syncthreads();
 }
@@ -744,63 +774,98 @@ __device__ __noinline__ void block_column_update(const float *__restrict__ LU, i
     }
 }
 
-__device__ void lu_solve_shared(int n, const float *__restrict__ LU, double *r, float (*tri)[kNB + 1]) {
+// The 64 x 64 diagonal block in z (lane l: rows l and l + 32), FP64, one warp: four
+// pivots at a time.  Their values go to every lane together, each lane solves
+// the 4 x 4 triangle for itself and applies all four, so the chain meets one
+// exchange per four pivots.  tri[col][row]; rd: reciprocal diagonal (upper).
+constexpr int kTriPitch = kNB + 4;
+template <bool LOWER>
+__device__ __forceinline__ void diag_solve64(const float (*tri)[kTriPitch], const double *rd, double &z0, double &z1) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int q = 0; q < kNB / 4; ++q) {
+        const int kk = LOWER ? 4 * q : kNB - 4 - 4 * q;  // pivots kk .. kk + 3
+        double v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = __shfl_sync(0xffffffffu, kk < 32 ? z0 : z1, (kk + e) & 31);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int i = LOWER ? p : 3 - p;
+            if (!LOWER) v[i] *= rd[kk + i];
+#pragma unroll
+            for (int o = p + 1; o < 4; ++o) {
+                const int e = LOWER ? o : 3 - o;
+                v[e] = __fma_rn(-(double)tri[kk + i][kk + e], v[i], v[e]);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int k = kk + (LOWER ? p : 3 - p);
+            const double vk = v[LOWER ? p : 3 - p];
+            if (LOWER ? lane > k : lane < k) z0 = __fma_rn(-(double)tri[k][lane], vk, z0);
+            if (LOWER ? lane + 32 > k : lane + 32 < k) z1 = __fma_rn(-(double)tri[k][lane + 32], vk, z1);
+        }
+        // the pivots' own rows
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (lane == kk + e) z0 = v[e];
+            if (lane + 32 == kk + e) z1 = v[e];
+        }
+    }
+}
+
+// tri: two 64 x 64 blocks: the next diagonal block arrives under the current one's
+// column update.
+__device__ void lu_solve_shared(int n, const float *__restrict__ LU, double *r, float (*tri)[kNB][kTriPitch],
+                                double *rd) {
     const int64_t lda = n;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = n / kNB;
-    auto load_diag = [&](int c0) {  // tri[col][row] of the 64 x 64 diagonal block, coalesced
-        for (int idx = threadIdx.x; idx < kNB * kNB; idx += kBatchThreads) {
-            const int rr = idx % kNB, cc = idx / kNB;
-            tri[cc][rr] = LU[(int64_t)(c0 + cc) * lda + c0 + rr];
+    const bool vec = aligned16(LU) && (lda & 3) == 0;
+    auto request = [&](int blk, int buf) {  // tri[buf][col][row] of the 64 x 64 diagonal block
+        const float *D = LU + (int64_t)blk * kNB * (lda + 1);
+        if (vec) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int idx = threadIdx.x + kBatchThreads * q, c = idx >> 4, g = (idx & 15) * 4;
+                cp_async16(&tri[buf][c][g], D + (int64_t)c * lda + g, 16);
+            }
+        } else {
+            for (int idx = threadIdx.x; idx < kNB * kNB; idx += kBatchThreads)
+                tri[buf][idx / kNB][idx % kNB] = __ldcg(D + (int64_t)(idx / kNB) * lda + idx % kNB);
         }
-        __syncthreads();
+        cp_async_commit();
     };
-    for (int blk = 0; blk < nb; ++blk) {  // forward, unit lower
-        const int c0 = blk * kNB;
-        load_diag(c0);
+    request(0, 0);
+    for (int s = 0; s < 2 * nb; ++s) {  // forward (unit lower), then backward (upper)
+        const bool lower = s < nb;
+        const int blk = lower ? s : 2 * nb - 1 - s, buf = s & 1, c0 = blk * kNB;
+        cp_async_wait<0>();
+        __syncthreads();
+        if (!lower) {
+            if (threadIdx.x < kNB) rd[threadIdx.x] = 1.0 / (double)tri[buf][threadIdx.x][threadIdx.x];
+            __syncthreads();
+        }
+        if (s + 1 < 2 * nb) request(s + 1 < nb ? s + 1 : 2 * nb - 2 - s, buf ^ 1);
         if (warp == 0) {
             double z0 = r[c0 + lane], z1 = r[c0 + 32 + lane];
-            for (int k = 0; k < kNB; ++k) {
-                const double zk = __shfl_sync(0xffffffffu, k < 32 ? z0 : z1, k & 31);
-                if (lane > k) z0 -= (double)tri[k][lane] * zk;
-                if (lane + 32 > k) z1 -= (double)tri[k][lane + 32] * zk;
-            }
+            if (lower) diag_solve64<true>(tri[buf], rd, z0, z1);
+            else diag_solve64<false>(tri[buf], rd, z0, z1);
             r[c0 + lane] = z0;
             r[c0 + 32 + lane] = z1;
         }
         __syncthreads();
-        block_column_update(LU, lda, c0, r, c0 + kNB, n);
-        __syncthreads();
+        block_column_update(LU, lda, c0, r, lower ? c0 + kNB : 0, lower ? n : c0);
     }
-    for (int blk = nb - 1; blk >= 0; --blk) {  // backward, upper non-unit
-        const int c0 = blk * kNB;
-        load_diag(c0);
-        if (warp == 0) {
-            double z0 = r[c0 + lane], z1 = r[c0 + 32 + lane];
-            for (int k = kNB - 1; k >= 0; --k) {
-                const double rdk = 1.0 / (double)tri[k][k];
-                if (k < 32) {
-                    if (lane == k) z0 = z0 * rdk;
-                } else if (lane + 32 == k) {
-                    z1 = z1 * rdk;
-                }
-                const double zk = __shfl_sync(0xffffffffu, k < 32 ? z0 : z1, k & 31);
-                if (lane < k) z0 -= (double)tri[k][lane] * zk;
-                if (lane + 32 < k) z1 -= (double)tri[k][lane + 32] * zk;
-            }
-            r[c0 + lane] = z0;
-            r[c0 + 32 + lane] = z1;
-        }
-        __syncthreads();
-        block_column_update(LU, lda, c0, r, 0, c0);
-        __syncthreads();
-    }
+    cp_async_wait<0>();
+    __syncthreads();
 }
 
 // Classic refinement of iterative_refinement.hpp:141-171 for one system whose
 // factors are in A; returns the number of corrections applied.
 __device__ void refine_system(int n, uint64_t seed, const float *A, const double *d, const double *b, double *x,
-                              int maxit, double *xs, double *rs, double *red, float (*tri)[kNB + 1], BatchOut *out) {
+                              int maxit, double *xs, double *rs, double *red, float (*tri)[kNB][kTriPitch], double *rd,
+                              BatchOut *out) {
     double mb = 0.0, md = 0.0;
     for (int i = threadIdx.x; i < n; i += kBatchThreads) {
         mb = fmax(mb, fabs(b[i]));
@@ -824,7 +889,7 @@ __device__ void refine_system(int n, uint64_t seed, const float *A, const double
         const double normx = block_max(mx, red);
         hpl = normr / (norma * normx + normb) * 1.0 / ((double)n * eps);
         if (!(hpl < 16.0) && isfinite(hpl)) {
-            lu_solve_shared(n, A, rs, tri);
+            lu_solve_shared(n, A, rs, tri, rd);
             for (int i = threadIdx.x; i < n; i += kBatchThreads) xs[i] += rs[i];
             __syncthreads();
             continue;
@@ -954,7 +1019,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(BatchKernelAr
         double *xs = reinterpret_cast<double *>(smem);
         double *rsv = xs + n;
         refine_system(n, S.seed, A, a.d + S.v_off, a.rhs + S.v_off, a.x + S.v_off, a.maxit, xs, rsv, red,
-                      reinterpret_cast<float(*)[kNB + 1]>(rsv + n), a.out + si);
+                      reinterpret_cast<float(*)[kNB][kTriPitch]>(rsv + n),
+                      reinterpret_cast<double *>(reinterpret_cast<float *>(rsv + n) + 2 * kNB * kTriPitch), a.out + si);
         if (threadIdx.x == 0) a.out[si].info = sst->code == MXP_ZERO_PIVOT ? sst->info0 : 0;
     }
 
@@ -1026,7 +1092,7 @@ int c_slots(const BatchConfig &c) {
 
 size_t smem_bytes(const mxp_batch *bt, const BatchConfig &c) {
     size_t s = ring_bytes(c.tile_n, c.stages) + c_slots(c) * kCbufBytes;
-    s = std::max(s, (size_t)16 * bt->nmax + sizeof(float) * kNB * (kNB + 1));  // x, r (FP64) + a 64 x 64 block
+    s = std::max(s, (size_t)16 * bt->nmax + 2 * sizeof(float) * kNB * kTriPitch + 8 * kNB);  // x, r (FP64) + two 64 x 64 blocks
     s = std::max(s, kColStageOff + kColStageBytes);
     s = std::max(s, sizeof(SmemGV));     // the diagonal block's cp.async-staged update tiles
     s = std::max(s, sizeof(StripSmem));  // the panel strips
