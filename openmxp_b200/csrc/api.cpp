@@ -99,7 +99,7 @@ struct mxp_workspace {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_inv[2] = {nullptr, nullptr};  // fork / join of the two inverse chains
     int *tile_ctr = nullptr;  // shared tile counter of the split trailing pass
-    int *trsm_ctr = nullptr;  // tile counter of the TRSM-by-inverse products (claimed dynamically)
+    int *trsm_ctr = nullptr;  // tile counters of a step's two TRSM-by-inverse products (claimed dynamically)
     int trsm_counter = 1;     // TRSM products take tiles from trsm_ctr (0: static round robin)
     // matrix the refinement's residual regenerates: the LCG matrix of the
     // seed (default) or Higham's matrix with parameters (h_alpha, h_beta)
@@ -136,7 +136,7 @@ struct mxp_workspace {
     int coop = 1;
     float *coop_tmp = nullptr;          // 2 x diag_factor_tmp_floats(b)
     unsigned int *coop_sync = nullptr;  // grid-barrier counter + abort word: [0, 2) diagonal block, [8, 10) triangular solves
-    void *split_big = nullptr, *split_u = nullptr, *split_l = nullptr;
+    void *split_big = nullptr, *split_big2 = nullptr, *split_u = nullptr, *split_l = nullptr;
     // GMRES-IR: basis V ((m+1) x n), Hessenberg H ((m+1) x m), rotations, scalars
     int gm_m = 30;
     double gm_tol = 1e-10;
@@ -170,7 +170,7 @@ static size_t trsm_bytes(int n, int b) {
     const int64_t ldk3 = panel_ldk(b, MXP_FORM_BF16X2);
     const int64_t rows = n > b ? n - b : 1;
     return 2 * (size_t)b * b * 4 + ((size_t)b * b / 4 + 64 * (size_t)b) * 4 +
-           (size_t)(rows + 2 * (int64_t)b) * ldk3 * 2 + 4096 + 2 * diag_factor_tmp_floats(b) * 4 + 256;
+           (size_t)(2 * rows + 2 * (int64_t)b) * ldk3 * 2 + 5120 + 2 * diag_factor_tmp_floats(b) * 4 + 256;
 }
 
 // Stored inverses of the diagonal blocks: 2 x (n / b) blocks of b x b floats.
@@ -261,6 +261,7 @@ extern "C" mxp_status mxp_workspace_create(int n, int b, int form, int device, m
         if (ok) ws->tile_ctr = reinterpret_cast<int *>(ws->coop_sync + 32);
         if (ok) ws->trsm_ctr = reinterpret_cast<int *>(ws->coop_sync + 33);
         ok = ok && (ws->split_big = alloc((size_t)rows * ws->ldk3 * 2 + 1024));
+        ok = ok && (ws->split_big2 = alloc((size_t)rows * ws->ldk3 * 2 + 1024));
         ok = ok && (ws->split_u = alloc((size_t)b * ws->ldk3 * 2 + 1024));
         ok = ok && (ws->split_l = alloc((size_t)b * ws->ldk3 * 2 + 1024));
         ws->inv_blocks = n / b;
@@ -761,8 +762,12 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
                 if (q == MXP_OK) q = launch_tri_inv_lower_unit(b, Akk, lda, ws->tinv_l, b, ws->tinv_tmp, st);
             }
             pt.mark(PH_CAST);
-            if (q == MXP_OK) q = launch_cast_left(bf, m, b, Lcol, lda, ws->split_big, ws->ldk3, nullptr, st);
-            if (q == MXP_OK) q = launch_cast_right(bf, b, b, inv_u(kk), b, ws->split_u, ws->ldk3, nullptr, st);
+            // the operands of both products in one launch
+            const CastJob ops[4] = {{0, m, b, Lcol, lda, ws->split_big, ws->ldk3},
+                                    {1, b, b, inv_u(kk), b, ws->split_u, ws->ldk3},
+                                    {0, b, b, inv_l(kk), b, ws->split_l, ws->ldk3},
+                                    {1, m, b, Urow, lda, ws->split_big2, ws->ldk3}};
+            if (q == MXP_OK) q = launch_casts(bf, ops, 4, st);
             pt.mark(PH_TGEMM);
             // FP8 form: the product's epilogue also writes the E4M3 L panel and
             // its scales into the panel slot (the separate casts below are skipped)
@@ -772,34 +777,28 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
                            Ls + (row0 / 128) * scl + slot * (int64_t)cdiv(b, 128), scl, 0};
             // The triangular K-skip makes the tiles' work uneven (1 to b/256 K blocks):
             // CTAs claim tiles from a counter instead of a static round robin.
-            SchurSched tsched;
+            SchurSched tsched, tschedu;
             tsched.counter = ws->trsm_ctr;
-            const SchurSched *ts = ws->trsm_pair || !ws->trsm_counter ? nullptr : &tsched;
-            if (q == MXP_OK && ts) {
-                cudaError_t e = cudaMemsetAsync(ws->trsm_ctr, 0, sizeof(int), st);
-                if (e != cudaSuccess) q = cuda_fail(e, "panel_lu: TRSM tile counter");
+            tschedu.counter = ws->trsm_ctr + 1;
+            const bool counted = !ws->trsm_pair && ws->trsm_counter;
+            const SchurSched *ts = counted ? &tsched : nullptr, *tsu = counted ? &tschedu : nullptr;
+            if (q == MXP_OK && counted) {
+                cudaError_t e = cudaMemsetAsync(ws->trsm_ctr, 0, 2 * sizeof(int), st);
+                if (e != cudaSuccess) q = cuda_fail(e, "panel_lu: TRSM tile counters");
             }
             if (q == MXP_OK)
                 q = launch_schur(bf, m, b, b, ws->split_big, ws->ldk3, nullptr, ws->split_u, ws->ldk3,
                                  nullptr, Lcol, lda, ws->status, st, /*store=*/1, 0, 0, /*tri=*/1, ws->trsm_pair,
                                  ts, fuse_f8 ? &f8 : nullptr);
-            pt.mark(PH_CAST);
-            if (q == MXP_OK) q = launch_cast_left(bf, b, b, inv_l(kk), b, ws->split_l, ws->ldk3, nullptr, st);
-            if (q == MXP_OK) q = launch_cast_right(bf, m, b, Urow, lda, ws->split_big, ws->ldk3, nullptr, st);
-            pt.mark(PH_TGEMM);
             // ... and the one that forms U12 the E4M3 R panel (transposed layout)
             F8Out f8u{nullptr, 0, nullptr, 0, 0};
             if (fuse_f8)
                 f8u = F8Out{Rb + (row0 * ldk + slot * kp) * es, ldk,
                             Rs + (row0 / 128) * scl + slot * (int64_t)cdiv(b, 128), scl, 1};
-            if (q == MXP_OK && ts) {
-                cudaError_t e = cudaMemsetAsync(ws->trsm_ctr, 0, sizeof(int), st);
-                if (e != cudaSuccess) q = cuda_fail(e, "panel_lu: TRSM tile counter");
-            }
             if (q == MXP_OK)
-                q = launch_schur(bf, b, m, b, ws->split_l, ws->ldk3, nullptr, ws->split_big, ws->ldk3,
+                q = launch_schur(bf, b, m, b, ws->split_l, ws->ldk3, nullptr, ws->split_big2, ws->ldk3,
                                  nullptr, Urow, lda, ws->status, st, /*store=*/1, 0, 0, /*tri=*/2, ws->trsm_pair,
-                                 ts, fuse_f8 ? &f8u : nullptr);
+                                 tsu, fuse_f8 ? &f8u : nullptr);
         } else {
             q = launch_trsm_runn(m, b, Akk, lda, Lcol, lda, st);
             if (q == MXP_OK) q = launch_trsm_llnu(b, m, Akk, lda, Urow, lda, st);
@@ -808,12 +807,17 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
         pt.mark(PH_CAST);
         const int64_t koff = slot * kp;
         const int64_t soff = slot * (int64_t)cdiv(b, 128);
-        if (!fuse_f8)
+        if (!fp8) {
+            const CastJob panels[2] = {{0, m, b, Lcol, lda, Lb + (row0 * ldk + koff) * es, ldk},
+                                       {1, m, b, Urow, lda, Rb + (row0 * ldk + koff) * es, ldk}};
+            q = launch_casts(form, panels, 2, st);
+        } else if (!fuse_f8) {
             q = launch_cast_left(form, m, b, Lcol, lda, Lb + (row0 * ldk + koff) * es, ldk,
-                                 fp8 ? Ls + (row0 / 128) * scl + soff : nullptr, st, scl);
-        if (q == MXP_OK && !fuse_f8)
-            q = launch_cast_right(form, m, b, Urow, lda, Rb + (row0 * ldk + koff) * es, ldk,
-                                  fp8 ? Rs + (row0 / 128) * scl + soff : nullptr, st, scl);
+                                 Ls + (row0 / 128) * scl + soff, st, scl);
+            if (q == MXP_OK)
+                q = launch_cast_right(form, m, b, Urow, lda, Rb + (row0 * ldk + koff) * es, ldk,
+                                      Rs + (row0 / 128) * scl + soff, st, scl);
+        }
         return q;
     };
 

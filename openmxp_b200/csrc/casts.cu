@@ -104,12 +104,9 @@ __device__ __forceinline__ void store16(void *out, int64_t ldk, int64_t row, int
 // L column panel: FP32 m x b column-major -> K-major rows (transpose through
 // shared memory: reads coalesced along rows, writes coalesced along k).
 template <int FORM>
-__global__ void __launch_bounds__(kCastThreads)
-cast_left_kernel(int m, int b, const float *__restrict__ A, int64_t lda, void *out, int64_t ldk,
-                 bool vec) {
-    __shared__ float tile[kTile][kTile + 1];
-    const int i0 = blockIdx.x * kTile;
-    const int k0 = blockIdx.y * kTile;
+__device__ __forceinline__ void cast_left_tile(float (*tile)[kTile + 1], int i0, int k0, int m, int b,
+                                               const float *__restrict__ A, int64_t lda, void *out, int64_t ldk,
+                                               bool vec) {
     const int t = threadIdx.x;
     const int ii = t % kTile;
 #pragma unroll
@@ -141,10 +138,9 @@ cast_left_kernel(int m, int b, const float *__restrict__ A, int64_t lda, void *o
 // K-major rows j (= U^T).  No transpose: column j of U is already contiguous
 // in k.
 template <int FORM>
-__global__ void __launch_bounds__(kCastThreads)
-cast_right_kernel(int m, int b, const float *__restrict__ A, int64_t lda, void *out, int64_t ldk,
-                  bool vec, bool vec_in) {
-    const int64_t gid = (int64_t)blockIdx.x * kCastThreads + threadIdx.x;
+__device__ __forceinline__ void cast_right_block(int64_t blk, int m, int b, const float *__restrict__ A, int64_t lda,
+                                                 void *out, int64_t ldk, bool vec, bool vec_in) {
+    const int64_t gid = blk * kCastThreads + threadIdx.x;
     const int kchunks = (b + 7) / 8;
     const int64_t j = gid / kchunks;
     const int k0 = (int)(gid % kchunks) * 8;
@@ -169,6 +165,32 @@ cast_right_kernel(int m, int b, const float *__restrict__ A, int64_t lda, void *
         const int k = k0 + q;
         if (k < b) store_lowp<FORM>(out, ldk, j, k, b, src[k], true);
     }
+}
+
+// Up to four casts of one form in one launch, side by side: a panel step casts
+// both panels and both inverses before its two products and both panels
+// after them, and for small blocks a launch costs more than its work.
+struct CastJobs {
+    int count;
+    struct Job {
+        CastJob c;
+        bool vec, vec_in;
+        unsigned gx, blocks;  // left: tiles along the rows; blocks of the job
+    } job[kMaxCastJobs];
+};
+
+template <int FORM>
+__global__ void __launch_bounds__(kCastThreads) cast_jobs_kernel(const __grid_constant__ CastJobs jobs) {
+    __shared__ float tile[kTile][kTile + 1];
+    unsigned blk = blockIdx.x;
+    int q = 0;
+    while (q + 1 < jobs.count && blk >= jobs.job[q].blocks) blk -= jobs.job[q++].blocks;
+    const CastJobs::Job &j = jobs.job[q];
+    if (j.c.right)
+        cast_right_block<FORM>(blk, j.c.m, j.c.b, j.c.A, j.c.lda, j.c.out, j.c.ldk, j.vec, j.vec_in);
+    else
+        cast_left_tile<FORM>(tile, (int)(blk % j.gx) * kTile, (int)(blk / j.gx) * kTile, j.c.m, j.c.b, j.c.A, j.c.lda,
+                             j.c.out, j.c.ldk, j.vec);
 }
 
 // ---- FP8 E4M3 with per-128x128-tile power-of-two scales -----------------
@@ -344,56 +366,67 @@ static mxp_status check_cast_args(int form, int m, int b, int64_t lda, int64_t l
     return MXP_OK;
 }
 
+mxp_status launch_casts(int form, const CastJob *jobs, int count, cudaStream_t st) {
+    if (form == MXP_FORM_FP8) return fail(MXP_UNSUPPORTED, "panel casts: FP8 panels are cast one by one");
+    CastJobs js;
+    js.count = 0;
+    int64_t total = 0;
+    for (int q = 0; q < count; ++q) {
+        const CastJob &c = jobs[q];
+        mxp_status s = check_cast_args(form, c.m, c.b, c.lda, c.ldk);
+        if (s != MXP_OK) return s;
+        if (c.m == 0) continue;
+        CastJobs::Job &j = js.job[js.count++];
+        j.c = c;
+        j.vec = vec_ok(c.out, c.ldk, c.b);
+        j.vec_in = (reinterpret_cast<uintptr_t>(c.A) % 16 == 0) && (c.lda % 4 == 0);
+        j.gx = (unsigned)cdiv(c.m, kTile);
+        const int64_t blocks = c.right ? cdiv((int64_t)c.m * ((c.b + 7) / 8), kCastThreads)
+                                       : (int64_t)j.gx * cdiv(c.b, kTile);
+        total += blocks;
+        if (total > INT32_MAX) return fail(MXP_INVALID_ARG, "panel cast: too large");
+        j.blocks = (unsigned)blocks;
+    }
+    if (js.count == 0) return MXP_OK;
+    if (form == MXP_FORM_FP16) cast_jobs_kernel<MXP_FORM_FP16><<<(unsigned)total, kCastThreads, 0, st>>>(js);
+    else if (form == kFormBf16) cast_jobs_kernel<kFormBf16><<<(unsigned)total, kCastThreads, 0, st>>>(js);
+    else cast_jobs_kernel<MXP_FORM_BF16X2><<<(unsigned)total, kCastThreads, 0, st>>>(js);
+    MXP_LAUNCHED();
+    return MXP_OK;
+}
+
 mxp_status launch_cast_left(int form, int m, int b, const float *A, int64_t lda, void *out,
                             int64_t ldk, uint8_t *scales, cudaStream_t st, int sc_ld) {
+    if (form != MXP_FORM_FP8) {
+        const CastJob j{0, m, b, A, lda, out, ldk};
+        return launch_casts(form, &j, 1, st);
+    }
     mxp_status s = check_cast_args(form, m, b, lda, ldk);
     if (s != MXP_OK) return s;
     if (m == 0) return MXP_OK;
-    if (form == MXP_FORM_FP8) {
-        if (!scales) return fail(MXP_INVALID_ARG, "FP8 cast needs a scale buffer");
-        dim3 grid((unsigned)cdiv(m, kF8Tile), (unsigned)cdiv(b, kF8Tile));
-        cast_left_fp8_kernel<<<grid, kCastThreads, 0, st>>>(m, b, A, lda, (uint8_t *)out, ldk,
-                                                            scales, sc_ld > 0 ? sc_ld : (int)grid.y);
-    } else {
-        const bool vec = vec_ok(out, ldk, b);
-        dim3 grid((unsigned)cdiv(m, kTile), (unsigned)cdiv(b, kTile));
-        if (form == MXP_FORM_FP16)
-            cast_left_kernel<MXP_FORM_FP16><<<grid, kCastThreads, 0, st>>>(m, b, A, lda, out, ldk, vec);
-        else if (form == kFormBf16)
-            cast_left_kernel<kFormBf16><<<grid, kCastThreads, 0, st>>>(m, b, A, lda, out, ldk, vec);
-        else
-            cast_left_kernel<MXP_FORM_BF16X2><<<grid, kCastThreads, 0, st>>>(m, b, A, lda, out, ldk, vec);
-    }
+    if (!scales) return fail(MXP_INVALID_ARG, "FP8 cast needs a scale buffer");
+    dim3 grid((unsigned)cdiv(m, kF8Tile), (unsigned)cdiv(b, kF8Tile));
+    cast_left_fp8_kernel<<<grid, kCastThreads, 0, st>>>(m, b, A, lda, (uint8_t *)out, ldk, scales,
+                                                        sc_ld > 0 ? sc_ld : (int)grid.y);
     MXP_LAUNCHED();
     return MXP_OK;
 }
 
 mxp_status launch_cast_right(int form, int m, int b, const float *A, int64_t lda, void *out,
                              int64_t ldk, uint8_t *scales, cudaStream_t st, int sc_ld) {
+    if (form != MXP_FORM_FP8) {
+        const CastJob j{1, m, b, A, lda, out, ldk};
+        return launch_casts(form, &j, 1, st);
+    }
     mxp_status s = check_cast_args(form, m, b, lda, ldk);
     if (s != MXP_OK) return s;
     if (m == 0) return MXP_OK;
-    if (form == MXP_FORM_FP8) {
-        if (!scales) return fail(MXP_INVALID_ARG, "FP8 cast needs a scale buffer");
-        dim3 grid((unsigned)cdiv(m, kF8Tile), (unsigned)cdiv(b, kF8Tile));
-        const bool vec4 = (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (lda % 4 == 0) &&
-                          (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (ldk % 4 == 0);
-        cast_right_fp8_kernel<<<grid, kCastThreads, 0, st>>>(m, b, A, lda, (uint8_t *)out, ldk,
-                                                             scales, sc_ld > 0 ? sc_ld : (int)grid.y, vec4);
-    } else {
-        const bool vec = vec_ok(out, ldk, b);
-        const bool vec_in = (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (lda % 4 == 0);
-        const int64_t threads = (int64_t)m * ((b + 7) / 8);
-        const unsigned blocks = (unsigned)cdiv(threads, kCastThreads);
-        if (form == MXP_FORM_FP16)
-            cast_right_kernel<MXP_FORM_FP16><<<blocks, kCastThreads, 0, st>>>(m, b, A, lda, out, ldk, vec,
-                                                                              vec_in);
-        else if (form == kFormBf16)
-            cast_right_kernel<kFormBf16><<<blocks, kCastThreads, 0, st>>>(m, b, A, lda, out, ldk, vec, vec_in);
-        else
-            cast_right_kernel<MXP_FORM_BF16X2><<<blocks, kCastThreads, 0, st>>>(m, b, A, lda, out,
-                                                                                 ldk, vec, vec_in);
-    }
+    if (!scales) return fail(MXP_INVALID_ARG, "FP8 cast needs a scale buffer");
+    dim3 grid((unsigned)cdiv(m, kF8Tile), (unsigned)cdiv(b, kF8Tile));
+    const bool vec4 = (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (lda % 4 == 0) &&
+                      (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (ldk % 4 == 0);
+    cast_right_fp8_kernel<<<grid, kCastThreads, 0, st>>>(m, b, A, lda, (uint8_t *)out, ldk, scales,
+                                                         sc_ld > 0 ? sc_ld : (int)grid.y, vec4);
     MXP_LAUNCHED();
     return MXP_OK;
 }

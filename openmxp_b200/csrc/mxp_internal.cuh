@@ -214,6 +214,17 @@ mxp_status launch_cast_left(int form, int m, int b, const float *A, int64_t lda,
                             int64_t ldk, uint8_t *scales, cudaStream_t st, int sc_ld = 0);
 mxp_status launch_cast_right(int form, int m, int b, const float *A, int64_t lda, void *out,
                              int64_t ldk, uint8_t *scales, cudaStream_t st, int sc_ld = 0);
+// One cast of launch_casts: an L panel (right = 0) or a U panel, as
+// launch_cast_left / _right; any form but FP8, the same for all jobs.
+constexpr int kMaxCastJobs = 4;
+struct CastJob {
+    int right, m, b;
+    const float *A;
+    int64_t lda;
+    void *out;
+    int64_t ldk;
+};
+mxp_status launch_casts(int form, const CastJob *jobs, int count, cudaStream_t st);
 mxp_status launch_half_left_ref(const float *C, int m, int b, int64_t plda, uint16_t *lp,
                                 int64_t lplda, cudaStream_t st);
 mxp_status launch_half_right_trans_ref(const float *C, int b, int m, int64_t plda, uint16_t *rp,
