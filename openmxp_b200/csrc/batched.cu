@@ -251,6 +251,7 @@ struct StripSmem {                                   // 1024-byte aligned
     uint8_t b[2][2][kWImgBytes];                     // per group, two buffers: W
     float wd[kMaxBk / kSB][kSB][kSB];                // diagonal blocks, wd[.][c][k] = W(k, c)
     float dinv[kMaxBk];
+    float xt[2][2][kRowTile][kSB + 4];               // U strip, per group, two buffers: 16 entries of each vector
 };
 struct StripBars {
     uint64_t *mma;      // per group: the products of one block are done
@@ -330,6 +331,7 @@ __device__ __noinline__ void strip_tiles(StripSmem &s, const StripBars &bars, St
     uint8_t *abuf = s.a[g];
     volatile int *ab = bars.abort_flag;
     bool ok = true;
+    auto group_sync = [&] { asm volatile("barrier.cta.sync %0, 128;" ::"r"(2 + g) : "memory"); };
     auto load_w = [&](int kb) {  // rows kSB (kb + 1) .. bk of image kb (one contiguous range), by the lead thread
         const uint32_t off = (uint32_t)(kb + 1) * kSB * 128, bytes = (uint32_t)bk * 128 - off;
         const uint32_t buf = ss.nb & 1, bar = smem_u32(bars.b + 2 * g + buf);
@@ -341,15 +343,30 @@ __device__ __noinline__ void strip_tiles(StripSmem &s, const StripBars &bars, St
         const bool act = v < m;
         float *vp = LEFT ? S + v : S + (int64_t)v * lda;
         float b[kSB];
+        // U strip: a vector's 16 entries are 64 contiguous bytes, so a warp moves
+        // eight vectors per instruction, whole sectors, through shared memory
+        // (a thread reading its own vector's 16 bytes at a time used half of
+        // every sector twice: U strips took 1.6 x the L strips' time)
+        auto request_x = [&](int kb) {
+            float(*xt)[kSB + 4] = s.xt[g][kb & 1];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = 32 * q + (tg >> 2), c = (tg & 3) * 4;
+                const bool in = rt * kRowTile + r < m;
+                cp_async16(&xt[r][c], in ? S + (int64_t)(rt * kRowTile + r) * lda + kb * kSB + c : S, in ? 16 : 0);
+            }
+            cp_async_commit();
+        };
         auto load_b = [&](int kb) {
             if (LEFT) {
 #pragma unroll
                 for (int k = 0; k < kSB; ++k) b[k] = act ? __ldcg(vp + (int64_t)(kb * kSB + k) * lda) : 0.0f;
-            } else if (vec) {
+            } else if (vec) {  // requested before; from every thread of the group
+                cp_async_wait<0>();
+                group_sync();
 #pragma unroll
                 for (int q = 0; q < kSB / 4; ++q) {
-                    const float4 f = act ? __ldcg(reinterpret_cast<const float4 *>(vp + kb * kSB) + q)
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 f = *reinterpret_cast<const float4 *>(&s.xt[g][kb & 1][tg][4 * q]);
                     b[4 * q] = f.x;
                     b[4 * q + 1] = f.y;
                     b[4 * q + 2] = f.z;
@@ -361,13 +378,15 @@ __device__ __noinline__ void strip_tiles(StripSmem &s, const StripBars &bars, St
             }
         };
         if (lead && nkb > 1) load_w(0);
-        load_b(0);
+        if (!LEFT && vec) request_x(0);
+        else load_b(0);
 #pragma unroll 1
         for (int kb = 0; kb < nkb; ++kb) {
             float x[kSB];
+            if (!LEFT && vec) load_b(kb);
 #pragma unroll
             for (int k = 0; k < kSB; ++k) x[k] = b[k];
-            if (kb + 1 < nkb) load_b(kb + 1);
+            if ((LEFT || !vec) && kb + 1 < nkb) load_b(kb + 1);
             if (kb > 0) {
                 if (!mbar_wait(mma_bar, ss.mma_phase, ab)) {  // raised at once: later waits then return
                     ok = false;
@@ -394,11 +413,17 @@ __device__ __noinline__ void strip_tiles(StripSmem &s, const StripBars &bars, St
                 }
                 if (LEFT) x[c] *= s.dinv[kb * kSB + c];
             }
+            if (!LEFT && vec) {
+#pragma unroll
+                for (int q = 0; q < kSB / 4; ++q)
+                    *reinterpret_cast<float4 *>(&s.xt[g][kb & 1][tg][4 * q]) =
+                        make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+            }
             if (kb + 1 < nkb) {
                 store_split_row(abuf, tg, x);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 tc_fence_before();
-                asm volatile("barrier.cta.sync %0, 128;" ::"r"(2 + g) : "memory");
+                group_sync();
                 const uint32_t buf = ss.nb & 1, bphase = (ss.nb >> 1) & 1u;
                 ++ss.nb;
                 if (lead) {
@@ -424,17 +449,24 @@ __device__ __noinline__ void strip_tiles(StripSmem &s, const StripBars &bars, St
                     }
                 }
                 __syncwarp();
+                // (the other buffer's vectors were stored before the barrier above)
+                if (!LEFT && vec) request_x(kb + 1);
+            } else if (!LEFT && vec) {
+                group_sync();
             }
             // X in FP32 and its FP16 rounding (padding vectors: zero rows), under the products
-            if (act) {
+            if (!LEFT && vec) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int r = 32 * q + (tg >> 2), c = (tg & 3) * 4;
+                    if (rt * kRowTile + r < m)
+                        *reinterpret_cast<float4 *>(S + (int64_t)(rt * kRowTile + r) * lda + kb * kSB + c) =
+                            *reinterpret_cast<const float4 *>(&s.xt[g][kb & 1][r][c]);
+                }
+            } else if (act) {
                 if (LEFT) {
 #pragma unroll
                     for (int k = 0; k < kSB; ++k) vp[(int64_t)(kb * kSB + k) * lda] = x[k];
-                } else if (vec) {
-#pragma unroll
-                    for (int q = 0; q < kSB / 4; ++q)
-                        reinterpret_cast<float4 *>(vp + kb * kSB)[q] =
-                            make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
                 } else {
 #pragma unroll
                     for (int k = 0; k < kSB; ++k) vp[kb * kSB + k] = x[k];
@@ -451,6 +483,7 @@ __device__ __noinline__ void strip_tiles(StripSmem &s, const StripBars &bars, St
                 *reinterpret_cast<uint4 *>(blk + sw128_offset(tg, (kb & 3) * 2 + h)) = q;
             }
         }
+        if (!LEFT && vec) group_sync();  // both buffers have been stored
     }
     if (!ok && lead) report(dst, MXP_TIMEOUT, 34, blockIdx.x);
     __syncthreads();
