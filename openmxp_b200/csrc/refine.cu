@@ -253,31 +253,35 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
 #pragma unroll
         for (int cc = 0; cc < 16; ++cc) d[cc] = (row_ok && cc < clen) ? col[cc * lda] : 0.0f;
     };
-    // Flags are polled by lane 0 of each warp only (every thread spinning on the
-    // same lines slows the producer's release) and the outcome is shared by a
-    // shuffle; the warp barrier orders the lanes' later loads after the acquire.
-    const bool lead = (tid & 31) == 0;
-    auto wait_flag = [&](int b) -> bool {
-        int ok = 1;
-        if (lead) {
+    // One thread of the CTA polls (the others wait at the CTA barrier, which
+    // orders their later loads after its acquire), and a block whose turn is
+    // far off sleeps between polls: every CTA's warps spinning on the few lines
+    // that hold the flags held back the one store the chain waits for.
+    __shared__ int s_seen;
+    auto wait_flag = [&](int b) -> bool {  // all threads; ends with a barrier
+        if (tid == 0) {
+            int ok = 1;
+            const int far = min(32, max(0, (LOWER ? rb - b : b - rb) - 3));
             const unsigned long long t0 = globaltimer_ns();
             uint32_t it = 0;
             while (!ld_acquire(&flags[b])) {
+                if (far) __nanosleep(100 * far);
                 if ((++it & 63u) == 0u && globaltimer_ns() - t0 > kWaitTimeoutNs) {
                     ok = 0;
                     break;
                 }
             }
+            s_seen = ok;
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        __syncwarp();
-        return ok != 0;
+        __syncthreads();
+        return s_seen != 0;
     };
     auto probe_flag = [&](int b) -> bool {
-        int v = lead ? ld_acquire(&flags[b]) : 0;
-        v = __shfl_sync(0xffffffffu, v, 0);
-        __syncwarp();
-        return v != 0;
+        if (tid == 0) s_seen = ld_acquire(&flags[b]);
+        __syncthreads();
+        const bool seen = s_seen != 0;
+        __syncthreads();  // s_seen is written again
+        return seen;
     };
     // The x of the streamed column blocks is staged in shared memory kXChunk
     // blocks at a time (one coalesced load per thread and one barrier per
@@ -340,7 +344,7 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
     w += __shfl_xor_sync(0xffffffffu, w, 1);
     w += __shfl_xor_sync(0xffffffffu, w, 2);
     // ---- the chain link: x_b = w - P x_adj ----
-    if (has_adj && !timed_out) {
+    if (has_adj && !timed_out) {  // (the same in every thread)
         timed_out = !wait_flag(adj);
         const int64_t c0 = (int64_t)adj * kRB + ph * 16;
         const int clen = (int)imin64(16, n - c0);
@@ -356,8 +360,7 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
     }
     if (timed_out) report(dst, MXP_TIMEOUT, 10 + (LOWER ? 0 : 1), rb);
     if (ph == 0 && pi < nrows) __stcg(x + row0 + pi, w);
-    __threadfence();
-    __syncthreads();
+    __syncthreads();  // the release below covers the CTA's stores
     // published even after a timeout, so successors never stall; `withhold` (a
     // test of the bounded waits) leaves one block's flag unset
     if (tid == 0 && rb != withhold) st_release(&flags[rb], 1);
@@ -747,6 +750,8 @@ mxp_status launch_lu_solve_inv(int n, int b, const float *LU, int64_t lda, const
     if (!lu_solve_inv_supported(n, b, LU, lda) || xstride % 4 != 0 ||
         ((reinterpret_cast<uintptr_t>(XU) | reinterpret_cast<uintptr_t>(XL)) & 15u))
         return fail(MXP_INVALID_ARG, "lu_solve_inv: shape or alignment not supported");
+    InvSolve a{n, b, LU, lda, {XU, XL}, xstride, x, t, sync_words, reinterpret_cast<int *>(sync_words + 1), dst};
+    void *args[] = {&a};
     const size_t smem = trsv_inv_smem(b);
     MXP_CUDA(cudaFuncSetAttribute(trsv_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
@@ -756,8 +761,6 @@ mxp_status launch_lu_solve_inv(int n, int b, const float *LU, int64_t lda, const
     const int64_t tiles = std::max<int64_t>(b / kIvRowsDiag, n / kIvRowsUpd);
     const int grid = (int)imin64(tiles, (int64_t)num_sms() * std::min(per_sm, 2));
     MXP_CUDA(cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), st));
-    InvSolve a{n, b, LU, lda, {XU, XL}, xstride, x, t, sync_words, reinterpret_cast<int *>(sync_words + 1), dst};
-    void *args[] = {&a};
     MXP_CUDA(cudaLaunchCooperativeKernel((const void *)trsv_inv_kernel, dim3(grid), dim3(kIvThreads), args, smem, st));
     MXP_LAUNCHED();
     return MXP_OK;
