@@ -31,11 +31,13 @@ constexpr int kGenThreads = 512;   // MATGEM_THREADS of matgen.hpp:7, pinned by 
 constexpr int kGenRows = 8;
 constexpr int kRedRows = 4;        // rows reduced together in shared memory
 
+constexpr int kJumps = 31;         // powers J_n^(2^i) of the column jump
+
 template <typename T>
 struct GenArgs {
     int n, diag_rule;
     uint64_t s00;
-    Aff jn, j512;      // jumps of one column and of 512 columns
+    Aff jn;            // jump of one column
     T *A;              // may be null, like d, rowsum and rhs
     int64_t lda;
     double *d, *rowsum, *rhs;
@@ -51,6 +53,7 @@ constexpr size_t gen_smem() {
 
 template <typename T, int ROWS>
 __device__ __forceinline__ void gen_rows(const GenArgs<T> &g, int64_t row0) {
+    static_assert(kGenThreads == 512, "jp[9] is the step of a thread");
     static_assert(ROWS % kRedRows == 0, "whole reduction groups");
     extern __shared__ __align__(16) unsigned char gen_mem[];
     double(*sh)[kGenThreads] = reinterpret_cast<double(*)[kGenThreads]>(gen_mem);
@@ -63,9 +66,29 @@ __device__ __forceinline__ void gen_rows(const GenArgs<T> &g, int64_t row0) {
 #pragma unroll
     for (int q = 0; q < ROWS; ++q) acc[q] = 0.0;
     const bool elements = g.A || g.d || g.rowsum;
+    // element (row0, c): J_n^c o INC1^row0 of the seed's state, from powers of the
+    // two jumps made once per CTA (all of them commute): a jump-ahead per thread by
+    // squaring took as long as a small system's elements
+    __shared__ Aff jp[kJumps];
+    __shared__ uint64_t base_sh;
+    if (t == 0) {
+        Aff f = g.jn;
+        for (int i = 0; i < kJumps && ((n >> i) || i < 10); ++i) {
+            jp[i] = f;
+            f = aff_mul(f, f);
+        }
+    } else if (t == 32) {
+        base_sh = aff_apply(aff_pow(inc1, (uint64_t)row0), g.s00);
+    }
+    __syncthreads();
+    auto element = [&](uint64_t s, unsigned c) {  // state of (row, c) from that of (row, 0)
+        for (int i = 0; c; ++i, c >>= 1)
+            if (c & 1u) s = aff_apply(jp[i], s);
+        return s;
+    };
     if (elements && t - lane < n) {
-        // element (row0, t): INC1^(row0 + n*t) = J_n^t o INC1^row0
-        uint64_t s0 = aff_apply(aff_pow(g.jn, (uint64_t)t), aff_apply(aff_pow(inc1, (uint64_t)row0), g.s00));
+        const Aff j512 = jp[9];
+        uint64_t s0 = element(base_sh, (unsigned)t);
         const bool vec = rows == ROWS && ((reinterpret_cast<uintptr_t>(g.A) | (uintptr_t)(g.lda * sizeof(T))) & 15) == 0;
         for (int64_t jb = t - lane; jb < n; jb += kGenThreads) {  // the warp's 32 columns
             const int64_t j = jb + lane;
@@ -89,7 +112,7 @@ __device__ __forceinline__ void gen_rows(const GenArgs<T> &g, int64_t row0) {
                         *reinterpret_cast<double2 *>(tile + lane * P + q0) = make_double2(v[0], v[1]);
                 }
             }
-            s0 = aff_apply(g.j512, s0);
+            s0 = aff_apply(j512, s0);
             if (!g.A) continue;
             __syncwarp();
             constexpr int L = ROWS / V;  // lanes per column
@@ -109,7 +132,8 @@ __device__ __forceinline__ void gen_rows(const GenArgs<T> &g, int64_t row0) {
         }
     }
     if (g.rhs && t < rows) {
-        const uint64_t s = aff_apply(aff_pow(inc1, (uint64_t)(row0 + t) + (uint64_t)n * (uint64_t)n), g.s00);
+        uint64_t s = element(base_sh, (unsigned)n);
+        for (int q = 0; q < t; ++q) s = aff_apply(inc1, s);
         g.rhs[row0 + t] = lcg_to_double(s);
     }
     if (!elements) return;
@@ -154,7 +178,6 @@ gen_batch_kernel(const GenSys *sys, int count, float *A, double *d, double *rhs)
         g.diag_rule = MXP_DIAG_ROWSUM;
         g.s00 = lcg_stat00(S.seed);
         g.jn = aff_pow(lcg_inc1(), (uint64_t)S.n);
-        g.j512 = aff_pow(g.jn, kGenThreads);
         g.A = A + S.a_off;
         g.lda = S.n;
         g.d = d + S.v_off;
@@ -183,7 +206,6 @@ mxp_status launch_gen(int n, uint64_t seed, int diag_rule, T *A, int64_t lda, do
     g.diag_rule = diag_rule;
     g.s00 = lcg_stat00(seed);
     g.jn = aff_pow(lcg_inc1(), (uint64_t)n);
-    g.j512 = aff_pow(g.jn, kGenThreads);
     g.A = A;
     g.lda = lda;
     g.d = d;
