@@ -403,8 +403,8 @@ constexpr int kIvRowsUpd = 32;   // rows per tile of the trailing products (a co
 constexpr int kIvRowsDiag = 8;   // rows per tile on the chain (many CTAs, whole 32-byte sectors)
 constexpr int kIvDepth = 4;      // 16-byte loads in flight per thread, two CTAs per SM
 
-// chain vector, bulk vector, the warps' row sums
-size_t trsv_inv_smem(int b) { return (2 * (size_t)b + kIvWarps * kIvRowsUpd) * sizeof(double); }
+// bulk vector, the warps' row sums
+size_t trsv_inv_smem(int b) { return ((size_t)b + kIvWarps * kIvRowsUpd) * sizeof(double); }
 
 struct InvSolve {
     int n, b;
@@ -452,19 +452,20 @@ __device__ __forceinline__ bool iv_wait(const InvSolve &a, unsigned &epoch, int 
 // One tile: ROWS rows (ROWS/4 quads of four rows, one float4 per column) x
 // kIvThreads / (ROWS/4) column groups (ROWS >= 8: a warp reads whole 32-byte
 // sectors).  M: column-major FP32, ldm % 4 == 0, 16-byte
-// aligned.  vs: cols doubles in shared memory, which fill() provides (called
-// when the first loads of M are under way).  With sum_i over the mode's
-// entries of row i:
+// aligned.  vs: cols doubles; VG: in global memory (written by other CTAs), else
+// shared.  ready() is called when the first loads of M are under way and
+// returns when vs may be read (the chain waits for its barrier there).  With
+// sum_i over the mode's entries of row i:
 //   MODE 0: out[i] = base[i] - sum_j M(i,j) v_j                 (all columns)
 //   MODE 1: out[i] = [base[i] +] v_i + sum_{j<i} M(i,j) v_j      (unit lower inverse)
 //   MODE 2: out[i] = [base[i] +] v_i / T(i,i) + sum_{j>i} M(i,j) v_j  (upper inverse)
 //   MODE 3: out[i] = base[i] - v_i - sum_{j<i} M(i,j) v_j        (v - T v, T unit lower)
 //   MODE 4: out[i] = base[i] - sum_{j>=i} M(i,j) v_j             (v - T v, T upper)
 // T(i,i) is read from tdiag (ld ldt).  base and out are data other CTAs write.
-template <int MODE, int ROWS, typename Fill>
+template <int MODE, int ROWS, bool VG, typename Ready>
 __device__ __forceinline__ void iv_tile(double (*red)[kIvRowsUpd], int cols, const float *__restrict__ M,
                                         int64_t ldm, int r0, const double *vs,
-                                        Fill fill, const float *__restrict__ tdiag, int64_t ldt, const double *base,
+                                        Ready ready, const float *__restrict__ tdiag, int64_t ldt, const double *base,
                                         double *out) {
     constexpr int QUADS = ROWS / 4;
     constexpr int GROUPS = kIvThreads / QUADS;
@@ -490,18 +491,25 @@ __device__ __forceinline__ void iv_tile(double (*red)[kIvRowsUpd], int cols, con
     };
     int j = jb + g;
     load(j);
-    fill();
+    ready();
+    auto value = [&](int q) { return VG ? __ldcg(vs + q) : vs[q]; };
     for (; j < je; j += kIvDepth * GROUPS) {
         float4 c[kIvDepth];
+        double v[VG ? kIvDepth : 1];
 #pragma unroll
-        for (int u = 0; u < kIvDepth; ++u) c[u] = m[u];
+        for (int u = 0; u < kIvDepth; ++u) {
+            c[u] = m[u];
+            if constexpr (VG) v[u] = j + GROUPS * u < je ? value(j + GROUPS * u) : 0.0;
+        }
         const int jn = j + kIvDepth * GROUPS;
-        if (jn < je) load(jn);
+        if (!VG && jn < je) load(jn);
 #pragma unroll
         for (int u = 0; u < kIvDepth; ++u) {
             const int jj = j + GROUPS * u;
             if (jj >= je) break;
-            const double vj = vs[jj];
+            double vj;
+            if constexpr (VG) vj = v[u];
+            else vj = vs[jj];
             if (MODE == 0) {
                 a0 = __fma_rn((double)c[u].x, vj, a0);
                 a1 = __fma_rn((double)c[u].y, vj, a1);
@@ -518,6 +526,7 @@ __device__ __forceinline__ void iv_tile(double (*red)[kIvRowsUpd], int cols, con
                 a3 = __fma_rn(k3 ? (double)c[u].w : 0.0, vj, a3);
             }
         }
+        if (VG && jn < je) load(jn);  // (the values of v take the registers a second batch would)
     }
     // sum over the column groups: the warp's by shuffles, the warps' in order
 #pragma unroll
@@ -543,38 +552,41 @@ __device__ __forceinline__ void iv_tile(double (*red)[kIvRowsUpd], int cols, con
         const int i = r0 + tid;
         double y;
         if (MODE == 0) y = __ldcg(base + i) - s;
-        else if (MODE == 1) y = vs[i] + s;
-        else if (MODE == 2) y = vs[i] / (double)tdiag[(int64_t)i * (ldt + 1)] + s;
-        else if (MODE == 3) y = __ldcg(base + i) - vs[i] - s;
+        else if (MODE == 1) y = value(i) + s;
+        else if (MODE == 2) y = value(i) / (double)tdiag[(int64_t)i * (ldt + 1)] + s;
+        else if (MODE == 3) y = __ldcg(base + i) - value(i) - s;
         else y = __ldcg(base + i) - s;
         if ((MODE == 1 || MODE == 2) && base) y += __ldcg(base + i);
         out[i] = y;
     }
 }
 
-// A product with a triangle of the diagonal block: out = ... over b rows, v in
-// global memory (staged in vs: the part the tile's rows use).
-template <int MODE>
-__device__ __forceinline__ void iv_chain(double (*red)[kIvRowsUpd], int b, const float *M, int64_t ldm, const double *v, double *vs,
-                                         const float *tdiag, int64_t ldt, const double *base, double *out) {
-    for (int t = blockIdx.x; t * kIvRowsDiag < b; t += gridDim.x) {
-        const int r0 = t * kIvRowsDiag;
-        auto fill = [&] {
-            constexpr bool low = MODE == 1 || MODE == 3;
-            const int s0 = low ? 0 : r0, s1 = low ? r0 + kIvRowsDiag : b;
-            __syncthreads();  // vs is free
-            for (int j = s0 + threadIdx.x; j < s1; j += kIvThreads) vs[j] = __ldcg(v + j);
-            __syncthreads();
-        };
-        iv_tile<MODE, kIvRowsDiag>(red, b, M, ldm, r0, vs, fill, tdiag, ldt, base, out);
+// A product with a triangle of the diagonal block: out = ... over b rows.  wait():
+// the barrier the product's vectors are complete after, called once, with the
+// first tile's loads of M under way.
+template <int MODE, typename Wait>
+__device__ __forceinline__ void iv_chain(double (*red)[kIvRowsUpd], int b, const float *M, int64_t ldm,
+                                         const double *v, const float *tdiag, int64_t ldt, const double *base,
+                                         double *out, Wait wait) {
+    int t = blockIdx.x;
+    if (t * kIvRowsDiag >= b) {
+        wait();
+        return;
     }
+    iv_tile<MODE, kIvRowsDiag, true>(red, b, M, ldm, t * kIvRowsDiag, v, wait, tdiag, ldt, base, out);
+    for (t += gridDim.x; t * kIvRowsDiag < b; t += gridDim.x)
+        iv_tile<MODE, kIvRowsDiag, true>(red, b, M, ldm, t * kIvRowsDiag, v, [] {}, tdiag, ldt, base, out);
 }
 
+// Both halves of a step's barriers are apart: a CTA arrives, works off a share of
+// the bulk update, requests its part of the next product's matrix and then
+// waits.  ok: cleared when a wait gave up (the CTA then leaves at the step's end).
 template <bool LOWER>
-__device__ bool iv_triangle(const InvSolve &a, double *vc, double *vb, double (*red)[kIvRowsUpd], unsigned &epoch) {
+__device__ bool iv_triangle(const InvSolve &a, double *vb, double (*red)[kIvRowsUpd], unsigned &epoch) {
     const int n = a.n, b = a.b, nb = n / b;
     double *t1 = a.t, *sv = a.t + b;
     const double *none = nullptr;
+    bool ok = true;
     // rows beyond the next block, updated with the last step's t2 (in vb)
     const float *bulk_m = nullptr;
     double *bulk_x = nullptr;
@@ -582,37 +594,47 @@ __device__ bool iv_triangle(const InvSolve &a, double *vc, double *vb, double (*
     auto bulk = [&](int parts) {  // 1/parts of what this CTA still has to do
         const int left = bulk_next < bulk_tiles ? (bulk_tiles - bulk_next + (int)gridDim.x - 1) / (int)gridDim.x : 0;
         for (int i = (left + parts - 1) / parts; i > 0; --i, bulk_next += gridDim.x)
-            iv_tile<0, kIvRowsUpd>(red, b, bulk_m, a.lda, bulk_next * kIvRowsUpd, vb, [] {}, nullptr, 0, bulk_x, bulk_x);
+            iv_tile<0, kIvRowsUpd, false>(red, b, bulk_m, a.lda, bulk_next * kIvRowsUpd, vb, [] {}, nullptr, 0, bulk_x,
+                                          bulk_x);
     };
+    auto wait = [&](int where) { ok = iv_wait(a, epoch, where) && ok; };
     for (int s = 0; s < nb; ++s) {
         const int k = LOWER ? s : nb - 1 - s;
         const int64_t kk = (int64_t)k * b;
         const float *X = a.X[LOWER ? 1 : 0] + k * a.xstride, *T = a.LU + kk + kk * a.lda;
         double *xk = a.x + kk, *t2 = a.t + (2 + (s & 1)) * (int64_t)b;
-        iv_chain<LOWER ? 1 : 2>(red, b, X, b, xk, vc, T, a.lda, none, t1);
+        // (the first step's x is complete at launch, or after the last triangle's final barrier)
+        iv_chain<LOWER ? 1 : 2>(red, b, X, b, xk, T, a.lda, none, t1, [&] {
+            if (s > 0) wait(53);
+        });
         iv_arrive(a);
         bulk(2);
-        if (!iv_wait(a, epoch, 50)) return false;
-        iv_chain<LOWER ? 3 : 4>(red, b, T, a.lda, t1, vc, T, a.lda, xk, sv);
+        iv_chain<LOWER ? 3 : 4>(red, b, T, a.lda, t1, T, a.lda, xk, sv, [&] { wait(50); });
         iv_arrive(a);
         bulk(1);
-        if (!iv_wait(a, epoch, 51)) return false;
-        iv_chain<LOWER ? 1 : 2>(red, b, X, b, sv, vc, T, a.lda, t1, t2);
+        iv_chain<LOWER ? 1 : 2>(red, b, X, b, sv, T, a.lda, t1, t2, [&] { wait(51); });
         iv_arrive(a);
-        if (!iv_wait(a, epoch, 52)) return false;
-        // t2 for this step's updates, and x_k
-        __syncthreads();
-        for (int j = threadIdx.x; j < b; j += kIvThreads) {
-            const double v = __ldcg(t2 + j);
-            vb[j] = v;
-            if (blockIdx.x == 0) xk[j] = v;
-        }
-        __syncthreads();
-        if (s + 1 < nb) {  // the next block's rows, on the chain
-            const int64_t nx = LOWER ? kk + b : kk - b;
-            for (int t = blockIdx.x; t * kIvRowsDiag < b; t += gridDim.x)
-                iv_tile<0, kIvRowsDiag>(red, b, a.LU + nx + kk * a.lda, a.lda, t * kIvRowsDiag, vb, [] {}, nullptr, 0,
-                                        a.x + nx, a.x + nx);
+        // the next block's rows, on the chain; t2 goes to vb for this step's updates, and is x_k
+        auto take = [&] {
+            wait(52);
+            for (int j = threadIdx.x; j < b; j += kIvThreads) {
+                const double v = __ldcg(t2 + j);
+                vb[j] = v;
+                if (blockIdx.x == 0) xk[j] = v;
+            }
+            __syncthreads();
+        };
+        int t = blockIdx.x;
+        const bool next = s + 1 < nb;
+        const int64_t nx = next ? (LOWER ? kk + b : kk - b) : 0;
+        const float *Mn = a.LU + nx + kk * a.lda;
+        if (next && t * kIvRowsDiag < b) {
+            iv_tile<0, kIvRowsDiag, false>(red, b, Mn, a.lda, t * kIvRowsDiag, vb, take, nullptr, 0, a.x + nx, a.x + nx);
+            for (t += gridDim.x; t * kIvRowsDiag < b; t += gridDim.x)
+                iv_tile<0, kIvRowsDiag, false>(red, b, Mn, a.lda, t * kIvRowsDiag, vb, [] {}, nullptr, 0, a.x + nx,
+                                               a.x + nx);
+        } else {
+            take();
         }
         const int64_t r0 = LOWER ? kk + 2 * (int64_t)b : 0;
         const int64_t rows = LOWER ? n - r0 : kk - b;
@@ -621,20 +643,21 @@ __device__ bool iv_triangle(const InvSolve &a, double *vc, double *vb, double (*
         bulk_tiles = rows > 0 ? (int)(rows / kIvRowsUpd) : 0;
         // the CTAs that had no tile on the chain take theirs first
         bulk_next = (int)gridDim.x - 1 - (int)blockIdx.x;
+        if (!ok) return false;
         iv_arrive(a);
         bulk(3);
-        if (!iv_wait(a, epoch, 53)) return false;
     }
-    return true;
+    wait(53);
+    return ok;
 }
 
 __global__ void __launch_bounds__(kIvThreads, 2) trsv_inv_kernel(InvSolve a) {
     extern __shared__ __align__(16) unsigned char iv_smem[];
-    double *vc = reinterpret_cast<double *>(iv_smem), *vb = vc + a.b;
+    double *vb = reinterpret_cast<double *>(iv_smem);
     double(*red)[kIvRowsUpd] = reinterpret_cast<double(*)[kIvRowsUpd]>(vb + a.b);
     unsigned epoch = 0;
-    if (!iv_triangle<true>(a, vc, vb, red, epoch)) return;
-    iv_triangle<false>(a, vc, vb, red, epoch);
+    if (!iv_triangle<true>(a, vb, red, epoch)) return;
+    iv_triangle<false>(a, vb, red, epoch);
 }
 
 // ---------------------------------------------------------------------------
