@@ -511,12 +511,12 @@ __device__ __forceinline__ void run_tiles64(SmemT64 &sm, int first, int stride, 
 typedef float (*Block64)[kNB + 4];
 
 // C[c][r] -= sum_{k = k0 .. k0+15} A[k][r] * B[c][k] for r in [r0, r0 + nr), c in
-// [c0, c0 + nc); nr and nc multiples of 4, at most 256 4 x 4 tiles.
+// [c0, c0 + nc); nr and nc multiples of 4, a 4 x 4 tile per thread tid = 0, 1, ...
 template <typename BA, typename BB, typename BC>
-__device__ __forceinline__ void sub_gemm16(BA A, BB B, BC C, int k0, int r0, int nr, int c0, int nc) {
+__device__ __forceinline__ void sub_gemm16(BA A, BB B, BC C, int k0, int r0, int nr, int c0, int nc, int tid) {
     const int tr = nr >> 2, tc = nc >> 2;
-    const int rg = threadIdx.x % tr, cg = threadIdx.x / tr;
-    if (cg >= tc) return;
+    const int rg = tid % tr, cg = tid / tr;
+    if (tid < 0 || cg >= tc) return;
     const int r = r0 + 4 * rg, c = c0 + 4 * cg;
     float x[4][4];
 #pragma unroll
@@ -548,6 +548,33 @@ __device__ __forceinline__ void sub_gemm16(BA A, BB B, BC C, int k0, int r0, int
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         *reinterpret_cast<float4 *>(&C[c + j][r]) = make_float4(x[j][0], x[j][1], x[j][2], x[j][3]);
+}
+
+// The same in 2 x 2 tiles for 16 columns: a few dozen 4 x 4 tiles would leave most warps
+// idle and run at one warp's issue rate.
+__device__ __forceinline__ void sub_gemm16_narrow(Block64 A, Block64 B, Block64 C, int k0, int r0, int nr, int c0) {
+    const int tr = nr >> 1;
+    const int rg = threadIdx.x % tr, cg = threadIdx.x / tr;
+    if (cg >= 8) return;
+    const int r = r0 + 2 * rg, c = c0 + 2 * cg;
+    float2 x0 = *reinterpret_cast<const float2 *>(&C[c][r]), x1 = *reinterpret_cast<const float2 *>(&C[c + 1][r]);
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {
+        const float4 b0 = *reinterpret_cast<const float4 *>(&B[c][k0 + 4 * k4]);
+        const float4 b1 = *reinterpret_cast<const float4 *>(&B[c + 1][k0 + 4 * k4]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 a = *reinterpret_cast<const float2 *>(&A[k0 + 4 * k4 + e][r]);
+            const float v0 = e == 0 ? b0.x : e == 1 ? b0.y : e == 2 ? b0.z : b0.w;
+            const float v1 = e == 0 ? b1.x : e == 1 ? b1.y : e == 2 ? b1.z : b1.w;
+            x0.x = fmaf(-v0, a.x, x0.x);
+            x0.y = fmaf(-v0, a.y, x0.y);
+            x1.x = fmaf(-v1, a.x, x1.x);
+            x1.y = fmaf(-v1, a.y, x1.y);
+        }
+    }
+    *reinterpret_cast<float2 *>(&C[c][r]) = x0;
+    *reinterpret_cast<float2 *>(&C[c + 1][r]) = x1;
 }
 
 // Rows k0 .. k0+15 of column X[c]: x_r -= l(r, k) x_k for r > k, L the unit lower
@@ -611,7 +638,7 @@ __device__ __forceinline__ void block_solve_upper(Block64 T, const float *dinv, 
         if (threadIdx.x < nr) sub_solve_upper(T, dinv, X, threadIdx.x, k0);
         __syncthreads();
         if (k0 + 16 < kNB) {
-            sub_gemm16(X, T, X, k0, 0, nr, k0 + 16, kNB - 16 - k0);
+            sub_gemm16(X, T, X, k0, 0, nr, k0 + 16, kNB - 16 - k0, threadIdx.x);
             __syncthreads();
         }
     }
@@ -623,7 +650,7 @@ __device__ __forceinline__ void block_solve_lower(Block64 T, BX X, int nc) {
         if (threadIdx.x < nc) sub_solve_lower(T, &X[threadIdx.x][0], k0);
         __syncthreads();
         if (k0 + 16 < kNB) {
-            sub_gemm16(T, X, X, k0, k0 + 16, kNB - 16 - k0, 0, nc);
+            sub_gemm16(T, X, X, k0, k0 + 16, kNB - 16 - k0, 0, nc, threadIdx.x);
             __syncthreads();
         }
     }
@@ -701,7 +728,9 @@ __device__ __forceinline__ void store_block(Block64 T, float *D, int64_t ld, int
 //    each lane eliminates the 4 x 4 block and the rest of those rows for
 //    itself, so the chain meets one exchange per four pivots (a shuffle per
 //    pivot and column took ~340 cycles per pivot);
-//  * then the 16 rows of U by sub_solve_lower and the rest by sub_gemm16.
+//  * then the 16 rows of U by sub_solve_lower and the next panel's columns by
+//    sub_gemm16_narrow; the columns beyond it wait for the warps that the next
+//    panel leaves idle.
 // Rows and columns past nb are those of the identity.
 // The 16 pivots of one panel on this warp's 32 rows (a: this lane's row).  kSafe:
 // reciprocals of pivots outside the fast form's range (subnormal, or 2^126 and
@@ -796,6 +825,10 @@ __device__ __noinline__ void getrf64(Smem &sm, int nb, float *D, int64_t lda, De
                 for (int c = 0; c < 16; ++c) a[c] = T[k0 + c][row];
                 bad = getrf64_panel<true>(a, sm.t.rows.r[warp], extreme);
             }
+        } else if (k0 > 0 && below) {
+            // the columns beyond this panel get the last panel's update from the
+            // warps that have no part in this one
+            sub_gemm16(T, T, T, k0 - 16, k0, kNB - k0, k0 + 16, kNB - 16 - k0, (int)threadIdx.x - 96);
         }
         __syncthreads();  // every warp has read the panel
         if (on && (ln >= 16 ? below : warp == 0)) {
@@ -808,7 +841,7 @@ __device__ __noinline__ void getrf64(Smem &sm, int nb, float *D, int64_t lda, De
         const int R = kNB - 16 - k0;
         if (threadIdx.x < R) sub_solve_lower(T, &T[k0 + 16 + threadIdx.x][0], k0);
         __syncthreads();
-        sub_gemm16(T, T, T, k0, k0 + 16, R, k0 + 16, R);
+        sub_gemm16_narrow(T, T, T, k0, k0 + 16, R, k0 + 16);  // the next panel's columns
         __syncthreads();
     }
     store_block(T, D, lda, nb, nb);
@@ -824,8 +857,7 @@ struct __align__(16) SmemStrip {
 
 // Look-ahead: T (in shared memory, for getrf64(..., in_smem = true)) = C - L U,
 // the next diagonal block (nb x nb) with the strips' first 64 rows and columns.
-// 8 x 4 outputs per thread of four warps; one fmaf chain over ascending k per
-// element, subtracted from C, as the other tiles of the update.
+// 8 x 4 outputs per thread.
 __device__ __noinline__ void look_ahead(SmemStrip &s, int nb, const float *L, const float *U, const float *C,
                                         int64_t ld) {
     request_block(s.x, L, ld, nb, kNB, false);
@@ -834,35 +866,47 @@ __device__ __noinline__ void look_ahead(SmemStrip &s, int nb, const float *L, co
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
-    if (threadIdx.x < 128) {
-        const int r = 4 * (threadIdx.x % 8), c = 4 * (threadIdx.x / 8);
-        float acc[4][8];
+    // two halves of k, 128 threads each, then one sum: eight warps hide the
+    // operand loads that bound it
+    const int id = threadIdx.x & 127, kh = threadIdx.x >> 7;
+    const int r = 4 * (id % 8), c = 4 * (id / 8);
+    float acc[4][8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[j][i] = 0.0f;
+        for (int i = 0; i < 8; ++i) acc[j][i] = 0.0f;
 #pragma unroll 4
-        for (int k4 = 0; k4 < kNB / 4; ++k4) {
-            float4 bq[4];
+    for (int k4 = kh * (kNB / 8); k4 < (kh + 1) * (kNB / 8); ++k4) {
+        float4 bq[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bq[j] = *reinterpret_cast<const float4 *>(&s.y[c + j][4 * k4]);
+        for (int j = 0; j < 4; ++j) bq[j] = *reinterpret_cast<const float4 *>(&s.y[c + j][4 * k4]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float4 a0 = *reinterpret_cast<const float4 *>(&s.x[4 * k4 + e][r]);
-                const float4 a1 = *reinterpret_cast<const float4 *>(&s.x[4 * k4 + e][32 + r]);
-                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        for (int e = 0; e < 4; ++e) {
+            const float4 a0 = *reinterpret_cast<const float4 *>(&s.x[4 * k4 + e][r]);
+            const float4 a1 = *reinterpret_cast<const float4 *>(&s.x[4 * k4 + e][32 + r]);
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float bv = e == 0 ? bq[j].x : e == 1 ? bq[j].y : e == 2 ? bq[j].z : bq[j].w;
+            for (int j = 0; j < 4; ++j) {
+                const float bv = e == 0 ? bq[j].x : e == 1 ? bq[j].y : e == 2 ? bq[j].z : bq[j].w;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[j][i] = fmaf(av[i], bv, acc[j][i]);
-                }
+                for (int i = 0; i < 8; ++i) acc[j][i] = fmaf(av[i], bv, acc[j][i]);
             }
         }
+    }
+    __syncthreads();  // the operands are read: each half's sums of the other's rows go to x
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4 *>(&s.x[c + j][32 * (1 - kh) + r]) =
+            make_float4(kh ? acc[j][0] : acc[j][4], kh ? acc[j][1] : acc[j][5], kh ? acc[j][2] : acc[j][6],
+                        kh ? acc[j][3] : acc[j][7]);
+    __syncthreads();
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s.t[c + j][(i < 4 ? 0 : 28) + r + i] -= acc[j][i];
+    for (int j = 0; j < 4; ++j) {
+        float4 *t = reinterpret_cast<float4 *>(&s.t[c + j][32 * kh + r]);
+        const float4 o = *reinterpret_cast<const float4 *>(&s.x[c + j][32 * kh + r]), v = *t;
+        const float m0 = kh ? acc[j][4] : acc[j][0], m1 = kh ? acc[j][5] : acc[j][1];
+        const float m2 = kh ? acc[j][6] : acc[j][2], m3 = kh ? acc[j][7] : acc[j][3];
+        *t = make_float4(v.x - (m0 + o.x), v.y - (m1 + o.y), v.z - (m2 + o.z), v.w - (m3 + o.w));
     }
     __syncthreads();
 }
