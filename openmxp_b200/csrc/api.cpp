@@ -137,6 +137,7 @@ struct mxp_workspace {
     float *coop_tmp = nullptr;          // 2 x diag_factor_tmp_floats(b)
     unsigned int *coop_sync = nullptr;  // grid-barrier counter + abort word: [0, 2) diagonal block, [8, 10) triangular solves
     void *split_big = nullptr, *split_big2 = nullptr, *split_u = nullptr, *split_l = nullptr;
+    size_t big2_bytes = 0;
     // GMRES-IR: basis V ((m+1) x n), Hessenberg H ((m+1) x m), rotations, scalars
     int gm_m = 30;
     double gm_tol = 1e-10;
@@ -166,11 +167,19 @@ static int64_t panel_ldk(int b, int form) {
     return (K + align - 1) / align * align;
 }
 
+// Second copy of a panel's product operand, so that both panels are cast in one
+// launch and their products can run side by side: kept for panels up to this
+// size (a launch does not matter beside the work of larger ones).
+constexpr size_t kSecondPanelMax = (size_t)192 << 20;
+static size_t second_panel_bytes(int64_t rows, int64_t ldk3) {
+    return std::min((size_t)rows * ldk3 * 2, kSecondPanelMax);
+}
+
 static size_t trsm_bytes(int n, int b) {
     const int64_t ldk3 = panel_ldk(b, MXP_FORM_BF16X2);
     const int64_t rows = n > b ? n - b : 1;
     return 2 * (size_t)b * b * 4 + ((size_t)b * b / 4 + 64 * (size_t)b) * 4 +
-           (size_t)(2 * rows + 2 * (int64_t)b) * ldk3 * 2 + 5120 + 2 * diag_factor_tmp_floats(b) * 4 + 256;
+           (size_t)(rows + 2 * (int64_t)b) * ldk3 * 2 + 5120 + second_panel_bytes(rows, ldk3) + 2 * diag_factor_tmp_floats(b) * 4 + 256;
 }
 
 // Stored inverses of the diagonal blocks: 2 x (n / b) blocks of b x b floats.
@@ -261,7 +270,8 @@ extern "C" mxp_status mxp_workspace_create(int n, int b, int form, int device, m
         if (ok) ws->tile_ctr = reinterpret_cast<int *>(ws->coop_sync + 32);
         if (ok) ws->trsm_ctr = reinterpret_cast<int *>(ws->coop_sync + 33);
         ok = ok && (ws->split_big = alloc((size_t)rows * ws->ldk3 * 2 + 1024));
-        ok = ok && (ws->split_big2 = alloc((size_t)rows * ws->ldk3 * 2 + 1024));
+        ws->big2_bytes = second_panel_bytes(rows, ws->ldk3);
+        ok = ok && (ws->split_big2 = alloc(ws->big2_bytes + 1024));
         ok = ok && (ws->split_u = alloc((size_t)b * ws->ldk3 * 2 + 1024));
         ok = ok && (ws->split_l = alloc((size_t)b * ws->ldk3 * 2 + 1024));
         ws->inv_blocks = n / b;
@@ -733,6 +743,22 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
                                    tmpU, tmpL, ws, on);
         return q;
     };
+    // Two independent tensor-core launches side by side (the second on the side
+    // stream) when their tiles leave SMs idle one after the other: a tile takes
+    // one SM, and a launch's pipeline fill and drain as long as a few short tiles.
+    auto pair_fits = [&](int64_t m0, int64_t n0, int64_t m1, int64_t n1) {
+        return ws->side && cdiv(m0, 128) * cdiv(n0, 256) + cdiv(m1, 128) * cdiv(n1, 256) <= num_sms();
+    };
+    auto fork = [&]() -> mxp_status {
+        MXP_CUDA(cudaEventRecord(ws->ev_inv[0], st));
+        MXP_CUDA(cudaStreamWaitEvent(ws->side, ws->ev_inv[0], 0));
+        return MXP_OK;
+    };
+    auto join = [&]() -> mxp_status {
+        MXP_CUDA(cudaEventRecord(ws->ev_inv[1], ws->side));
+        MXP_CUDA(cudaStreamWaitEvent(st, ws->ev_inv[1], 0));
+        return MXP_OK;
+    };
     // Factor the diagonal block of step kk (unless diag_done: it was factored
     // on the side stream), solve its two panels, and cast them into panel slot
     // `slot` (0 .. kMaxMerge-1) of the buffers at buffer row `row0`.
@@ -762,12 +788,15 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
                 if (q == MXP_OK) q = launch_tri_inv_lower_unit(b, Akk, lda, ws->tinv_l, b, ws->tinv_tmp, st);
             }
             pt.mark(PH_CAST);
-            // the operands of both products in one launch
+            // the operands of both products in one launch (a U panel larger than its
+            // own buffer: after the first product, in the L panel's)
+            const bool own = (size_t)m * ws->ldk3 * 2 <= ws->big2_bytes;
+            void *ubuf = own ? ws->split_big2 : ws->split_big;
             const CastJob ops[4] = {{0, m, b, Lcol, lda, ws->split_big, ws->ldk3},
                                     {1, b, b, inv_u(kk), b, ws->split_u, ws->ldk3},
                                     {0, b, b, inv_l(kk), b, ws->split_l, ws->ldk3},
-                                    {1, m, b, Urow, lda, ws->split_big2, ws->ldk3}};
-            if (q == MXP_OK) q = launch_casts(bf, ops, 4, st);
+                                    {1, m, b, Urow, lda, ubuf, ws->ldk3}};
+            if (q == MXP_OK) q = launch_casts(bf, ops, own ? 4 : 3, st);
             pt.mark(PH_TGEMM);
             // FP8 form: the product's epilogue also writes the E4M3 L panel and
             // its scales into the panel slot (the separate casts below are skipped)
@@ -786,6 +815,8 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
                 cudaError_t e = cudaMemsetAsync(ws->trsm_ctr, 0, 2 * sizeof(int), st);
                 if (e != cudaSuccess) q = cuda_fail(e, "panel_lu: TRSM tile counters");
             }
+            const bool both = own && pair_fits(m, b, b, m);
+            if (q == MXP_OK && both) q = fork();
             if (q == MXP_OK)
                 q = launch_schur(bf, m, b, b, ws->split_big, ws->ldk3, nullptr, ws->split_u, ws->ldk3,
                                  nullptr, Lcol, lda, ws->status, st, /*store=*/1, 0, 0, /*tri=*/1, ws->trsm_pair,
@@ -795,10 +826,19 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
             if (fuse_f8)
                 f8u = F8Out{Rb + (row0 * ldk + slot * kp) * es, ldk,
                             Rs + (row0 / 128) * scl + slot * (int64_t)cdiv(b, 128), scl, 1};
+            if (!own) {
+                pt.mark(PH_CAST);
+                if (q == MXP_OK) q = launch_casts(bf, ops + 3, 1, st);
+                pt.mark(PH_TGEMM);
+            }
             if (q == MXP_OK)
-                q = launch_schur(bf, b, m, b, ws->split_l, ws->ldk3, nullptr, ws->split_big2, ws->ldk3,
-                                 nullptr, Urow, lda, ws->status, st, /*store=*/1, 0, 0, /*tri=*/2, ws->trsm_pair,
-                                 tsu, fuse_f8 ? &f8u : nullptr);
+                q = launch_schur(bf, b, m, b, ws->split_l, ws->ldk3, nullptr, ubuf, ws->ldk3,
+                                 nullptr, Urow, lda, ws->status, both ? ws->side : st, /*store=*/1, 0, 0, /*tri=*/2,
+                                 ws->trsm_pair, tsu, fuse_f8 ? &f8u : nullptr);
+            if (both) {
+                const mxp_status jq = join();
+                if (q == MXP_OK) q = jq;
+            }
         } else {
             q = launch_trsm_runn(m, b, Akk, lda, Lcol, lda, st);
             if (q == MXP_OK) q = launch_trsm_llnu(b, m, Akk, lda, Urow, lda, st);
@@ -845,13 +885,19 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
             if (rem == 0 || r0 >= n) continue;
             pt.mark(PH_SCHUR);
             // column blocks of the later panels: rows r0..n, columns r0..r0+rem*b
-            s = schur(n - r0, (int64_t)rem * b, 1, (int64_t)j * b, (int64_t)j * b, d_A + r0 + r0 * lda, 0,
-                      nullptr, nullptr, j);
+            const int64_t w = (int64_t)rem * b, c0 = r0 + w;
+            const bool both = c0 < n && pair_fits(n - r0, w, w, n - c0);
+            if (both) s = fork();
+            if (s == MXP_OK)
+                s = schur(n - r0, w, 1, (int64_t)j * b, (int64_t)j * b, d_A + r0 + r0 * lda, 0, nullptr, nullptr, j);
             // their row blocks: rows r0..r0+rem*b, columns right of the group
-            const int64_t c0 = r0 + (int64_t)rem * b;
             if (s == MXP_OK && c0 < n)
-                s = schur((int64_t)rem * b, n - c0, 1, (int64_t)j * b, (int64_t)j * b + (int64_t)rem * b,
-                          d_A + r0 + c0 * lda, 0, nullptr, nullptr, j);
+                s = schur(w, n - c0, 1, (int64_t)j * b, (int64_t)j * b + w, d_A + r0 + c0 * lda, 0, nullptr,
+                          both ? ws->side : nullptr, j);
+            if (both) {
+                const mxp_status js = join();
+                if (s == MXP_OK) s = js;
+            }
         }
         diag_done = false;
         if (s != MXP_OK) break;
