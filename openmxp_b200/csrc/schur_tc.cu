@@ -478,6 +478,13 @@ schur_tc_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
 }
 
+__device__ __forceinline__ void copy16(float *dst, const float *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy4(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
 // ---- FP8 E4M3, block-scaled (kind::mxf8f6f4.block_scale) ---------------------
 //
 // Same pipeline with 128-byte K stages (128 FP8 values).  Each 128 x 128 tile
@@ -501,8 +508,17 @@ constexpr int kF8StageA = kBM * 128;
 constexpr int kF8StageB = kF8BN * 128;
 constexpr int kF8StageSF = 2048;  // SFA 512 B + SFB 1024 B, padded
 constexpr int kF8StageBytes = kF8StageA + kF8StageB + kF8StageSF;
-constexpr int kF8Stages = 4;
-constexpr int kF8SmemBytes = 1024 + kF8Stages * kF8StageBytes + 512;
+// Two forms.  Long K: four operand stages, C loaded by the epilogue into
+// registers (16 columns at a time: 16 KB in flight per SM, hidden by the
+// products).  Short K (kF8ShortK): the C read-modify-write bounds a tile (256 KB
+// against 128 KB of operands at K = 512), so one stage gives way to C: every
+// epilogue warp requests its 32 rows' next two 32-column pieces by cp.async
+// (64 KB in flight per SM), across tiles, while it stores the ones before.
+constexpr int kF8StagesLong = 4, kF8StagesShort = 3;
+constexpr int kF8CStage = 2 * 32 * 32 * 4 * kEpiWarps;  // two pieces of 32 x 32 per epilogue warp
+constexpr int kF8SmemLong = 1024 + kF8StagesLong * kF8StageBytes + 512;
+constexpr int kF8SmemShort = 1024 + kF8StagesShort * kF8StageBytes + kF8CStage + 512;
+constexpr int kF8ShortK = 1024;
 constexpr int kF8SfCol0 = 256;
 // Stages whose scale factors share one TMEM copy: a tile's scale is uniform
 // over its 128 x 128 block, so the four K blocks of a stage use one byte of
@@ -544,6 +560,7 @@ __host__ __device__ constexpr uint32_t idesc_mxf8(uint32_t sf_id) {
            ((uint32_t)(kBM >> 4) << 24) | (sf_id << 29);
 }
 
+template <bool kShort>
 __global__ void __launch_bounds__(kThreads, 1)
 schur_tc_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     int M, int N, int K, const uint8_t *__restrict__ lsc,
@@ -552,7 +569,9 @@ schur_tc_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                 ~uintptr_t(1023));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kF8Stages * kF8StageBytes);
+    constexpr int kF8Stages = kShort ? kF8StagesShort : kF8StagesLong;
+    float *cstage = reinterpret_cast<float *>(smem + kF8Stages * kF8StageBytes);  // kShort
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kF8Stages * kF8StageBytes + (kShort ? kF8CStage : 0));
     uint64_t *full = bars;
     uint64_t *empty = bars + kF8Stages;
     uint64_t *tfull = bars + 2 * kF8Stages;
@@ -751,49 +770,129 @@ schur_tc_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         int rslot = 0;
         uint32_t rphase = 0;
         bool ok = true;
-        for (;; ++it) {
-            int t;
-            if (!ring_take_warp(ring, rslot, rphase, t, abort_flag)) {
-                ok = false;
-                break;
+        if constexpr (kShort) {
+            float *cw = cstage + ew * 2048;
+            const bool vec = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & 3) == 0;
+            auto request = [&](int t, int q) {  // piece q of tile t (t < 0: nothing); always one copy group
+                if (t >= 0) {
+                    int tm, tn;
+                    tiles.get(t, tm, tn);
+                    const int64_t row0 = (int64_t)tm * kBM + quarter * 32;
+                    const int64_t col0 = (int64_t)tn * kF8BN + col_half * 128 + 32 * q;
+                    float *slot = cw + (q & 1) * 1024;  // [column][row]
+                    const float *cp = C + col0 * ldc + row0;
+                    if (vec) {
+                        const int r = (lane & 7) * 4;
+                        const int by = 4 * (int)max((int64_t)0, min((int64_t)4, M - row0 - r));
+#pragma unroll
+                        for (int c = lane >> 3; c < 32; c += 4)
+                            if (col0 + c < N && by > 0) copy16(slot + c * 32 + r, cp + c * ldc + r, by);
+                    } else if (row0 + lane < M) {
+#pragma unroll 8
+                        for (int c = 0; c < 32; ++c)
+                            if (col0 + c < N) copy4(slot + c * 32 + lane, cp + c * ldc + lane);
+                    }
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            int t = -1;
+            if (!ring_take_warp(ring, rslot, rphase, t, abort_flag)) ok = false;
+            if (ok) {
+                request(t, 0);
+                request(t, 1);
             }
-            if (t < 0) break;
-            int tm, tn;
-            tiles.get(t, tm, tn);
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(tfull), it & 1u, abort_flag))) {
-                ok = false;
-                break;
-            }
-            __syncwarp();
-            tc_fence_after();
-            uint32_t r[4][32];
+            for (; ok && t >= 0; ++it) {
+                int tm, tn, next = -1;
+                tiles.get(t, tm, tn);
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(tfull), it & 1u, abort_flag))) {
+                    ok = false;
+                    break;
+                }
+                __syncwarp();
+                tc_fence_after();
+                uint32_t r[4][32];
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + col_half * 128 + 32 * c, r[c]);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(tempty));  // accumulator free: next tile may start
-            const int64_t row = (int64_t)tm * kBM + quarter * 32 + lane;
-            if (row < M) {
+                for (int c = 0; c < 4; ++c)
+                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + col_half * 128 + 32 * c, r[c]);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(tempty));  // accumulator free: next tile may start
+                // (the producer names the next tile once it has issued this one's loads)
+                if (!ring_take_warp(ring, rslot, rphase, next, abort_flag)) {
+                    ok = false;
+                    break;
+                }
+                const int64_t row = (int64_t)tm * kBM + quarter * 32 + lane;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int64_t col0 = (int64_t)tn * kF8BN + col_half * 128 + 32 * c;
-                    const int ncol = (int)imin64(32, (int64_t)N - col0);
-                    float *cp = C + col0 * ldc + row;
-                    if (ncol >= 32) {
+                for (int q = 0; q < 4; ++q) {
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                    __syncwarp();
+                    const int64_t col0 = (int64_t)tn * kF8BN + col_half * 128 + 32 * q;
+                    const float *slot = cw + (q & 1) * 1024 + lane;
+                    if (row < M) {
+                        float *cp = C + col0 * ldc + row;
+                        const int ncol = (int)imin64(32, (int64_t)N - col0);
+                        if (ncol >= 32) {
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float cv[16];
+                            for (int j = 0; j < 32; ++j, cp += ldc) __stcs(cp, slot[32 * j] - __uint_as_float(r[q][j]));
+                        } else {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) cv[j] = __ldcs(cp + (16 * h + j) * ldc);
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                __stcs(cp + (16 * h + j) * ldc, cv[j] - __uint_as_float(r[c][16 * h + j]));
+                            for (int j = 0; j < 32; ++j, cp += ldc)
+                                if (j < ncol) __stcs(cp, slot[32 * j] - __uint_as_float(r[q][j]));
                         }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (j < ncol) cp[j * ldc] = cp[j * ldc] - __uint_as_float(r[c][j]);
+                    }
+                    __syncwarp();  // the slot has been read
+                    if (q < 2) request(t, q + 2);
+                    else request(next, q - 2);
+                }
+                t = next;
+            }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        } else {
+            for (;; ++it) {
+                int t;
+                if (!ring_take_warp(ring, rslot, rphase, t, abort_flag)) {
+                    ok = false;
+                    break;
+                }
+                if (t < 0) break;
+                int tm, tn;
+                tiles.get(t, tm, tn);
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(tfull), it & 1u, abort_flag))) {
+                    ok = false;
+                    break;
+                }
+                __syncwarp();
+                tc_fence_after();
+                uint32_t r[4][32];
+    #pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + col_half * 128 + 32 * c, r[c]);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(tempty));  // accumulator free: next tile may start
+                const int64_t row = (int64_t)tm * kBM + quarter * 32 + lane;
+                if (row < M) {
+    #pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const int64_t col0 = (int64_t)tn * kF8BN + col_half * 128 + 32 * c;
+                        const int ncol = (int)imin64(32, (int64_t)N - col0);
+                        float *cp = C + col0 * ldc + row;
+                        if (ncol >= 32) {
+    #pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                float cv[16];
+    #pragma unroll
+                                for (int j = 0; j < 16; ++j) cv[j] = __ldcs(cp + (16 * h + j) * ldc);
+    #pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    __stcs(cp + (16 * h + j) * ldc, cv[j] - __uint_as_float(r[c][16 * h + j]));
+                            }
+                        } else {
+    #pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                if (j < ncol) cp[j * ldc] = cp[j * ldc] - __uint_as_float(r[c][j]);
+                        }
                     }
                 }
             }
@@ -910,12 +1009,16 @@ mxp_status launch_schur(int form, int m, int n, int k, const void *L, int64_t ld
         if (s != MXP_OK) return s;
         static bool attr8 = false;
         if (!attr8) {
-            MXP_CUDA(cudaFuncSetAttribute(schur_tc_fp8_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kF8SmemBytes));
+            MXP_CUDA(cudaFuncSetAttribute(schur_tc_fp8_kernel<false>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kF8SmemLong));
+            MXP_CUDA(cudaFuncSetAttribute(schur_tc_fp8_kernel<true>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kF8SmemShort));
             attr8 = true;
         }
         const int kt = (int)cdiv(K, 128);
-        schur_tc_fp8_kernel<<<grid, kThreads, kF8SmemBytes, st>>>(
+        const bool is_short = K <= kF8ShortK;
+        auto kernel = is_short ? schur_tc_fp8_kernel<true> : schur_tc_fp8_kernel<false>;
+        kernel<<<grid, kThreads, is_short ? kF8SmemShort : kF8SmemLong, st>>>(
             mapA, mapB, m, n, (int)K, lsc, rsc, lsc_ld > 0 ? lsc_ld : kt, rsc_ld > 0 ? rsc_ld : kt, C,
             ldc, tiles, src, dst);
         MXP_LAUNCHED();
