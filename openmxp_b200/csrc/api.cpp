@@ -193,7 +193,7 @@ static size_t ws_layout(int n, int b, int form, size_t *panel_bytes, size_t *sca
     *panel_bytes = (size_t)(rows * kMaxMerge * ldk * esize + 1024) / 256 * 256 + 256;
     *scale_bytes = (size_t)(cdiv(rows, 128) * kMaxMerge * cdiv(b, 128) + 256) / 256 * 256 + 256;
     *vec_doubles = (size_t)n * (4 + 16) + 64;
-    *flag_ints = lu_solve_flag_ints(n) + 64;
+    *flag_ints = 64;  // tickets of the triangular chain
     *vec_doubles += (size_t)31 * n + 64 * 32 + 2 * 31 * 64 + 31 * (size_t)(2 * 148 + 2) + 1024;
     return 2 * *panel_bytes + 2 * *scale_bytes + *vec_doubles * 8 + *flag_ints * 4 + 256 +
            trsm_bytes(n, b) + inv_store_bytes(n, b) + (size_t)4 * b * 8 + 256;
@@ -988,7 +988,8 @@ static mxp_status lu_solve_ws(mxp_workspace *ws, int n, const float *LU, int64_t
         return launch_lu_solve_inv(n, ws->b, LU, lda, ws->inv_store, ws->inv_store + bb, 2 * bb, x, ws->trsv_t,
                                    ws->coop_sync + 8, ws->status, st);
     }
-    return launch_lu_solve(n, LU, lda, x, ws->flags, ws->status, st, withhold);
+    // (the residual product's partial sums are not in use meanwhile: 16 n doubles)
+    return launch_lu_solve(n, LU, lda, x, ws->partials, ws->flags, ws->status, st, withhold);
 }
 
 extern "C" mxp_status mxp_otf_gemv(int n, uint64_t seed, const double *d_d, double alpha,

@@ -265,11 +265,11 @@ mxp_status launch_schur(int form, int m, int n, int k, const void *L, int64_t ld
 mxp_status launch_otf_gemv(int n, uint64_t seed, const double *d, double alpha, const double *x,
                            double beta, double *y, double *partials, int max_splits,
                            cudaStream_t st);
-// withhold >= 0: the forward solve never publishes that row block's flag, so
-// the blocks that need it give up after the bounded wait (tests of MXP_TIMEOUT).
-mxp_status launch_lu_solve(int n, const float *LU, int64_t lda, double *x, int *flags,
+// mail: 2 n doubles, tickets: 2 ints of device memory (set on the stream first).
+// withhold >= 0: the forward solve never publishes that row block, so the
+// blocks that need it give up after the bounded wait (tests of MXP_TIMEOUT).
+mxp_status launch_lu_solve(int n, const float *LU, int64_t lda, double *x, double *mail, int *tickets,
                            DevStatus *dst, cudaStream_t st, int withhold = -1);
-size_t lu_solve_flag_ints(int n);
 // Block triangular solves with the stored FP32 inverses of the b x b diagonal
 // blocks (XU: inv(U_kk), XL: inv(L_kk), block k at offset k*xstride, ld b):
 // x <- U^{-1} L^{-1} x, one cooperative launch.  t: 4 b doubles of scratch;

@@ -15,7 +15,7 @@
 //    trsvU_h, panel_trsv.hpp:308-597).  One persistent launch per triangle:
 //    row blocks of 64 are claimed in order through an atomic ticket; a row
 //    block streams its part of the factor against the already-solved blocks
-//    (waiting, bounded, on per-block completion flags), then solves its 64 x
+//    (waiting, bounded, for their values), then solves its 64 x
 //    64 diagonal triangle in FP64 and publishes.  Claim order guarantees every
 //    awaited block is owned by a CTA that is already running.
 //  * lu_solve_inv: the same solve in nb steps of bandwidth-bound products
@@ -139,13 +139,8 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
     return v;
 }
 
-__device__ __forceinline__ void st_release(int *p, int v) {
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // Block forward (LOWER: unit L) or backward (upper: U) substitution, one
 // 64-row block per CTA, CTAs taking row blocks in solve order from a ticket.
-// flags[0..nrb): block done; flags[nrb]: ticket.
 //
 // The blocks form a chain (block b needs x of every earlier block), so the
 // time per link is what bounds the solve.  Everything that does not depend
@@ -157,22 +152,58 @@ __device__ __forceinline__ void st_release(int *p, int v) {
 //   * w = Minv (r_b - those products).
 // When the predecessor publishes its x, the block finishes with one 64 x 64
 // FP64 matrix-vector product, x_b = w - P x_adj, and publishes its own x.
+// A value is published by its own 8-byte store to `mail`, which starts out as
+// kNoMail everywhere: the value itself says that it is there, so a link
+// takes neither a fence, a flag nor a second load (with a flag released after
+// the values and polled before they are read a link took 3.7 us, of which
+// ~1.4 us were those).  Sums run in four interleaved parts: a chain of
+// dependent FP64 operations per column cost as much as the exchange.
 // This is the block substitution of the reference's trsvL_h / trsvU_h
 // (panel_trsv.hpp:308-597: FP64 solve of each upcast diagonal block, FP32 x
 // FP64 products for the rest) with the diagonal solve applied as a product
 // with its inverse.
+constexpr unsigned long long kNoMail = ~0ull;  // a NaN no operation returns (published values are kept off it)
+
+__device__ __forceinline__ unsigned long long ld_mail(const double *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_mail(double *p, double x) {
+    unsigned long long v = (unsigned long long)__double_as_longlong(x);
+    if (v == kNoMail) v = 0x7ff8000000000000ull;
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// The value at p, waited for (bounded): between polls the thread sleeps 100 ns for
+// each of the `far` links the chain is away.  ok: cleared when the wait gave up.
+__device__ __forceinline__ double take_mail(const double *p, int far, bool &ok) {
+    unsigned long long v = ld_mail(p);
+    if (v == kNoMail && ok) {
+        const unsigned long long t0 = globaltimer_ns();
+        for (uint32_t it = 1; (v = ld_mail(p)) == kNoMail; ++it) {
+            if (far > 0) __nanosleep(100 * far);
+            if ((it & 63u) == 0u && globaltimer_ns() - t0 > kWaitTimeoutNs) {
+                ok = false;
+                break;
+            }
+        }
+    }
+    return v == kNoMail ? 0.0 : __longlong_as_double((long long)v);
+}
+
 constexpr int kXChunk = 8;  // column blocks whose x is staged in shared memory at a time
-constexpr size_t kTrsvSmem = 2 * sizeof(double) * kRB * (kRB + 1) + sizeof(float) * kRB * (kRB + 1) +
+constexpr int kMP = kRB + 4;    // pitch of Minv and P: four rows x four lanes on 16 banks
+constexpr size_t kTrsvSmem = 2 * sizeof(double) * kRB * kMP + sizeof(float) * kRB * (kRB + 1) +
                              sizeof(double) * kRB + sizeof(double) * 4 * kRB +
                              sizeof(double) * 2 * kXChunk * kRB + 16;
 
 template <bool LOWER>
 __global__ void __launch_bounds__(kTrsvThreads)
-trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *flags,
+trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, double *mail, int *ticket,
             DevStatus *dst, int withhold) {
     extern __shared__ __align__(16) unsigned char trsv_smem[];
-    double(*minv)[kRB + 1] = reinterpret_cast<double(*)[kRB + 1]>(trsv_smem);
-    double(*pm)[kRB + 1] = minv + kRB;
+    double(*minv)[kMP] = reinterpret_cast<double(*)[kMP]>(trsv_smem);
+    double(*pm)[kMP] = minv + kRB;
     float(*blk)[kRB + 1] = reinterpret_cast<float(*)[kRB + 1]>(pm + kRB);   // blk[col][row]
     double *zs = reinterpret_cast<double *>(blk + kRB);
     double(*part)[kRB] = reinterpret_cast<double(*)[kRB]>(zs + kRB);
@@ -181,7 +212,7 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
 
     const int nrb = (n + kRB - 1) / kRB;
     const int tid = threadIdx.x;
-    if (tid == 0) *s_ticket = atomicAdd(&flags[nrb], 1);
+    if (tid == 0) *s_ticket = atomicAdd(ticket, 1);
     __syncthreads();
     const int rb = LOWER ? *s_ticket : nrb - 1 - *s_ticket;
     const int64_t row0 = (int64_t)rb * kRB;
@@ -189,6 +220,7 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
     const int ncb = LOWER ? rb : nrb - 1 - rb;  // off-diagonal column blocks
     const bool has_adj = ncb > 0;
     const int adj = LOWER ? rb - 1 : rb + 1;    // chain predecessor
+    const double rhs = tid < nrows ? x[row0 + tid] : 0.0;
 
     // ---- Minv: inverse of the diagonal block (padded with the identity) ----
     for (int idx = tid; idx < kRB * kRB; idx += kTrsvThreads) {
@@ -198,27 +230,37 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
         blk[cc][rr] = v;
     }
     __syncthreads();
-    if (tid < kRB) {  // column j of the inverse: T y = e_j
-        const int j = tid;
-        if (LOWER) {
-            for (int i = 0; i < kRB; ++i) {
-                double v = (i == j) ? 1.0 : 0.0;
-                if (i > j)
-                    for (int k = j; k < i; ++k) v = __fma_rn(-(double)blk[k][i], minv[k][j], v);
-                minv[i][j] = (i >= j) ? v : 0.0;
+    const int pi = tid >> 2, ph = tid & 3;
+    {   // column pi of the inverse, T y = e_pi: four lanes share each sum over k
+        const int j = pi;
+        auto dot = [&](int i, int k0, int k1) {  // sum of T(i, k) y_k, k0 <= k < k1
+            double s0 = 0.0, s1 = 0.0;
+            int k = k0 + ph;
+            for (; k + 4 < k1; k += 8) {
+                s0 = __fma_rn((double)blk[k][i], minv[k][j], s0);
+                s1 = __fma_rn((double)blk[k + 4][i], minv[k + 4][j], s1);
             }
-        } else {
-            for (int i = kRB - 1; i >= 0; --i) {
-                double v = (i == j) ? 1.0 : 0.0;
-                if (i < j)
-                    for (int k = i + 1; k <= j; ++k) v = __fma_rn(-(double)blk[k][i], minv[k][j], v);
-                minv[i][j] = (i <= j) ? v / (double)blk[i][i] : 0.0;
+            if (k < k1) s0 = __fma_rn((double)blk[k][i], minv[k][j], s0);
+            s0 += s1;
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+            return s0;
+        };
+#pragma unroll 1
+        for (int q = 0; q < kRB; ++q) {
+            const int i = LOWER ? q : kRB - 1 - q;
+            const double s = LOWER ? dot(i, j, i) : dot(i, i + 1, j + 1);
+            if (ph == 0) {
+                const double e = i == j ? 1.0 : 0.0;
+                if (LOWER) minv[i][j] = i < j ? 0.0 : e - s;
+                else minv[i][j] = i > j ? 0.0 : (e - s) / (double)blk[i][i];
             }
+            __syncwarp();
         }
     }
     __syncthreads();
     // ---- P = Minv * A_adj ----
-    const int pi = tid >> 2, ph = tid & 3;  // row of a 64-vector, quarter of its columns
+    // (row pi of a 64-vector, quarter ph of its columns)
     if (has_adj) {
         const int64_t c0 = (int64_t)adj * kRB;
         const int ncols = (int)imin64(kRB, n - c0);
@@ -228,17 +270,21 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
         }
         __syncthreads();
 #pragma unroll 1
-        for (int c = ph * 16; c < ph * 16 + 16; ++c) {
-            double v = 0.0;
-#pragma unroll 8
-            for (int k = 0; k < kRB; ++k) v = __fma_rn(minv[pi][k], (double)blk[c][k], v);
-            pm[pi][c] = v;
+        for (int c = ph * 16; c < ph * 16 + 16; c += 4) {  // four columns: independent sums
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+            for (int k = 0; k < kRB; ++k) {
+                const double m = minv[pi][k];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = __fma_rn(m, (double)blk[c + e][k], v[e]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) pm[pi][c + e] = v[e];
         }
     }
 
     // ---- products with every other off-diagonal block ----
-    double acc = 0.0;
-    int known = LOWER ? -1 : nrb;  // furthest block known complete
+    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
     bool timed_out = false;
     const int r = tid % kRB, cph = tid / kRB;  // 4 column phases of 16
     const int64_t grow = row0 + r;
@@ -253,36 +299,6 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
 #pragma unroll
         for (int cc = 0; cc < 16; ++cc) d[cc] = (row_ok && cc < clen) ? col[cc * lda] : 0.0f;
     };
-    // One thread of the CTA polls (the others wait at the CTA barrier, which
-    // orders their later loads after its acquire), and a block whose turn is
-    // far off sleeps between polls: every CTA's warps spinning on the few lines
-    // that hold the flags held back the one store the chain waits for.
-    __shared__ int s_seen;
-    auto wait_flag = [&](int b) -> bool {  // all threads; ends with a barrier
-        if (tid == 0) {
-            int ok = 1;
-            const int far = min(32, max(0, (LOWER ? rb - b : b - rb) - 3));
-            const unsigned long long t0 = globaltimer_ns();
-            uint32_t it = 0;
-            while (!ld_acquire(&flags[b])) {
-                if (far) __nanosleep(100 * far);
-                if ((++it & 63u) == 0u && globaltimer_ns() - t0 > kWaitTimeoutNs) {
-                    ok = 0;
-                    break;
-                }
-            }
-            s_seen = ok;
-        }
-        __syncthreads();
-        return s_seen != 0;
-    };
-    auto probe_flag = [&](int b) -> bool {
-        if (tid == 0) s_seen = ld_acquire(&flags[b]);
-        __syncthreads();
-        const bool seen = s_seen != 0;
-        __syncthreads();  // s_seen is written again
-        return seen;
-    };
     // The x of the streamed column blocks is staged in shared memory kXChunk
     // blocks at a time (one coalesced load per thread and one barrier per
     // chunk, double-buffered) instead of one L2 round trip per column block:
@@ -290,7 +306,12 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
     auto consume = [&](int buf, int qq, const float *lv) {
         const double *xv = xs[buf] + qq * kRB + cph * 16;
 #pragma unroll
-        for (int cc = 0; cc < 16; ++cc) acc = __fma_rn((double)lv[cc], xv[cc], acc);
+        for (int cc = 0; cc < 16; cc += 4) {
+            acc0 = __fma_rn((double)lv[cc], xv[cc], acc0);
+            acc1 = __fma_rn((double)lv[cc + 1], xv[cc + 1], acc1);
+            acc2 = __fma_rn((double)lv[cc + 2], xv[cc + 2], acc2);
+            acc3 = __fma_rn((double)lv[cc + 3], xv[cc + 3], acc3);
+        }
     };
     // factor values do not depend on other blocks: keep four column blocks of
     // loads in flight (a register ring, unrolled so its indices stay static)
@@ -302,23 +323,15 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
     int buf = 0;
     for (int q0 = 0; q0 < nstream; q0 += kXChunk, buf ^= 1) {
         const int qn = min(kXChunk, nstream - q0);
-        const int cb_last = LOWER ? q0 + qn - 1 : nrb - 1 - (q0 + qn - 1);
-        // blocks complete in chain order: once the chunk's last block (or the
-        // block before the predecessor) is published, so is the whole chunk
-        if (!timed_out && (LOWER ? (cb_last > known) : (cb_last < known))) {
-            if (probe_flag(adj - (LOWER ? 1 : -1))) {
-                known = adj - (LOWER ? 1 : -1);
-            } else {
-                timed_out = !wait_flag(cb_last);
-                known = cb_last;
-            }
-        }
+        bool ok = true;
         for (int e = tid; e < qn * kRB; e += kTrsvThreads) {
             const int qq = e / kRB, cc = e % kRB;
             const int cb = LOWER ? q0 + qq : nrb - 1 - (q0 + qq);
             const int64_t col = (int64_t)cb * kRB + cc;
-            xs[buf][e] = (col < n) ? __ldcg(x + col) : 0.0;
+            const int far = min(32, (LOWER ? rb - cb : cb - rb) - 3);
+            xs[buf][e] = (col < n) ? take_mail(mail + col, far, ok) : 0.0;
         }
+        timed_out = !ok;
         // a wait that gave up anywhere in the CTA ends the stream everywhere
         timed_out = __syncthreads_or(timed_out) != 0;
         if (timed_out) break;
@@ -330,40 +343,67 @@ trsv_kernel(int n, const float *__restrict__ LU, int64_t lda, double *x, int *fl
             if (qq + 3 < qn) { consume(buf, qq + 3, b3); load_l(q0 + qq + 7, b3); }
         }
     }
-    part[cph][r] = acc;
+    part[cph][r] = (acc0 + acc1) + (acc2 + acc3);
     __syncthreads();
     if (tid < kRB) {
-        const double s = part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid];
-        zs[tid] = (tid < nrows) ? __ldcg(x + row0 + tid) - s : 0.0;
+        const double s = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+        zs[tid] = rhs - s;
     }
     __syncthreads();
-    // ---- w = Minv z (row pi, four lanes per row) ----
-    double w = 0.0;
+    // ---- w = Minv z (row pi; lane ph of its four takes columns 4 c + ph) ----
+    auto row_product = [&](const double (*m)[kMP], const double *v) {
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
-    for (int c = 0; c < 16; ++c) w = __fma_rn(minv[pi][ph * 16 + c], zs[ph * 16 + c], w);
-    w += __shfl_xor_sync(0xffffffffu, w, 1);
-    w += __shfl_xor_sync(0xffffffffu, w, 2);
+        for (int c = 0; c < 16; c += 4) {
+            s0 = __fma_rn(m[pi][4 * c + ph], v[c], s0);
+            s1 = __fma_rn(m[pi][4 * c + 4 + ph], v[c + 1], s1);
+            s2 = __fma_rn(m[pi][4 * c + 8 + ph], v[c + 2], s2);
+            s3 = __fma_rn(m[pi][4 * c + 12 + ph], v[c + 3], s3);
+        }
+        double s = (s0 + s1) + (s2 + s3);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        return s;
+    };
+    double xa[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) xa[c] = zs[4 * c + ph];
+    double w = row_product(minv, xa);
     // ---- the chain link: x_b = w - P x_adj ----
     if (has_adj && !timed_out) {  // (the same in every thread)
-        timed_out = !wait_flag(adj);
-        const int64_t c0 = (int64_t)adj * kRB + ph * 16;
-        const int clen = (int)imin64(16, n - c0);
-        double xa[16];
+        const int64_t c0 = (int64_t)adj * kRB;
+        bool ok = true;
+        // all sixteen together, again until none is missing (one by one each
+        // would cost a round trip of its own)
+        const double *mp = mail + c0 + ph;
+        const int have = (int)imin64(kRB, n - c0) - ph;  // columns 4 c < have exist
+        const unsigned long long t0 = globaltimer_ns();
+        for (uint32_t it = 1;; ++it) {
+            unsigned long long raw[16];
+            bool missing = false;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) xa[c] = (c < clen) ? __ldcg(x + c0 + c) : 0.0;
-        double p = 0.0;
+            for (int c = 0; c < 16; ++c) raw[c] = 4 * c < have ? ld_mail(mp + 4 * c) : 0ull;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) p = __fma_rn(pm[pi][ph * 16 + c], xa[c], p);
-        p += __shfl_xor_sync(0xffffffffu, p, 1);
-        p += __shfl_xor_sync(0xffffffffu, p, 2);
-        w -= p;
+            for (int c = 0; c < 16; ++c) {
+                missing |= raw[c] == kNoMail;
+                xa[c] = __longlong_as_double((long long)raw[c]);
+            }
+            if (!missing) break;
+            if ((it & 63u) == 0u && globaltimer_ns() - t0 > kWaitTimeoutNs) {
+                ok = false;
+                break;
+            }
+        }
+        w -= row_product(pm, xa);
+        timed_out = !ok;
+    }
+    // published even after a timeout, so successors never stall; `withhold` (a
+    // test of the bounded waits) leaves one block unpublished
+    if (ph == 0 && pi < nrows) {
+        if (rb != withhold) st_mail(mail + row0 + pi, w);
+        x[row0 + pi] = w;
     }
     if (timed_out) report(dst, MXP_TIMEOUT, 10 + (LOWER ? 0 : 1), rb);
-    if (ph == 0 && pi < nrows) __stcg(x + row0 + pi, w);
-    __syncthreads();  // the release below covers the CTA's stores
-    // published even after a timeout, so successors never stall; `withhold` (a
-    // test of the bounded waits) leaves one block's flag unset
-    if (tid == 0 && rb != withhold) st_release(&flags[rb], 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -744,19 +784,18 @@ mxp_status launch_otf_gemv(int n, uint64_t seed, const double *d, double alpha, 
     return MXP_OK;
 }
 
-size_t lu_solve_flag_ints(int n) { return 2 * ((size_t)cdiv(n, kRB) + 1); }
-
-mxp_status launch_lu_solve(int n, const float *LU, int64_t lda, double *x, int *flags,
+mxp_status launch_lu_solve(int n, const float *LU, int64_t lda, double *x, double *mail, int *tickets,
                            DevStatus *dst, cudaStream_t st, int withhold) {
     if (n <= 0) return MXP_OK;
     if (lda < n) return fail(MXP_INVALID_ARG, "lu_solve: lda < n");
     const int nrb = (int)cdiv(n, kRB);
-    MXP_CUDA(cudaMemsetAsync(flags, 0, lu_solve_flag_ints(n) * sizeof(int), st));
+    MXP_CUDA(cudaMemsetAsync(tickets, 0, 2 * sizeof(int), st));
+    MXP_CUDA(cudaMemsetAsync(mail, 0xff, 2 * (size_t)n * sizeof(double), st));
     MXP_CUDA(cudaFuncSetAttribute(trsv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsvSmem));
     MXP_CUDA(cudaFuncSetAttribute(trsv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrsvSmem));
-    trsv_kernel<true><<<nrb, kTrsvThreads, kTrsvSmem, st>>>(n, LU, lda, x, flags, dst, withhold);
+    trsv_kernel<true><<<nrb, kTrsvThreads, kTrsvSmem, st>>>(n, LU, lda, x, mail, tickets, dst, withhold);
     MXP_LAUNCHED();
-    trsv_kernel<false><<<nrb, kTrsvThreads, kTrsvSmem, st>>>(n, LU, lda, x, flags + nrb + 1, dst, -1);
+    trsv_kernel<false><<<nrb, kTrsvThreads, kTrsvSmem, st>>>(n, LU, lda, x, mail + n, tickets + 1, dst, -1);
     MXP_LAUNCHED();
     return MXP_OK;
 }
