@@ -702,22 +702,21 @@ __device__ double block_max(double v, double *red) {
 // The sum over j runs in increasing j.  R rows per thread, 256 apart: their
 // independent chains (LCG step, one subtraction, two FMAs per element) are
 // what hides latency with two warps per scheduler.  The element as in
-// otf_gemv_kernel: both 32-bit halves of the state in the mantissas of
-// biased doubles, the low half's bias (2^52 x_j) and the diagonal's
-// generator value taken out at the end.
+// otf_gemv_kernel: a sum for each 32-bit half of the state, the high one
+// converted, the low one in the mantissa of a biased double, whose bias (2^52
+// x_j) and the diagonal's generator value are taken out at the end.
 template <int R>
 __device__ __noinline__ void otf_rows(int n, uint64_t s00, Aff jn, const double *__restrict__ d,
                                       const double *__restrict__ b, const double *xs, double *rs, int i0) {
     constexpr double kScale = 0x1.fffffffffffffP-65;
-    constexpr double kHiBias = 0x1p84 + 0x1p63;
     const Aff inc1 = lcg_inc1(), step = aff_pow(inc1, (uint64_t)kBatchThreads);
     uint64_t s[R];
-    double acc[R], sum = 0.0;
+    double acc[R], hi[R], sum = 0.0;
     s[0] = aff_apply(aff_pow(inc1, (uint64_t)i0), s00);  // element (i0, 0)
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         if (q) s[q] = aff_apply(step, s[q - 1]);
-        acc[q] = 0.0;
+        acc[q] = hi[q] = 0.0;
     }
 #pragma unroll 2
     for (int j = 0; j < n; ++j) {
@@ -725,8 +724,7 @@ __device__ __noinline__ void otf_rows(int n, uint64_t s00, Aff jn, const double 
         sum += xj;
 #pragma unroll
         for (int q = 0; q < R; ++q) {
-            const double h = __hiloint2double(0x45300000, (int)((uint32_t)(s[q] >> 32) ^ 0x80000000u)) - kHiBias;
-            acc[q] = __fma_rn(h, xj, acc[q]);
+            hi[q] = __fma_rn((double)(int)(s[q] >> 32), xj, hi[q]);
             acc[q] = __fma_rn(__hiloint2double(0x43300000, (int)(uint32_t)s[q]), xj, acc[q]);
             s[q] = aff_apply(jn, s[q]);
         }
@@ -736,7 +734,7 @@ __device__ __noinline__ void otf_rows(int n, uint64_t s00, Aff jn, const double 
         const int i = i0 + q * kBatchThreads;
         if (i >= n) break;
         const uint64_t sd = aff_apply(aff_pow(inc1, (uint64_t)i * (uint64_t)(n + 1)), s00);
-        double v = __fma_rn(-0x1p52, sum, acc[q]);
+        double v = __fma_rn(hi[q], 0x1p32, __fma_rn(-0x1p52, sum, acc[q]));
         v = __fma_rn(-i64_to_double_rn(sd), xs[i] * kScale, v);
         rs[i] = b[i] - (v + d[i] * xs[i]);
     }

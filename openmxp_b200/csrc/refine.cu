@@ -40,12 +40,15 @@ constexpr int kGemvXChunk = 1024;
 constexpr double kLcgScale = 0x1.fffffffffffffP-65;
 
 // Per element the state s = hi * 2^32 + lo (hi signed, lo unsigned) enters
-// as two exact doubles, both made by placing the integer in the mantissa of
-// a biased constant: hi * 2^32 = (2^84 + (hi ^ 2^31) * 2^32) - (2^84 + 2^63),
-// and 2^52 + lo, whose bias 2^52 is not removed per element: the CTA sums
+// as two exact doubles with a sum each: hi by the 32-bit integer converter (its
+// sum times 2^32 at the end), and 2^52 + lo by placing lo in the mantissa of
+// a biased constant, whose bias 2^52 is not removed per element: the CTA sums
 // 2^52 * xs over its columns once and subtracts it from every row at the
 // end (the bias terms are 2^-12 |x| each against |a_ij x| ~ |x|/4, so the
-// extra rounding stays far below the FP64 rounding of the sum itself).  The
+// extra rounding stays far below the FP64 rounding of the sum itself).  What
+// bounds it is instructions per element (a loop of this element alone: 8.5
+// elements per clock and SM; 7.8 with hi, too, built by a biased constant
+// and a subtraction).  The
 // diagonal column is accumulated like the others and its LCG value taken
 // out afterwards (no compare per element), then d_i x_i is added.
 __global__ void __launch_bounds__(kGemvThreads)
@@ -58,14 +61,13 @@ otf_gemv_kernel(int n, uint64_t s00, Aff jn, const double *__restrict__ d,
     const int64_t r1 = r0 + kGemvThreads;
     const int64_t j_begin = (int64_t)blockIdx.y * cols_per_split;
     const int64_t j_end = imin64(n, j_begin + cols_per_split);
-    constexpr double kHiBias = 0x1p84 + 0x1p63;
     constexpr double kLoBias = 0x1p52;
 
     const Aff inc1 = lcg_inc1();
     // states of (r0, j_begin) and (r1, j_begin)
     uint64_t s0 = aff_apply(aff_pow(inc1, (uint64_t)r0 + (uint64_t)n * (uint64_t)j_begin), s00);
     uint64_t s1 = aff_apply(aff_pow(inc1, (uint64_t)kGemvThreads), s0);
-    double acc0 = 0.0, acc1 = 0.0, bias = 0.0;
+    double acc0 = 0.0, acc1 = 0.0, hi0 = 0.0, hi1 = 0.0, bias = 0.0;
     for (int64_t jc = j_begin; jc < j_end; jc += kGemvXChunk) {
         const int len = (int)imin64(kGemvXChunk, j_end - jc);
         __syncthreads();
@@ -78,10 +80,8 @@ otf_gemv_kernel(int n, uint64_t s00, Aff jn, const double *__restrict__ d,
 #pragma unroll 4
         for (int q = 0; q < len; ++q) {
             const double xq = xs[q];
-            const double h0 = __hiloint2double(0x45300000, (int)((uint32_t)(s0 >> 32) ^ 0x80000000u)) - kHiBias;
-            const double h1 = __hiloint2double(0x45300000, (int)((uint32_t)(s1 >> 32) ^ 0x80000000u)) - kHiBias;
-            acc0 = __fma_rn(h0, xq, acc0);
-            acc1 = __fma_rn(h1, xq, acc1);
+            hi0 = __fma_rn((double)(int)(s0 >> 32), xq, hi0);
+            hi1 = __fma_rn((double)(int)(s1 >> 32), xq, hi1);
             acc0 = __fma_rn(__hiloint2double(0x43300000, (int)(uint32_t)s0), xq, acc0);
             acc1 = __fma_rn(__hiloint2double(0x43300000, (int)(uint32_t)s1), xq, acc1);
             s0 = aff_apply(jn, s0);
@@ -96,8 +96,8 @@ otf_gemv_kernel(int n, uint64_t s00, Aff jn, const double *__restrict__ d,
         __syncthreads();
     }
     bias = bias_red[0];
-    acc0 -= bias;
-    acc1 -= bias;
+    acc0 = __fma_rn(hi0, 0x1p32, acc0 - bias);
+    acc1 = __fma_rn(hi1, 0x1p32, acc1 - bias);
     // diagonal entries come from d (otf_gemv_diag_d, panel_gemv.hpp:26): the
     // LCG value accumulated at (r, r) is taken out, d_r x_r added
     if (r0 < n && r0 >= j_begin && r0 < j_end) {
