@@ -1147,10 +1147,9 @@ extern "C" mxp_status mxp_iterative_refinement(int n, uint64_t seed, const float
     }
     s = launch_infnorm(n, d_rhs, sc + 3, st);
     if (s != MXP_OK) return s;
+    // (read at the first residual's synchronisation)
     MXP_CUDA(cudaMemcpyAsync(h + 2, sc + 2, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    MXP_CUDA(cudaStreamSynchronize(st));
-    if (norma <= 0.0) norma = h[2];
-    const double normb = h[3];
+    double normb = 0.0;
     s = launch_ir_init(n, d_rhs, d_d, d_x, st);
     if (s != MXP_OK) return s;
     const double eps = 0x1p-53;  // DBL_EPSILON / 2
@@ -1159,12 +1158,18 @@ extern "C" mxp_status mxp_iterative_refinement(int n, uint64_t seed, const float
     double normr = -1.0, hpl = -1.0, normx = 0.0;
     int gemv_calls = 0, trsv_calls = 0, inner = 0;
     for (it = 0; it < maxit; ++it) {
-        s = launch_copy(n, d_rhs, r, st);
-        if (s == MXP_OK) s = launch_infnorm(n, d_x, sc + 0, st);
-        cudaEventRecord(g0, st);
-        if (s == MXP_OK) s = residual_gemv(ws, n, seed, d_d, -1.0, d_x, 1.0, r, st);
-        cudaEventRecord(g1, st);
-        if (s == MXP_OK) s = launch_infnorm(n, r, sc + 1, st);
+        if (ws->higham) {
+            s = launch_copy(n, d_rhs, r, st);
+            if (s == MXP_OK) s = launch_infnorm(n, d_x, sc + 0, st);
+            cudaEventRecord(g0, st);
+            if (s == MXP_OK) s = residual_gemv(ws, n, seed, d_d, -1.0, d_x, 1.0, r, st);
+            cudaEventRecord(g1, st);
+            if (s == MXP_OK) s = launch_infnorm(n, r, sc + 1, st);
+        } else {
+            cudaEventRecord(g0, st);
+            s = launch_residual(n, seed, d_d, d_rhs, d_x, r, sc, ws->partials, ws->max_splits, st);
+            cudaEventRecord(g1, st);
+        }
         if (s != MXP_OK) return s;
         ++gemv_calls;
         MXP_CUDA(cudaMemcpyAsync(h, sc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1172,6 +1177,10 @@ extern "C" mxp_status mxp_iterative_refinement(int n, uint64_t seed, const float
         ms_gemv += elapsed(g0, g1);
         if (trsv_pending) ms_trsv += elapsed(t0, t1);
         trsv_pending = false;
+        if (it == 0) {
+            if (norma <= 0.0) norma = h[2];
+            normb = h[3];
+        }
         normx = h[0];
         normr = h[1];
         hpl = normr / (norma * normx + normb) * 1.0 / ((double)n * eps);

@@ -265,6 +265,10 @@ mxp_status launch_schur(int form, int m, int n, int k, const void *L, int64_t ld
 mxp_status launch_otf_gemv(int n, uint64_t seed, const double *d, double alpha, const double *x,
                            double beta, double *y, double *partials, int max_splits,
                            cudaStream_t st);
+// r = b - A x and norms[0] = max |x|, norms[1] = max |r| (device, 2 doubles); partials:
+// max_splits * n doubles.
+mxp_status launch_residual(int n, uint64_t seed, const double *d, const double *b, const double *x, double *r,
+                           double *norms, double *partials, int max_splits, cudaStream_t st);
 // mail: 2 n doubles, tickets: 2 ints of device memory (set on the stream first).
 // withhold >= 0: the forward solve never publishes that row block, so the
 // blocks that need it give up after the bounded wait (tests of MXP_TIMEOUT).

@@ -127,6 +127,34 @@ __global__ void gemv_reduce_kernel(int n, int splits, const double *__restrict__
     y[i] = (beta == 0.0 ? 0.0 : beta * y[i]) + alpha * t;
 }
 
+// The refinement's residual from the split partial sums, r = b - A x, with
+// max |x| and max |r| for the stopping test (norms[0], norms[1]; zero at
+// launch): as a copy, two norms and their clears each a launch or memset of its
+// own, a refinement step of a small system spent ~25 us on them.
+__global__ void residual_reduce_kernel(int n, int splits, const double *__restrict__ partials,
+                                       const double *__restrict__ b, const double *__restrict__ x,
+                                       double *__restrict__ r, unsigned long long *norms) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double mx = 0.0, mr = 0.0;
+    if (i < n) {
+        double t = 0.0;
+        for (int s = 0; s < splits; ++s) t += partials[(int64_t)s * n + i];
+        const double v = b[i] - t;
+        r[i] = v;
+        mx = fmax(mx, fabs(x[i]));
+        mr = fmax(mr, fabs(v));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, o));
+    }
+    if ((threadIdx.x & 31) == 0) {  // (as infnorm_kernel: non-negative doubles order like their bits)
+        atomicMax(norms, (unsigned long long)__double_as_longlong(mx));
+        atomicMax(norms + 1, (unsigned long long)__double_as_longlong(mr));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // sync-free block triangular solves
 // ---------------------------------------------------------------------------
@@ -755,22 +783,25 @@ __global__ void axpy_kernel(int n, double alpha, const double *__restrict__ x, d
 
 }  // namespace
 
-mxp_status launch_otf_gemv(int n, uint64_t seed, const double *d, double alpha, const double *x,
-                           double beta, double *y, double *partials, int max_splits,
-                           cudaStream_t st) {
-    if (n <= 0) return MXP_OK;
-    const int row_blocks = (int)cdiv(n, kGemvRows);
+// How a product of order n is split: row blocks x column splits of `cols` columns.
+static void gemv_grid(int n, int max_splits, int *row_blocks, int *splits, int64_t *cols) {
+    *row_blocks = (int)cdiv(n, kGemvRows);
     // 12 CTAs (48 warps) per SM where the column splits allow: an element is a
     // chain of an LCG step and three FP64 operations, hidden only by other warps
     // (n = 30011: 468 us with 4 CTAs per SM, 457 with 12)
     const int target = 12 * num_sms();
-    int splits = (target + row_blocks - 1) / row_blocks;
-    if (splits > max_splits) splits = max_splits;
-    if (!partials) splits = 1;
-    int64_t cols = cdiv(n, splits);
-    cols = cdiv(cols, 64) * 64;
-    splits = (int)cdiv(n, cols);
-    if (splits < 1) splits = 1;
+    int s = std::min((target + *row_blocks - 1) / *row_blocks, max_splits);
+    *cols = cdiv(cdiv(n, s), 64) * 64;
+    *splits = std::max(1, (int)cdiv(n, *cols));
+}
+
+mxp_status launch_otf_gemv(int n, uint64_t seed, const double *d, double alpha, const double *x,
+                           double beta, double *y, double *partials, int max_splits,
+                           cudaStream_t st) {
+    if (n <= 0) return MXP_OK;
+    int row_blocks, splits;
+    int64_t cols;
+    gemv_grid(n, partials ? max_splits : 1, &row_blocks, &splits, &cols);
     const uint64_t s00 = lcg_stat00(seed);
     const Aff jn = aff_pow(lcg_inc1(), (uint64_t)n);
     dim3 grid((unsigned)row_blocks, (unsigned)splits);
@@ -781,6 +812,24 @@ mxp_status launch_otf_gemv(int n, uint64_t seed, const double *d, double alpha, 
         gemv_reduce_kernel<<<(unsigned)cdiv(n, 256), 256, 0, st>>>(n, splits, partials, alpha, beta, y);
         MXP_LAUNCHED();
     }
+    return MXP_OK;
+}
+
+mxp_status launch_residual(int n, uint64_t seed, const double *d, const double *b, const double *x, double *r,
+                           double *norms, double *partials, int max_splits, cudaStream_t st) {
+    if (n <= 0) return MXP_OK;
+    int row_blocks, splits;
+    int64_t cols;
+    gemv_grid(n, max_splits, &row_blocks, &splits, &cols);
+    const uint64_t s00 = lcg_stat00(seed);
+    const Aff jn = aff_pow(lcg_inc1(), (uint64_t)n);
+    MXP_CUDA(cudaMemsetAsync(norms, 0, 2 * sizeof(double), st));
+    dim3 grid((unsigned)row_blocks, (unsigned)splits);
+    otf_gemv_kernel<<<grid, kGemvThreads, 0, st>>>(n, s00, jn, d, x, cols, 1.0, 0.0, nullptr, partials);
+    MXP_LAUNCHED();
+    residual_reduce_kernel<<<(unsigned)cdiv(n, 256), 256, 0, st>>>(n, splits, partials, b, x, r,
+                                                                   reinterpret_cast<unsigned long long *>(norms));
+    MXP_LAUNCHED();
     return MXP_OK;
 }
 
