@@ -83,6 +83,10 @@ mxp_status launch_sqrt(const double *in, double *out, cudaStream_t st);
 // pass (K = kMaxMerge * b).
 constexpr int kMaxMerge = 4;
 
+// Words of coop_sync that one clear covers: the barrier words of the diagonal kernel (0, 1)
+// to the tile counters (32: split trailing pass, 33 and 34: panel products).
+constexpr int kSyncWords = 35;
+
 struct mxp_workspace {
     int n = 0, b = 0, form = 0, device = 0;
     int64_t ldk = 0;         // K-major panel row stride (elements): kMaxMerge panel slots side by side
@@ -737,7 +741,8 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
         // stream; not beside a trailing pass, whose SMs they would share)
         const int tc = coop_inv && max_grid == 0 ? inv_tc_start(ws, b) : 0;
         mxp_status q = launch_diag_factor(b, Akk, lda, coop_inv ? XU : nullptr, coop_inv ? XL : nullptr, b,
-                                          tmpU, tmpL, ws->coop_sync, ws->status, (int)kk, on, max_grid, tc);
+                                          tmpU, tmpL, ws->coop_sync, ws->status, (int)kk, on, max_grid, tc,
+                                          on == st ? kSyncWords : 2);
         if (q == MXP_OK && tc > 0)
             q = finish_inverses_tc(b, Akk, lda, XU, XL, b, tc, ws->trsm_single ? kFormBf16 : MXP_FORM_BF16X2,
                                    tmpU, tmpL, ws, on);
@@ -811,7 +816,8 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
             tschedu.counter = ws->trsm_ctr + 1;
             const bool counted = !ws->trsm_pair && ws->trsm_counter;
             const SchurSched *ts = counted ? &tsched : nullptr, *tsu = counted ? &tschedu : nullptr;
-            if (q == MXP_OK && counted) {
+            // (cleared with the diagonal kernel's barrier words when that ran on this stream)
+            if (q == MXP_OK && counted && (diag_done || !ws->coop)) {
                 cudaError_t e = cudaMemsetAsync(ws->trsm_ctr, 0, 2 * sizeof(int), st);
                 if (e != cudaSuccess) q = cuda_fail(e, "panel_lu: TRSM tile counters");
             }

@@ -209,7 +209,7 @@ size_t diag_factor_tmp_floats(int n) { return (size_t)n * n / 2 + (size_t)64 * n
 
 mxp_status launch_diag_factor(int n, float *A, int64_t lda, float *XU, float *XL, int64_t ldx,
                               float *tmpU, float *tmpL, unsigned int *sync_words, DevStatus *dst,
-                              int pivot_base, cudaStream_t st, int max_grid, int inv_stop) {
+                              int pivot_base, cudaStream_t st, int max_grid, int inv_stop, int clear_words) {
     if (n <= 0) return MXP_OK;
     if (lda < n || (XU && ldx < n)) return fail(MXP_INVALID_ARG, "diag_factor: bad leading dimension");
     if ((XU == nullptr) != (XL == nullptr)) return fail(MXP_INVALID_ARG, "diag_factor: both inverses or none");
@@ -223,7 +223,7 @@ mxp_status launch_diag_factor(int n, float *A, int64_t lda, float *XU, float *XL
     const int tm = (n + kNB - 1) / kNB;
     int grid = (int)imin64(sms, std::max<int64_t>(2, (int64_t)tm * tm));
     if (max_grid > 0) grid = min(grid, max(2, max_grid));
-    MXP_CUDA(cudaMemsetAsync(sync_words, 0, 2 * sizeof(unsigned int), st));
+    MXP_CUDA(cudaMemsetAsync(sync_words, 0, (size_t)clear_words * sizeof(unsigned int), st));
     Ctl ctl{sync_words, reinterpret_cast<int *>(sync_words + 1), dst};
     void *args[] = {&n, &A, &lda, &XU, &XL, &ldx, &tmpU, &tmpL, &ctl, &pivot_base, &inv_stop};
     MXP_CUDA(cudaLaunchCooperativeKernel((const void *)diag_factor_kernel, dim3(grid), dim3(kCT), args, kCoopSmem, st));
