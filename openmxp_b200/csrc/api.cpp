@@ -983,13 +983,23 @@ static mxp_status residual_gemv(mxp_workspace *ws, int n, uint64_t seed, const d
     return launch_otf_gemv(n, seed, dd, a, x, b, y, ws->partials, ws->max_splits, st);
 }
 
+// Whether the stored inverses solve faster than the chain of 64-row blocks.  A
+// step of theirs (two grid barriers and the product with the block's strip)
+// takes 8 to 11 us whatever b is, the chain 2.6 us for each 64 rows and about
+// 40 us to start, so the inverses win from some b on and, below it, while n is
+// small.  Two solves of a refinement, inverses / chain, us: b = 64, n = 2048:
+// 1021 / 405; b = 128, n = 1024: 292 / 294, n = 2048: 567 / 412, n = 4096:
+// 1078 / 666; b = 256, n = 2048: 312 / 406, n = 8192: 1429 / 1342, n = 24576:
+// 5005 / 3893; b = 512, n = 8192: 798 / 1348, n = 16384: 1770 / 2633.
+static bool inverses_faster(int n, int b) { return b > 256 || (int64_t)n * 8 < (int64_t)b * b; }
+
 // x <- U^{-1} L^{-1} x with the factor LU: by the stored inverses of the
 // diagonal blocks when they belong to this factor (the last mxp_panel_lu on
-// the workspace), else by the chain of 64-row blocks.
+// the workspace) and are the faster way, else by the chain of 64-row blocks.
 static mxp_status lu_solve_ws(mxp_workspace *ws, int n, const float *LU, int64_t lda, double *x,
                               cudaStream_t st, int withhold = -1) {
     if (withhold < 0 && ws->trsv_inv && ws->inv_lu && LU == ws->inv_lu && n == ws->inv_n &&
-        lda == ws->inv_lda && lu_solve_inv_supported(n, ws->b, LU, lda)) {
+        lda == ws->inv_lda && inverses_faster(n, ws->b) && lu_solve_inv_supported(n, ws->b, LU, lda)) {
         const int64_t bb = (int64_t)ws->b * ws->b;
         return launch_lu_solve_inv(n, ws->b, LU, lda, ws->inv_store, ws->inv_store + bb, 2 * bb, x, ws->trsv_t,
                                    ws->coop_sync + 8, ws->status, st);

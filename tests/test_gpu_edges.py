@@ -176,6 +176,26 @@ def test_stored_inverse_solve_edges(mxp, orc, torch_cuda, n, b):
     assert np.max(np.abs(dx.cpu().numpy() - want)) <= 1e-12 * np.max(np.abs(want))
 
 
+@pytest.mark.parametrize("n,b,chain", [(1920, 128, False), (2048, 128, True), (512, 64, True), (8192, 256, True)])
+def test_which_solve_a_factor_takes(mxp, torch_cuda, n, b, chain):
+    """Either side of the line between the stored inverses and the chain: the chain's
+    results are the chain's bits; the inverses' differ and agree to rounding."""
+    torch = torch_cuda
+    p = mxp.panel_matgen(n, 3)
+    ws = mxp.Workspace(n, b, 0)
+    mxp.panel_lu(p, b, ws)
+    x = np.random.default_rng(n).standard_normal(n)
+    got = []
+    for off in (False, True):
+        if off:
+            ws.set_option(mxp.OPT_TRSV_INV, 0)
+        dx = torch.from_numpy(x.copy()).cuda()
+        mxp.lu_solve(p.A, n, n, dx, ws)
+        got.append(dx.cpu().numpy())
+    assert np.array_equal(got[0], got[1]) == chain
+    assert np.max(np.abs(got[0] - got[1])) <= 1e-12 * np.max(np.abs(got[1]))
+
+
 @pytest.mark.parametrize("m,n,k,ldc", [(129, 257, 4096, 132), (300, 260, 4224, 300), (640, 1000, 128, 643),
                                        (4097, 300, 640, 4097), (127, 33, 256, 128)])
 def test_fp8_update_short_and_long_k(mxp, orc, torch_cuda, m, n, k, ldc):
