@@ -112,7 +112,7 @@ typedef enum {
                                    barriers; 0: one launch per 64-column step */
     MXP_OPT_TRSM_PAIR = 7,      /* 1: TRSM-by-inverse products on the 2-SM kernel; 0 (default): 1-SM */
     MXP_OPT_TEST_WITHHOLD_FLAG = 8, /* test of the bounded device waits: the next mxp_lu_solve never
-                                       publishes the completion flag of this 64-row block of the
+                                       publishes the values of this 64-row block of the
                                        forward solve, so the blocks waiting for it give up after
                                        the 2 s bound and the call returns MXP_TIMEOUT (-1: off) */
     MXP_OPT_OVERLAP_DIAG = 9,   /* merged schedule: > 0 factors the diagonal block of the next pair
@@ -142,11 +142,11 @@ typedef enum {
                                    (b > 256, or 8 n < b^2); 0: always the chain of 64-row blocks,
                                    substituting exactly in FP64.  Setting the option forgets
                                    the stored inverses. */
-    MXP_OPT_FP8_FUSED_CAST = 15, /* FP8 form, tensor-core TRSM, b % 256 == 0: 1 (default) the
-                                   TRSM products that form the L and U panels also write their
-                                   E4M3 copies and per-tile scales (the same bytes as the FP8 panel
-                                   casts of the stored FP32 panels, without reading them back);
-                                   0: separate cast launches */
+    MXP_OPT_FP8_FUSED_CAST = 15, /* tensor-core TRSM, b % 256 == 0 (FP8 form) or b % 32 == 0 (FP16,
+                                   BF16X2): 1 (default) the TRSM products that form the L and U
+                                   panels also write their low-precision copies and FP8 scales
+                                   (the same bytes as the panel casts of the stored FP32 panels,
+                                   without reading them back); 0: separate cast launches */
     MXP_OPT_TRSM_COUNTER = 16,  /* 1-SM TRSM-by-inverse products: 1 (default) CTAs claim output
                                    tiles from a device counter (the triangular K-skip makes tile
                                    work uneven); 0: static round robin.  Each tile is computed the

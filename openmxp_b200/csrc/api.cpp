@@ -123,7 +123,7 @@ struct mxp_workspace {
     // tensor-core panel TRSM: FP32 triangular inverses and split-BF16 operands
     int trsm_tc = 1;
     int trsm_single = 0;     // one BF16 product instead of three split products
-    int fp8_fused = 1;       // FP8 form: the L panel's E4M3 copy written by the TRSM product's epilogue
+    int fused_cast = 1;      // the panels' low-precision copies written by the TRSM products' epilogues
     int inv_tc = 1024;       // inverse doubling levels from this block size on the tensor cores (0: none)
     int64_t ldk3 = 0;
     float *tinv_u = nullptr, *tinv_l = nullptr, *tinv_tmp = nullptr;
@@ -356,7 +356,7 @@ extern "C" mxp_status mxp_workspace_set_option(mxp_workspace *ws, int key, int v
             ws->inv_tc = value;
             return MXP_OK;
         case MXP_OPT_FP8_FUSED_CAST:
-            ws->fp8_fused = value ? 1 : 0;
+            ws->fused_cast = value ? 1 : 0;
             return MXP_OK;
         case MXP_OPT_TRSM_COUNTER:
             ws->trsm_counter = value ? 1 : 0;
@@ -771,7 +771,8 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
         float *Akk = d_A + kk + kk * lda;
         const int m = n - (int)kk - b;
         const bool coop_inv = ws->coop && ws->trsm_tc && m > 0;
-        const bool fuse_f8 = fp8 && ws->trsm_tc && ws->fp8_fused && !ws->trsm_pair && b % 256 == 0 && m > 0;
+        // the products also write the panels' low-precision copies
+        const bool fuse = ws->trsm_tc && ws->fused_cast && !ws->trsm_pair && m > 0 && b % (fp8 ? 256 : 32) == 0;
         mxp_status q = MXP_OK;
         if (!diag_done) {
             pt.mark(PH_DIAG);
@@ -803,12 +804,10 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
                                     {1, m, b, Urow, lda, ubuf, ws->ldk3}};
             if (q == MXP_OK) q = launch_casts(bf, ops, own ? 4 : 3, st);
             pt.mark(PH_TGEMM);
-            // FP8 form: the product's epilogue also writes the E4M3 L panel and
-            // its scales into the panel slot (the separate casts below are skipped)
-            F8Out f8{nullptr, 0, nullptr, 0, 0};
-            if (fuse_f8)
-                f8 = F8Out{Lb + (row0 * ldk + slot * kp) * es, ldk,
-                           Ls + (row0 / 128) * scl + slot * (int64_t)cdiv(b, 128), scl, 0};
+            // (the casts below are skipped then)
+            const int64_t doff = row0 * ldk + slot * kp, sof = (row0 / 128) * scl + slot * (int64_t)cdiv(b, 128);
+            const PanelCopy pl{form, Lb + doff * es, ldk, fp8 ? Ls + sof : nullptr, scl, 0, b};
+            const PanelCopy pu{form, Rb + doff * es, ldk, fp8 ? Rs + sof : nullptr, scl, 1, b};
             // The triangular K-skip makes the tiles' work uneven (1 to b/256 K blocks):
             // CTAs claim tiles from a counter instead of a static round robin.
             SchurSched tsched, tschedu;
@@ -826,12 +825,7 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
             if (q == MXP_OK)
                 q = launch_schur(bf, m, b, b, ws->split_big, ws->ldk3, nullptr, ws->split_u, ws->ldk3,
                                  nullptr, Lcol, lda, ws->status, st, /*store=*/1, 0, 0, /*tri=*/1, ws->trsm_pair,
-                                 ts, fuse_f8 ? &f8 : nullptr);
-            // ... and the one that forms U12 the E4M3 R panel (transposed layout)
-            F8Out f8u{nullptr, 0, nullptr, 0, 0};
-            if (fuse_f8)
-                f8u = F8Out{Rb + (row0 * ldk + slot * kp) * es, ldk,
-                            Rs + (row0 / 128) * scl + slot * (int64_t)cdiv(b, 128), scl, 1};
+                                 ts, fuse ? &pl : nullptr);
             if (!own) {
                 pt.mark(PH_CAST);
                 if (q == MXP_OK) q = launch_casts(bf, ops + 3, 1, st);
@@ -840,7 +834,7 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
             if (q == MXP_OK)
                 q = launch_schur(bf, b, m, b, ws->split_l, ws->ldk3, nullptr, ubuf, ws->ldk3,
                                  nullptr, Urow, lda, ws->status, both ? ws->side : st, /*store=*/1, 0, 0, /*tri=*/2,
-                                 ws->trsm_pair, tsu, fuse_f8 ? &f8u : nullptr);
+                                 ws->trsm_pair, tsu, fuse ? &pu : nullptr);
             if (both) {
                 const mxp_status jq = join();
                 if (q == MXP_OK) q = jq;
@@ -849,7 +843,7 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
             q = launch_trsm_runn(m, b, Akk, lda, Lcol, lda, st);
             if (q == MXP_OK) q = launch_trsm_llnu(b, m, Akk, lda, Urow, lda, st);
         }
-        if (q != MXP_OK) return q;
+        if (q != MXP_OK || fuse) return q;
         pt.mark(PH_CAST);
         const int64_t koff = slot * kp;
         const int64_t soff = slot * (int64_t)cdiv(b, 128);
@@ -857,7 +851,7 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
             const CastJob panels[2] = {{0, m, b, Lcol, lda, Lb + (row0 * ldk + koff) * es, ldk},
                                        {1, m, b, Urow, lda, Rb + (row0 * ldk + koff) * es, ldk}};
             q = launch_casts(form, panels, 2, st);
-        } else if (!fuse_f8) {
+        } else {
             q = launch_cast_left(form, m, b, Lcol, lda, Lb + (row0 * ldk + koff) * es, ldk,
                                  Ls + (row0 / 128) * scl + soff, st, scl);
             if (q == MXP_OK)

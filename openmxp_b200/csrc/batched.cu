@@ -7,18 +7,20 @@
 //  * one CTA (256 threads) per SM, each taking whole systems from a ticket in
 //    descending order of size (longest first), so a CTA runs one system's
 //    LU and refinement start to finish with no grid-wide synchronisation;
-//  * per block step of B columns: the B x B diagonal block and the two panel
-//    strips are factored with the SIMT FP32 pieces of dense_tile.cuh (same
-//    algorithm as the single-system path: no-pivot LU, TRSM against the
-//    diagonal triangles, sgetrf_nopiv_naive order); the strips are then cast
-//    to FP16 into a per-CTA staging area laid out as the shared-memory image
-//    of a 128-byte-swizzled K-major tile (16 KB per 128 rows x 64 columns), so
-//    the Schur phase moves each operand tile with one plain bulk copy
-//    (cp.async.bulk, no tensor map) into a ring of shared-memory stages;
+//  * per block step of B columns: the B x B diagonal block with the SIMT FP32
+//    pieces of dense_tile.cuh (no-pivot LU, sgetrf_nopiv_naive order); both panel
+//    strips as independent vectors of length B against a triangle, 16 columns
+//    at a time, the products with the columns to the right on tcgen05 from
+//    exact three-way BF16 splits (strip_tiles); the solved strips are written
+//    once in FP32 and once in FP16, into a per-CTA staging area laid out as the
+//    shared-memory image of a 128-byte-swizzled K-major tile (16 KB per 128
+//    rows x 64 columns), so the Schur phase moves each operand tile with one
+//    plain bulk copy (cp.async.bulk, no tensor map) into a ring of
+//    shared-memory stages;
 //  * the trailing update C -= L R^T runs warp-specialised on the CTA's own
 //    tensor core: warp 0 issues the bulk copies, warp 1 the tcgen05.mma
 //    (M = 128, N = TN, K = 16) into one of two TMEM accumulators, warps 4-7
-//    drain the accumulator and apply it to C in HBM;
+//    request C ahead into shared memory, drain the accumulator and write C back;
 //  * refinement follows iterative_refinement.hpp:141-171 per system: x0 = b/d,
 //    r = b - A x with A regenerated in FP64 from the LCG (otf_gemv), stop at
 //    scaled residual < 16, else x += U^{-1} L^{-1} r (block substitution with

@@ -244,25 +244,31 @@ struct SchurSched {
     int skip_rows = 0, skip_cols = 0;
 };
 
-// Optional FP8 copy of a store-mode product (FP16/BF16 operands, single-SM
-// kernel, n % 256 == 0), with one power-of-two scale per 128 x 128 block of C,
-// exactly as the FP8 panel casts of C would write them.  trans == 0 (L panel
-// layout): out[i * ldk + j] = E4M3(C(i, j) * 2^e), byte 127 - e at
-// sc[(i / 128) * sc_ld + j / 128]; trans == 1 (R panel layout, C holds U
-// columns): out[j * ldk + i], scale at sc[(j / 128) * sc_ld + i / 128].
-struct F8Out {
+// Optional low-precision copy of a store-mode product (FP16/BF16 operands,
+// single-SM kernel) in the operand layout of `form`, the same bytes as the
+// panel casts of C would write.  trans == 0: L panel, C(i, j) goes to row i;
+// trans == 1: R panel (C holds U columns), C(i, j) goes to row j.  ldk in
+// elements of the form.
+//   FP16, BF16X2: m or n (the block size) % 32 == 0, rows 16-byte aligned; k:
+//     distance of the three BF16X2 segments (the block size).
+//   FP8: n % 256 == 0; one power-of-two scale 2^e per 128 x 128 block of C,
+//     byte 127 - e at sc[(i / 128) * sc_ld + j / 128] (trans:
+//     sc[(j / 128) * sc_ld + i / 128]).
+struct PanelCopy {
+    int form;
     uint8_t *out;
     int64_t ldk;
     uint8_t *sc;
     int sc_ld;
     int trans;
+    int k;
 };
 
 mxp_status launch_schur(int form, int m, int n, int k, const void *L, int64_t ldl,
                         const uint8_t *lsc, const void *R, int64_t ldr, const uint8_t *rsc,
                         float *C, int64_t ldc, DevStatus *dst, cudaStream_t st, int store = 0,
                         int lsc_ld = 0, int rsc_ld = 0, int tri_mode = 0, int pair = 0,
-                        const SchurSched *sched = nullptr, const F8Out *f8out = nullptr);
+                        const SchurSched *sched = nullptr, const PanelCopy *copy_out = nullptr);
 
 mxp_status launch_otf_gemv(int n, uint64_t seed, const double *d, double alpha, const double *x,
                            double beta, double *y, double *partials, int max_splits,

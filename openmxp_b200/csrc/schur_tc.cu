@@ -26,6 +26,8 @@
 // as written by the panel-cast kernels.  Out-of-range rows / K columns are
 // zero-filled by TMA; C is masked in the epilogue.
 #include <cudaTypedefs.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <mutex>
 
@@ -152,11 +154,83 @@ __device__ __forceinline__ void ring_init(const TileRing &r) {
     }
 }
 
-template <bool F8>
+// FP16 or BF16X2 copy of a 32-column piece of a store-mode product, from the
+// registers that the FP32 store holds (the bytes of cast_left_tile and
+// cast_right_block).  v: this lane's row.  L panel: a thread writes its row's 32
+// consecutive k.  R panel: the 32 lanes hold 32 consecutive k, so lanes pair up
+// and each writes two k of every other column (16 stores instead of 32).
+// A cast launch of its own reads the panel back (4 bytes for 2 written) and at small
+// blocks costs a launch.  FP16 solves with it / with casts, ms: n = 1024, b = 128
+// 1.365 / 1.42; n = 8192, b = 256 8.40 / 8.82; n = 61440, b = 2560 208.1 / 211.6.
+// BF16X2 writes three times the bytes here: 1.40 / 1.45 at n = 1024, 8.59 / 8.77 at
+// n = 8192, the same time from n = 16384 on.
+__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ float bf16_rest(float x) {
+    return __fsub_rn(x, __bfloat162float(__float2bfloat16_rn(x)));
+}
+
+template <int COPY>
+__device__ __forceinline__ void copy_piece(const PanelCopy &pc, const float (&v)[32], int64_t row, int64_t col0,
+                                           int lane) {
+    uint16_t *out = reinterpret_cast<uint16_t *>(pc.out);
+    if (!pc.trans) {
+        uint16_t *d = out + row * pc.ldk + col0;
+#pragma unroll
+        for (int q = 0; q < 32; q += 8) {
+            if (COPY == MXP_FORM_FP16) {
+                *reinterpret_cast<uint4 *>(d + q) =
+                    make_uint4(pack_f16(v[q], v[q + 1]), pack_f16(v[q + 2], v[q + 3]), pack_f16(v[q + 4], v[q + 5]),
+                               pack_f16(v[q + 6], v[q + 7]));
+            } else {
+                const uint4 hi = make_uint4(pack_bf16(v[q], v[q + 1]), pack_bf16(v[q + 2], v[q + 3]),
+                                            pack_bf16(v[q + 4], v[q + 5]), pack_bf16(v[q + 6], v[q + 7]));
+                *reinterpret_cast<uint4 *>(d + q) = hi;
+                *reinterpret_cast<uint4 *>(d + pc.k + q) = hi;
+                *reinterpret_cast<uint4 *>(d + 2 * pc.k + q) =
+                    make_uint4(pack_bf16(bf16_rest(v[q]), bf16_rest(v[q + 1])),
+                               pack_bf16(bf16_rest(v[q + 2]), bf16_rest(v[q + 3])),
+                               pack_bf16(bf16_rest(v[q + 4]), bf16_rest(v[q + 5])),
+                               pack_bf16(bf16_rest(v[q + 6]), bf16_rest(v[q + 7])));
+            }
+        }
+    } else {
+        const int odd = lane & 1;
+        uint16_t *d = out + (col0 + odd) * pc.ldk + (row - odd);
+        const uint32_t sel = odd ? 0x3276u : 0x5410u;  // (row - 1, row) of column j + 1 / (row, row + 1) of j
+        auto pair = [&](uint32_t mine) {
+            return __byte_perm(mine, __shfl_xor_sync(0xffffffffu, mine, 1), sel);
+        };
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+            uint16_t *dj = d + j * pc.ldk;
+            if (COPY == MXP_FORM_FP16) {
+                *reinterpret_cast<uint32_t *>(dj) = pair(pack_f16(v[j], v[j + 1]));
+            } else {
+                const uint32_t hi = pair(pack_bf16(v[j], v[j + 1]));
+                *reinterpret_cast<uint32_t *>(dj) = hi;
+                *reinterpret_cast<uint32_t *>(dj + pc.k) = pair(pack_bf16(bf16_rest(v[j]), bf16_rest(v[j + 1])));
+                *reinterpret_cast<uint32_t *>(dj + 2 * pc.k) = hi;
+            }
+        }
+    }
+}
+
+constexpr int kNoCopy = -1;
+
+// COPY: kNoCopy, or the form of the low-precision copy that store mode also writes.
+template <int COPY>
 __global__ void __launch_bounds__(kThreads, 1)
 schur_tc_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     int M, int N, int K, float *__restrict__ C, int64_t ldc, uint32_t idesc,
-                    TileMap tiles, TileSrc src, int store, int tri_mode, int seg, F8Out f8, DevStatus *dst) {
+                    TileMap tiles, TileSrc src, int store, int tri_mode, int seg, PanelCopy pc, DevStatus *dst) {
+    constexpr bool F8 = COPY == MXP_FORM_FP8;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                 ~uintptr_t(1023));
@@ -371,6 +445,11 @@ schur_tc_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
                             if (j < ncol) __stcs(cp + j * ldc, sg * __uint_as_float(r[j]));
+                        if ((COPY == MXP_FORM_FP16 || COPY == MXP_FORM_BF16X2) && ncol > 0) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) cv[j] = sg * __uint_as_float(r[j]);
+                            copy_piece<COPY>(pc, cv, row, col0, lane);
+                        }
                         if (F8) {
 #pragma unroll
                             for (int j = 0; j < 32; ++j) rmax = fmaxf(rmax, fabsf(sg * __uint_as_float(r[j])));
@@ -411,14 +490,14 @@ schur_tc_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 for (int c0 = col_half * 128; c0 < col_half * 128 + 128; c0 += 32) {
                     uint32_t r[32];
                     tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * kBN + c0, r);
-                    if (row_ok && f8.trans) {
+                    if (row_ok && pc.trans) {
                         // R layout: row j of the panel holds its k contiguously, so for
                         // each column j the 32 lanes (32 consecutive k) store one
                         // 32-byte run
-                        uint8_t *dp = f8.out + ((int64_t)tn * kBN + c0) * f8.ldk + row;
+                        uint8_t *dp = pc.out + ((int64_t)tn * kBN + c0) * pc.ldk + row;
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            dp[j * f8.ldk] = to_e4m3(__fmul_rn(sg * __uint_as_float(r[j]), up));
+                            dp[j * pc.ldk] = to_e4m3(__fmul_rn(sg * __uint_as_float(r[j]), up));
                     } else if (row_ok) {
                         uint32_t w[8];
 #pragma unroll
@@ -429,14 +508,14 @@ schur_tc_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                 v |= (uint32_t)to_e4m3(__fmul_rn(sg * __uint_as_float(r[4 * q + b4]), up)) << (8 * b4);
                             w[q] = v;
                         }
-                        uint4 *dp = reinterpret_cast<uint4 *>(f8.out + row * f8.ldk + (int64_t)tn * kBN + c0);
+                        uint4 *dp = reinterpret_cast<uint4 *>(pc.out + row * pc.ldk + (int64_t)tn * kBN + c0);
                         dp[0] = make_uint4(w[0], w[1], w[2], w[3]);
                         dp[1] = make_uint4(w[4], w[5], w[6], w[7]);
                     }
                 }
                 if (lane == 0 && quarter == 0) {
-                    if (f8.trans) f8.sc[(int64_t)(2 * tn + col_half) * f8.sc_ld + tm] = (uint8_t)(127 - e);
-                    else f8.sc[(int64_t)tm * f8.sc_ld + 2 * tn + col_half] = (uint8_t)(127 - e);
+                    if (pc.trans) pc.sc[(int64_t)(2 * tn + col_half) * pc.sc_ld + tm] = (uint8_t)(127 - e);
+                    else pc.sc[(int64_t)tm * pc.sc_ld + 2 * tn + col_half] = (uint8_t)(127 - e);
                 }
             }
             tc_fence_before();
@@ -965,9 +1044,9 @@ mxp_status launch_schur(int form, int m, int n, int k, const void *L, int64_t ld
                         const uint8_t *lsc, const void *R, int64_t ldr, const uint8_t *rsc,
                         float *C, int64_t ldc, DevStatus *dst, cudaStream_t st, int store,
                         int lsc_ld, int rsc_ld, int tri_mode, int pair, const SchurSched *sched,
-                        const F8Out *f8out) {
+                        const PanelCopy *copy_out) {
     if (pair) {
-        if (f8out && f8out->out) return fail(MXP_UNSUPPORTED, "schur: the FP8 copy is single-SM only");
+        if (copy_out && copy_out->out) return fail(MXP_UNSUPPORTED, "schur: the FP8 copy is single-SM only");
         if (sched) return fail(MXP_UNSUPPORTED, "schur: tile schedules are single-SM only");
         return launch_schur2(form, m, n, k, L, ldl, lsc, R, ldr, rsc, C, ldc, dst, st, store, lsc_ld,
                              rsc_ld, tri_mode);
@@ -1030,30 +1109,30 @@ mxp_status launch_schur(int form, int m, int n, int k, const void *L, int64_t ld
     if (s != MXP_OK) return s;
     s = make_kmajor_map(&mapB, dt, 2, R, K, n, ldr, 64, kBN);
     if (s != MXP_OK) return s;
-    static bool attr_done = false;
-    if (!attr_done) {
-        MXP_CUDA(cudaFuncSetAttribute(schur_tc_f16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kSmemBytes));
-        MXP_CUDA(cudaFuncSetAttribute(schur_tc_f16_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kSmemBytes));
-        attr_done = true;
-    }
     const uint32_t idesc = idesc_f16(form == MXP_FORM_FP16 ? 0u : 1u);
     // the triangular skip needs whole stages inside one K segment
     if (tri_mode != 0 && (k % 64 != 0)) tri_mode = 0;
-    F8Out f8{nullptr, 0, nullptr, 0, 0};
-    if (f8out && f8out->out) {
-        if (!store || n % kBN != 0 || !f8out->sc ||
-            (!f8out->trans && (f8out->ldk % 16 != 0 || (reinterpret_cast<uintptr_t>(f8out->out) & 15u))))
-            return fail(MXP_INVALID_ARG, "schur: FP8 copy needs store mode, n % 256 == 0 and 16-byte rows");
-        f8 = *f8out;
+    PanelCopy pc{kNoCopy, nullptr, 0, nullptr, 0, 0, 0};
+    if (copy_out && copy_out->out) {
+        pc = *copy_out;
+        if (!store) return fail(MXP_INVALID_ARG, "schur: a low-precision copy needs store mode");
+        const bool aligned = pc.ldk % 16 == 0 && (reinterpret_cast<uintptr_t>(pc.out) & 15u) == 0;
+        if (pc.form == MXP_FORM_FP8 ? n % kBN != 0 || !pc.sc || (!pc.trans && !aligned)
+                                    : m % 32 != 0 || n % 32 != 0 || pc.k % 32 != 0 || !aligned)
+            return fail(MXP_INVALID_ARG, "schur: shape or alignment of the low-precision copy not supported");
     }
-    if (f8.out)
-        schur_tc_f16_kernel<true><<<grid, kThreads, kSmemBytes, st>>>(mapA, mapB, m, n, (int)K, C, ldc, idesc,
-                                                                      tiles, src, store, tri_mode, k, f8, dst);
-    else
-        schur_tc_f16_kernel<false><<<grid, kThreads, kSmemBytes, st>>>(mapA, mapB, m, n, (int)K, C, ldc, idesc,
-                                                                       tiles, src, store, tri_mode, k, f8, dst);
+    auto kernel = pc.form == MXP_FORM_FP8     ? schur_tc_f16_kernel<MXP_FORM_FP8>
+                  : pc.form == MXP_FORM_FP16   ? schur_tc_f16_kernel<MXP_FORM_FP16>
+                  : pc.form == MXP_FORM_BF16X2 ? schur_tc_f16_kernel<MXP_FORM_BF16X2>
+                                               : schur_tc_f16_kernel<kNoCopy>;
+    static bool attr_done[4] = {};
+    const int which = pc.form - kNoCopy;
+    if (!attr_done[which]) {
+        MXP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        attr_done[which] = true;
+    }
+    kernel<<<grid, kThreads, kSmemBytes, st>>>(mapA, mapB, m, n, (int)K, C, ldc, idesc, tiles, src, store, tri_mode, k,
+                                               pc, dst);
     MXP_LAUNCHED();
     return MXP_OK;
 }

@@ -176,6 +176,22 @@ def test_stored_inverse_solve_edges(mxp, orc, torch_cuda, n, b):
     assert np.max(np.abs(dx.cpu().numpy() - want)) <= 1e-12 * np.max(np.abs(want))
 
 
+@pytest.mark.parametrize("n,b,form", [(192, 32, 0), (480, 96, 0), (640, 160, 1), (1280, 128, 0), (2000, 200, 0),
+                                      (2304, 256, 1), (3200, 640, 0)])
+def test_panel_copies_written_by_the_products(mxp, torch_cuda, n, b, form):
+    """The FP16 and BF16X2 copies of the panels from the products' epilogues are the
+    casts of the stored panels: the same factors bit for bit (b = 200: not that way)."""
+    got = []
+    for fused in (1, 0):
+        p = mxp.panel_matgen(n, 9)
+        ws = mxp.Workspace(n, b, form)
+        ws.set_option(mxp.OPT_FP8_FUSED_CAST, fused)
+        mxp.panel_lu(p, b, ws)
+        got.append(p.A.cpu().numpy())
+        ws.close()
+    assert np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("n,b,chain", [(1920, 128, False), (2048, 128, True), (512, 64, True), (8192, 256, True)])
 def test_which_solve_a_factor_takes(mxp, torch_cuda, n, b, chain):
     """Either side of the line between the stored inverses and the chain: the chain's
