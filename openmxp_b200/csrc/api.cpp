@@ -673,11 +673,14 @@ struct PhaseTimer {
         cudaEventRecord(e, st);
         marks.push_back({e, phase});
     }
-    // returns ms per phase id
+    // returns ms per phase id.  Called while the stream still works: each interval is
+    // read as soon as its end is reached, so the reads (about 1 us each, some 200 for 32
+    // panels) run beside the factorisation instead of after it.
     void collect(double *ms, int nphase) {
         for (int i = 0; i < nphase; ++i) ms[i] = 0.0;
         for (size_t i = 0; i + 1 < marks.size(); ++i) {
             float t = 0.f;
+            cudaEventSynchronize(marks[i + 1].first);
             cudaEventElapsedTime(&t, marks[i].first, marks[i + 1].first);
             const int ph = marks[i].second;
             if (ph >= 0 && ph < nphase) ms[ph] += t;
@@ -950,6 +953,8 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
         return s;
     }
     DevStatus h;
+    double ms[6];
+    if (stats) pt.collect(ms, 6);
     mxp_status rs = read_status(ws, st, &h);
     if (rs == MXP_OK && keep_inv) {
         ws->inv_lu = d_A;
@@ -957,8 +962,6 @@ extern "C" mxp_status mxp_panel_lu(int n, int b, float *d_A, int64_t lda, mxp_wo
         ws->inv_lda = lda;
     }
     if (stats) {
-        double ms[6];
-        pt.collect(ms, 6);
         stats->ms_diag_lu = ms[PH_DIAG];
         stats->ms_trsm = ms[PH_TRSM] + ms[PH_TINV] + ms[PH_TGEMM];
         stats->ms_trsm_inv = ms[PH_TINV];
