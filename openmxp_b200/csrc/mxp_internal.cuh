@@ -49,6 +49,10 @@ __device__ __forceinline__ void report(DevStatus *st, int code, int i0, int i1) 
     }
 }
 
+// The larger of two values, NaN when either is (fmax drops a NaN: the norm of a
+// vector of NaN would be 0, and a refinement would take it for a solution).
+__device__ __forceinline__ double max_nan(double a, double b) { return a > b || a != a ? a : b; }
+
 // Bounded waits give up after this many nanoseconds of %globaltimer.
 constexpr unsigned long long kWaitTimeoutNs = 2000000000ull;
 

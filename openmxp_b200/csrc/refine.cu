@@ -141,15 +141,15 @@ __global__ void residual_reduce_kernel(int n, int splits, const double *__restri
         for (int s = 0; s < splits; ++s) t += partials[(int64_t)s * n + i];
         const double v = b[i] - t;
         r[i] = v;
-        mx = fmax(mx, fabs(x[i]));
-        mr = fmax(mr, fabs(v));
+        mx = max_nan(mx, fabs(x[i]));
+        mr = max_nan(mr, fabs(v));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, o));
+        mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mr = max_nan(mr, __shfl_xor_sync(0xffffffffu, mr, o));
     }
-    if ((threadIdx.x & 31) == 0) {  // (as infnorm_kernel: non-negative doubles order like their bits)
+    if ((threadIdx.x & 31) == 0) {  // (as infnorm_kernel: values without a sign order like their bits)
         atomicMax(norms, (unsigned long long)__double_as_longlong(mx));
         atomicMax(norms + 1, (unsigned long long)__double_as_longlong(mr));
     }
@@ -735,15 +735,15 @@ __global__ void infnorm_kernel(int n, const double *__restrict__ x, unsigned lon
     double m = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-        m = fmax(m, fabs(x[i]));
+        m = max_nan(m, fabs(x[i]));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
     __shared__ double red[32];
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-        // non-negative doubles order like their bit patterns; NaN sorts high
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = max_nan(m, red[w]);
+        // values without a sign order like their bit patterns, NaN above infinity
         atomicMax(out, (unsigned long long)__double_as_longlong(m));
     }
 }
@@ -753,14 +753,14 @@ __global__ void norma_kernel(int n, const double *__restrict__ d, const double *
     double m = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-        m = fmax(m, rs ? rs[i] + d[i] : 2.0 * d[i]);
+        m = max_nan(m, rs ? rs[i] + d[i] : 2.0 * d[i]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
     __shared__ double red[32];
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = max_nan(m, red[w]);
         atomicMax(out, (unsigned long long)__double_as_longlong(m));
     }
 }
