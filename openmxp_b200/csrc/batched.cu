@@ -689,13 +689,13 @@ __device__ bool schur_step(const Ring &rg, RoleState &rs, volatile int *abort_fl
 // ---- per-system refinement (whole CTA) -----------------------------------------
 __device__ double block_max(double v, double *red) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = max_nan(v, __shfl_xor_sync(0xffffffffu, v, o));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     double m = red[0];
 #pragma unroll
-    for (int w = 1; w < kBatchThreads / 32; ++w) m = fmax(m, red[w]);
+    for (int w = 1; w < kBatchThreads / 32; ++w) m = max_nan(m, red[w]);
     return m;
 }
 
@@ -901,8 +901,8 @@ __device__ void refine_system(int n, uint64_t seed, const float *A, const double
                               BatchOut *out) {
     double mb = 0.0, md = 0.0;
     for (int i = threadIdx.x; i < n; i += kBatchThreads) {
-        mb = fmax(mb, fabs(b[i]));
-        md = fmax(md, d[i]);
+        mb = max_nan(mb, fabs(b[i]));
+        md = max_nan(md, d[i]);
         xs[i] = b[i] / d[i];
     }
     const double normb = block_max(mb, red);
@@ -915,8 +915,8 @@ __device__ void refine_system(int n, uint64_t seed, const float *A, const double
         otf_residual(n, seed, d, b, xs, rs);
         double mr = 0.0, mx = 0.0;
         for (int i = threadIdx.x; i < n; i += kBatchThreads) {
-            mr = fmax(mr, fabs(rs[i]));
-            mx = fmax(mx, fabs(xs[i]));
+            mr = max_nan(mr, fabs(rs[i]));
+            mx = max_nan(mx, fabs(xs[i]));
         }
         normr = block_max(mr, red);
         const double normx = block_max(mx, red);

@@ -46,3 +46,23 @@ def test_refinement_with_nan_in_the_right_hand_side(mxp, torch_cuda, higham):
     p.rhs[100] = float("nan")
     x, st, status = mxp.iterative_refinement(p, ws, raise_on_fail=False)
     assert status == mxp.NONFINITE and st["converged"] == 0
+
+
+@pytest.mark.parametrize("where", ["matrix", "rhs", "d"])
+def test_batch_system_with_nan(mxp, torch_cuda, where):
+    """The system that holds the NaN is not converged (and its pivots are reported
+    when the matrix holds it); the others are solved."""
+    bt = mxp.Batch([256, 384, 128], [4, 5, 6])
+    bt.set_config(64, 128, 3)
+    bt.matgen()
+    if where == "matrix":
+        bt.matrix(1)[3, 200] = float("nan")
+    else:
+        bt.vec(getattr(bt, where), 1)[7] = float("nan")
+    bt.solve()
+    got = bt.results()
+    assert got[1]["converged"] == 0 and math.isnan(got[1]["hpl_harness"])
+    assert (got[1]["info"] > 0) == (where == "matrix")
+    for i in (0, 2):
+        assert got[i]["converged"] == 1 and got[i]["hpl_harness"] < 16.0 and got[i]["info"] == 0
+    bt.close()
