@@ -768,8 +768,9 @@ __device__ void otf_residual(int n, uint64_t seed, const double *__restrict__ d,
 // [i_begin, i_end): a thread takes four consecutive rows and reads the block
 // column with 16-byte loads (sixteen in flight), instead of one row at a time
 // with 4-byte loads; each row's sum is the same.  Its own register allocation
-// (the persistent kernel around it is at the register limit).
-__device__ __noinline__ void block_column_update(const float *__restrict__ LU, int64_t lda, int c0, double *r,
+// (the persistent kernel around it is at the register limit).  The factors were
+// written by this kernel: read through L2, never by the read-only path.
+__device__ __noinline__ void block_column_update(const float *LU, int64_t lda, int c0, double *r,
                                                  int i_begin, int i_end) {
     const bool vec = ((reinterpret_cast<uintptr_t>(LU) & 15) == 0) && (lda & 3) == 0 && (i_begin & 3) == 0;
     if (vec) {
@@ -778,7 +779,7 @@ __device__ __noinline__ void block_column_update(const float *__restrict__ LU, i
                 double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
 #pragma unroll 16
                 for (int k = 0; k < kNB; ++k) {
-                    const float4 v = __ldg(reinterpret_cast<const float4 *>(LU + (int64_t)(c0 + k) * lda + i));
+                    const float4 v = __ldcg(reinterpret_cast<const float4 *>(LU + (int64_t)(c0 + k) * lda + i));
                     const double rk = r[c0 + k];
                     a0 = __fma_rn((double)v.x, rk, a0);
                     a1 = __fma_rn((double)v.y, rk, a1);
@@ -792,7 +793,7 @@ __device__ __noinline__ void block_column_update(const float *__restrict__ LU, i
             } else {
                 for (int e = i; e < i_end; ++e) {
                     double acc = 0.0;
-                    for (int k = 0; k < kNB; ++k) acc = __fma_rn((double)__ldg(LU + (int64_t)(c0 + k) * lda + e), r[c0 + k], acc);
+                    for (int k = 0; k < kNB; ++k) acc = __fma_rn((double)__ldcg(LU + (int64_t)(c0 + k) * lda + e), r[c0 + k], acc);
                     r[e] -= acc;
                 }
             }
@@ -801,7 +802,7 @@ __device__ __noinline__ void block_column_update(const float *__restrict__ LU, i
         for (int i = i_begin + threadIdx.x; i < i_end; i += kBatchThreads) {
             double acc = 0.0;
 #pragma unroll 16
-            for (int k = 0; k < kNB; ++k) acc = __fma_rn((double)__ldg(LU + (int64_t)(c0 + k) * lda + i), r[c0 + k], acc);
+            for (int k = 0; k < kNB; ++k) acc = __fma_rn((double)__ldcg(LU + (int64_t)(c0 + k) * lda + i), r[c0 + k], acc);
             r[i] -= acc;
         }
     }
@@ -849,7 +850,7 @@ __device__ __forceinline__ void diag_solve64(const float (*tri)[kTriPitch], cons
 
 // tri: two 64 x 64 blocks: the next diagonal block arrives under the current one's
 // column update.
-__device__ void lu_solve_shared(int n, const float *__restrict__ LU, double *r, float (*tri)[kNB][kTriPitch],
+__device__ void lu_solve_shared(int n, const float *LU, double *r, float (*tri)[kNB][kTriPitch],
                                 double *rd) {
     const int64_t lda = n;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
