@@ -174,7 +174,8 @@ static int64_t panel_ldk(int b, int form) {
 
 // Second copy of a panel's product operand, so that both panels are cast in one
 // launch and their products can run side by side: kept for panels up to this
-// size (a launch does not matter beside the work of larger ones).
+// size (a launch does not matter beside the work of larger ones), and where
+// device memory allows.
 constexpr size_t kSecondPanelMax = (size_t)192 << 20;
 static size_t second_panel_bytes(int64_t rows, int64_t ldk3) {
     return std::min((size_t)rows * ldk3 * 2, kSecondPanelMax);
@@ -285,6 +286,12 @@ extern "C" mxp_status mxp_workspace_create(int n, int b, int form, int device, m
         return at;
     };
     bool ok = cudaMalloc(&ws->slab, lay_out(nullptr)) == cudaSuccess;
+    if (!ok && ws->big2_bytes > 0) {
+        // the second panel copy saves a launch per panel: a workspace fits without it
+        cudaGetLastError();
+        ws->big2_bytes = 0;
+        ok = cudaMalloc(&ws->slab, lay_out(nullptr)) == cudaSuccess;
+    }
     if (ok) {
         lay_out(static_cast<char *>(ws->slab));
         ws->tile_ctr = reinterpret_cast<int *>(ws->coop_sync + 32);

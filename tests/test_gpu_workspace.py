@@ -26,3 +26,31 @@ def test_one_allocation(mxp, torch_cuda, n, b, form):
     # the estimate a caller plans with holds the whole (buffers start on 256-byte boundaries)
     assert got.pop()[1] <= mxp.Workspace.bytes(n, b, form) + (2 << 20) + 32 * 256
     ws.close()
+
+
+def test_memory_short_of_the_second_panel_copy(mxp, torch_cuda):
+    """A workspace needs no second copy of the panel operands: where the device has room
+    for all but that, it is created without, the U panel is cast into the L panel's
+    buffer after the first product, and the factors are the same bits."""
+    torch = torch_cuda
+    n, b = 12288, 2048
+    second = (n - b) * 3 * b * 2  # rows x split-BF16 operand, below the copy's own limit
+    p = mxp.panel_matgen(n, 9)
+    ws = mxp.Workspace(n, b, 0)
+    mxp.panel_lu(p, b, ws)
+    want = p.A.cpu()
+    ws.close()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    room = mxp.Workspace.bytes(n, b, 0) - second // 2
+    fill = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+    ws = mxp.Workspace(n, b, 0)
+    base, size = _allocation_of(ws.panel_view(0)["data"])
+    assert size < mxp.Workspace.bytes(n, b, 0) - second // 2
+    del fill
+    torch.cuda.empty_cache()
+    mxp.regenerate(p)
+    mxp.panel_lu(p, b, ws)
+    assert torch.equal(p.A.cpu(), want)
+    ws.close()
