@@ -139,9 +139,9 @@ typedef enum {
                                    of bandwidth-bound products with them (each diagonal block:
                                    product with its inverse, then one refinement step against
                                    the factor block, in FP64) where that is the faster way
-                                   (b > 256, or 8 n < b^2); 0: always the chain of 64-row blocks,
-                                   substituting exactly in FP64.  Setting the option forgets
-                                   the stored inverses. */
+                                   (b >= 340, or n (340 - b) < 1700 b); 0: always the chain of
+                                   64-row blocks, substituting exactly in FP64.  Setting the
+                                   option forgets the stored inverses. */
     MXP_OPT_FP8_FUSED_CAST = 15, /* tensor-core TRSM, b % 256 == 0 (FP8 form) or b % 32 == 0 (FP16,
                                    BF16X2): 1 (default) the TRSM products that form the L and U
                                    panels also write their low-precision copies and FP8 scales
@@ -347,9 +347,9 @@ mxp_status mxp_workspace_set_matrix_higham(mxp_workspace *ws, double alpha, doub
 /* trsvL_h + trsvU_h (panel_trsv.hpp:308-597): x <- U^{-1} L^{-1} x with
  * the FP32 factors of mxp_panel_lu, vectors in FP64, block substitution.
  * When d_LU, n and lda are those of the last successful mxp_panel_lu on this
- * workspace (and MXP_OPT_TRSV_INV is on, and b > 256 or 8 n < b^2), the diagonal
- * blocks are solved with the inverses that LU kept (a product, then one
- * refinement step against the factor block); a factor written into that buffer by other means must be
+ * workspace (and MXP_OPT_TRSV_INV is on, and b >= 340 or n (340 - b) < 1700 b), the
+ * diagonal blocks are solved with the inverses that LU kept (a product, then
+ * one refinement step against the factor block); a factor written into that buffer by other means must be
  * solved after MXP_OPT_TRSV_INV is set again (setting it, to either value,
  * forgets the stored inverses) or from another buffer.  Otherwise 64-row
  * blocks substitute exactly in FP64 along a chain.  Blocking: reads the

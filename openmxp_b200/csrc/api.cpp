@@ -995,15 +995,19 @@ static mxp_status residual_gemv(mxp_workspace *ws, int n, uint64_t seed, const d
     return launch_otf_gemv(n, seed, dd, a, x, b, y, ws->partials, ws->max_splits, st);
 }
 
-// Whether the stored inverses solve faster than the chain of 64-row blocks.  A
-// step of theirs (two grid barriers and the product with the block's strip)
-// takes 8 to 11 us whatever b is, the chain 2.6 us for each 64 rows and about
-// 40 us to start, so the inverses win from some b on and, below it, while n is
-// small.  Two solves of a refinement, inverses / chain, us: b = 64, n = 2048:
-// 1021 / 405; b = 128, n = 1024: 292 / 294, n = 2048: 567 / 412, n = 4096:
-// 1078 / 666; b = 256, n = 2048: 312 / 406, n = 8192: 1429 / 1342, n = 24576:
-// 5005 / 3893; b = 512, n = 8192: 798 / 1348, n = 16384: 1770 / 2633.
-static bool inverses_faster(int n, int b) { return b > 256 || (int64_t)n * 8 < (int64_t)b * b; }
+// Whether the stored inverses solve faster than the chain of 64-row blocks.  Both
+// triangles of a block step of theirs (four grid barriers each, and the products)
+// take ~16.5 us at small n whatever b is, after 36 us; the chain takes 107 us and
+// 0.0575 us a row, so the inverses win while n (287 - b) < 1235 b.  From n ~ 6000 on
+// the factor leaves the L2 cache and either way slows down (16 to 35 us a step, 0.07
+// to 0.1 us a row): the constants below put the line through the measured crossings,
+// b: n = 64: ~390, 96: ~720, 128: ~1050, 160: ~1480, 192: ~2150, 256: ~6100,
+// 320: ~20000 (the rule: 394, 669, 1026, 1511, 2205, 5181, 27200; b = 384: none up to
+// 49152).  Inverses / chain, us per solve of both triangles: b = 64, n = 512: 154 /
+// 133; b = 128, n = 1024: 167 / 169, n = 1920: 284 / 215; b = 192, n = 1536: 173 / 193,
+// n = 4032: 410 / 339; b = 256, n = 4096: 325 / 342, n = 8192: 719 / 692, n = 24576:
+// 2478 / 1970; b = 512, n = 8192: 414 / 690, n = 49152: 3768 / 4787.
+static bool inverses_faster(int n, int b) { return b >= 340 || (int64_t)n * (340 - b) < (int64_t)1700 * b; }
 
 // x <- U^{-1} L^{-1} x with the factor LU: by the stored inverses of the
 // diagonal blocks when they belong to this factor (the last mxp_panel_lu on

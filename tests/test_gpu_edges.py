@@ -192,7 +192,9 @@ def test_panel_copies_written_by_the_products(mxp, torch_cuda, n, b, form):
     assert np.array_equal(got[0], got[1])
 
 
-@pytest.mark.parametrize("n,b,chain", [(1920, 128, False), (2048, 128, True), (512, 64, True), (8192, 256, True)])
+@pytest.mark.parametrize("n,b,chain", [(1024, 128, False), (1152, 128, True), (1920, 128, True), (384, 64, False), (512, 64, True),
+                                       (2112, 192, False), (2304, 192, True), (5120, 256, False), (8192, 256, True),
+                                       (3200, 320, False), (28160, 320, True), (2048, 512, False)])
 def test_which_solve_a_factor_takes(mxp, torch_cuda, n, b, chain):
     """Either side of the line between the stored inverses and the chain: the chain's
     results are the chain's bits; the inverses' differ and agree to rounding."""
