@@ -368,6 +368,20 @@ mxp_status launch_sgemm_sub(int m, int n, int k, const float *A, int64_t lda, co
     return MXP_OK;
 }
 
+mxp_status launch_trsm_runn_small(int m, int nb, const float *U, int64_t ldu, float *B, int64_t ldb,
+                                  cudaStream_t st) {
+    trsm_runn_small_kernel<<<(unsigned)cdiv(m, 128), 128, 0, st>>>(m, nb, U, ldu, B, ldb);
+    MXP_LAUNCHED();
+    return MXP_OK;
+}
+
+mxp_status launch_trsm_llnu_small(int nb, int n, const float *L, int64_t ldl, float *B, int64_t ldb,
+                                  cudaStream_t st) {
+    trsm_llnu_small_kernel<<<(unsigned)cdiv(n, 64), 256, 0, st>>>(n, nb, L, ldl, B, ldb);
+    MXP_LAUNCHED();
+    return MXP_OK;
+}
+
 mxp_status launch_getrf_blocked(int n, float *A, int64_t lda, DevStatus *dst, int pivot_base,
                                 cudaStream_t st) {
     if (n <= 0) return MXP_OK;
@@ -379,14 +393,11 @@ mxp_status launch_getrf_blocked(int n, float *A, int64_t lda, DevStatus *dst, in
         MXP_LAUNCHED();
         const int rem = n - jb - nbk;
         if (rem <= 0) continue;
-        trsm_runn_small_kernel<<<(unsigned)cdiv(rem, 128), 128, 0, st>>>(rem, nbk, Ajj, lda,
-                                                                         Ajj + nbk, lda);
-        MXP_LAUNCHED();
-        trsm_llnu_small_kernel<<<(unsigned)cdiv(rem, 64), 256, 0, st>>>(
-            rem, nbk, Ajj, lda, Ajj + (int64_t)nbk * lda, lda);
-        MXP_LAUNCHED();
-        mxp_status s = launch_sgemm_sub(rem, rem, nbk, Ajj + nbk, lda, Ajj + (int64_t)nbk * lda,
-                                        lda, Ajj + nbk + (int64_t)nbk * lda, lda, st);
+        mxp_status s = launch_trsm_runn_small(rem, nbk, Ajj, lda, Ajj + nbk, lda, st);
+        if (s == MXP_OK) s = launch_trsm_llnu_small(nbk, rem, Ajj, lda, Ajj + (int64_t)nbk * lda, lda, st);
+        if (s != MXP_OK) return s;
+        s = launch_sgemm_sub(rem, rem, nbk, Ajj + nbk, lda, Ajj + (int64_t)nbk * lda, lda,
+                             Ajj + nbk + (int64_t)nbk * lda, lda, st);
         if (s != MXP_OK) return s;
     }
     return MXP_OK;

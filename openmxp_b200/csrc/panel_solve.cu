@@ -231,6 +231,26 @@ int panel_slice(int64_t m) {
     return (int)std::min<int64_t>(kSlice, cdiv(cdiv(m, sms * waves), 4) * 4);
 }
 
+// Narrow triangles against many rows.  The CTAs of the panel kernels hold a slice
+// of whole panels, one to an SM, so from the second wave on (9472 rows) nothing
+// hides a slice's loads, and a narrow triangle gives them little else to do.
+// A thread per row (64 columns at a time, an SGEMM between) is then the better
+// way, up to a width that grows with the waves; us, thread per row / slices:
+// 32 wide 9500 rows 6.8 / 9.4, 60000 12.9 / 32.1; 64 wide 9500 11.6 / 9.8, 20000
+// 12.5 / 13.9, 60000 22.7 / 35.0; 80 wide 20000 38.7 / 30.4; 96 wide 20000 39.2 /
+// 30.5, 30000 41.7 / 45.2, 60000 76.5 / 79.9; 112 wide 40000 68.7 / 53.3, 60000
+// 82.4 / 80.9.
+bool rows_by_thread(int64_t m, int n) {
+    const int64_t waves = cdiv(m, (int64_t)num_sms() * kSlice);
+    return waves > 1 && n <= (waves == 2 ? 48 : waves == 3 ? 64 : 96);
+}
+
+// The same for the columns of the left solve, a warp per column: only for triangles of
+// at most 16 (8 high 9500 columns 5.9 / 8.2 us, 60000 13.7 / 26.7; 16 high 9500 7.9 /
+// 8.0, 60000 22.1 / 26.8; 32 high 9500 12.2 / 8.2), and for as few columns as
+// each get a warp soon (16 high, 16 columns 2.8 / 3.8; 200 columns 7.3 / 4.1).
+bool cols_by_warp(int m, int64_t n) { return m <= 16 && (n <= 32 || n > (int64_t)num_sms() * kSlice); }
+
 }  // namespace
 
 mxp_status launch_trsm_runn(int m, int n, const float *U, int64_t ldu, float *B, int64_t ldb,
@@ -239,15 +259,22 @@ mxp_status launch_trsm_runn(int m, int n, const float *U, int64_t ldu, float *B,
     if (ldu < n || ldb < m) return fail(MXP_INVALID_ARG, "trsm_right_upper: bad leading dimension");
     MXP_CUDA(cudaFuncSetAttribute(panel_right_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemRight)));
     const int slice = panel_slice(m);
-    for (int j = 0; j < n; j += kPanN) {
-        const int w = std::min(kPanN, n - j), rem = n - j - w;
+    const bool narrow = rows_by_thread(m, n);
+    const int step = narrow ? kNB : kPanN;
+    for (int j = 0; j < n; j += step) {
+        const int w = std::min(step, n - j), rem = n - j - w;
+        const float *Uj = U + (int64_t)j * (ldu + 1);
         float *Bj = B + (int64_t)j * ldb;
-        panel_right_kernel<<<(unsigned)cdiv(m, slice), kCT, sizeof(SmemRight), st>>>(m, w, slice, U + (int64_t)j * (ldu + 1),
-                                                                                     ldu, Bj, ldb);
-        MXP_LAUNCHED();
+        mxp_status s = MXP_OK;
+        if (narrow) {
+            s = launch_trsm_runn_small(m, w, Uj, ldu, Bj, ldb, st);
+        } else {
+            panel_right_kernel<<<(unsigned)cdiv(m, slice), kCT, sizeof(SmemRight), st>>>(m, w, slice, Uj, ldu, Bj, ldb);
+            MXP_LAUNCHED();
+        }
+        if (s != MXP_OK) return s;
         if (rem <= 0) break;
-        mxp_status s = launch_sgemm_sub(m, rem, w, Bj, ldb, U + j + (int64_t)(j + w) * ldu, ldu, Bj + (int64_t)w * ldb,
-                                        ldb, st);
+        s = launch_sgemm_sub(m, rem, w, Bj, ldb, U + j + (int64_t)(j + w) * ldu, ldu, Bj + (int64_t)w * ldb, ldb, st);
         if (s != MXP_OK) return s;
     }
     return MXP_OK;
@@ -257,6 +284,7 @@ mxp_status launch_trsm_llnu(int m, int n, const float *L, int64_t ldl, float *B,
                             cudaStream_t st) {
     if (m <= 0 || n <= 0) return MXP_OK;
     if (ldl < m || ldb < m) return fail(MXP_INVALID_ARG, "trsm_left_lower_unit: bad leading dimension");
+    if (cols_by_warp(m, n)) return launch_trsm_llnu_small(m, n, L, ldl, B, ldb, st);
     MXP_CUDA(cudaFuncSetAttribute(panel_left_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemLeft)));
     const int slice = panel_slice(n);
     for (int j = 0; j < m; j += kPanN) {

@@ -80,6 +80,21 @@ def test_panel_solves_against_64_bits(mxp, orc, torch_cuda, m, n, pad):
     assert rel_fro(to_np_colmajor(dL, n, m, n + pad), want.numpy()) < tol
 
 
+@pytest.mark.parametrize("m,n,pad", [(9472, 48, 0), (9473, 48, 1), (9473, 49, 0), (18945, 64, 0), (18945, 65, 0),
+                                     (28417, 65, 3), (28417, 96, 0), (28417, 97, 0)])
+def test_right_solves_of_narrow_triangles(mxp, orc, torch_cuda, m, n, pad):
+    """Either side of the line between slices and a thread per row; a triangle of more
+    than 64 columns goes there in two steps.  Tolerance as above."""
+    test_panel_solves_against_64_bits(mxp, orc, torch_cuda, m, n, pad)
+
+
+@pytest.mark.parametrize("columns,n,pad", [(32, 16, 1), (33, 16, 0), (32, 17, 0), (9472, 16, 0), (9473, 16, 3),
+                                           (9473, 17, 0)])
+def test_left_solves_of_narrow_triangles(mxp, orc, torch_cuda, columns, n, pad):
+    """The same for the left solve: a warp per column, or slices."""
+    test_panel_solves_against_64_bits(mxp, orc, torch_cuda, columns, n, pad)
+
+
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 65, 96, 127, 130, 191, 321])
 @pytest.mark.parametrize("pad", [0, 1])
 def test_diagonal_block_edges(mxp, orc, torch_cuda, n, pad):
