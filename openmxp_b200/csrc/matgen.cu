@@ -188,13 +188,12 @@ gen_batch_kernel(const GenSys *sys, int count, float *A, double *d, double *rhs)
     }
 }
 
-template <typename T, int ROWS>
-mxp_status launch_gen_rows(const GenArgs<T> &g, cudaStream_t st) {
-    const size_t smem = gen_smem<T, ROWS>();
-    MXP_CUDA(cudaFuncSetAttribute(gen_kernel<T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gen_kernel<T, ROWS><<<(unsigned)cdiv(g.n, ROWS), kGenThreads, smem, st>>>(g);
-    MXP_LAUNCHED();
-    return MXP_OK;
+// The right-hand side by itself (stream column n), a thread per row: in the kernel
+// above its eight rows per CTA cost a CTA's jump powers each (n = 20000: 17 us, here
+// 3).
+__global__ void __launch_bounds__(256) rhs_kernel(int n, uint64_t s00, double *rhs) {
+    const int64_t row = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (row < n) rhs[row] = lcg_to_double(aff_apply(aff_pow(lcg_inc1(), (uint64_t)row + (uint64_t)n * (uint64_t)n), s00));
 }
 
 template <typename T>
@@ -211,7 +210,15 @@ mxp_status launch_gen(int n, uint64_t seed, int diag_rule, T *A, int64_t lda, do
     g.d = d;
     g.rowsum = rowsum;
     g.rhs = rhs;
-    return launch_gen_rows<T, kGenRows>(g, st);
+    if (!A && !d && !rowsum) {
+        rhs_kernel<<<(unsigned)cdiv(n, 256), 256, 0, st>>>(n, g.s00, rhs);
+    } else {
+        constexpr size_t smem = gen_smem<T, kGenRows>();
+        static_assert(smem <= 48 * 1024, "no function attribute needed");
+        gen_kernel<T, kGenRows><<<(unsigned)cdiv(n, kGenRows), kGenThreads, smem, st>>>(g);
+    }
+    MXP_LAUNCHED();
+    return MXP_OK;
 }
 
 }  // namespace
@@ -229,8 +236,7 @@ mxp_status launch_matgen_batch(int count, const GenSys *sys, int nmax, float *A,
                                cudaStream_t st) {
     if (count <= 0) return MXP_OK;
     const dim3 grid((unsigned)cdiv(nmax, kGenRows), (unsigned)std::min(count, 65535));
-    const size_t smem = gen_smem<float, kGenRows>();
-    MXP_CUDA(cudaFuncSetAttribute(gen_batch_kernel<kGenRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t smem = gen_smem<float, kGenRows>();
     gen_batch_kernel<kGenRows><<<grid, kGenThreads, smem, st>>>(sys, count, A, d, rhs);
     MXP_LAUNCHED();
     return MXP_OK;

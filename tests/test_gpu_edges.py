@@ -41,6 +41,17 @@ def test_generation_of_single_outputs(mxp, orc, torch_cuda):
         assert np.array_equal(out[k].cpu().numpy().view(np.uint64), want.view(np.uint64))
 
 
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 5000, 20011])
+def test_right_hand_side_alone(mxp, orc, torch_cuda, n):
+    """The right-hand side by itself is the one of the whole system."""
+    torch = torch_cuda
+    rhs = torch.full((n + 1,), -2.0, dtype=torch.float64, device="cuda")
+    mxp.check(mxp.lib().mxp_matgen(n, 11, 0, None, n, None, None, rhs.data_ptr(), None))
+    _, _, _, want = orc.matgen(n, 11, with_matrix=False)
+    assert np.array_equal(rhs[:n].cpu().numpy().view(np.uint64), want.view(np.uint64))
+    assert float(rhs[n]) == -2.0
+
+
 def test_batch_generation_is_the_systems(mxp, orc, torch_cuda):
     sizes = [128, 640, 256, 1152]
     bt = mxp.Batch(sizes, [5, 6, 7, 8])
