@@ -160,7 +160,7 @@ __device__ __forceinline__ void gen_rows(const GenArgs<T> &g, int64_t row0) {
 }
 
 template <typename T, int ROWS>
-__global__ void __launch_bounds__(kGenThreads, 2) gen_kernel(GenArgs<T> g) {
+__global__ void __launch_bounds__(kGenThreads, ROWS > kGenRows ? 1 : 2) gen_kernel(GenArgs<T> g) {
     gen_rows<T, ROWS>(g, (int64_t)blockIdx.x * ROWS);
 }
 
@@ -196,6 +196,16 @@ __global__ void __launch_bounds__(256) rhs_kernel(int n, uint64_t s00, double *r
     if (row < n) rhs[row] = lcg_to_double(aff_apply(aff_pow(lcg_inc1(), (uint64_t)row + (uint64_t)n * (uint64_t)n), s00));
 }
 
+template <typename T, int ROWS>
+mxp_status launch_gen_rows(const GenArgs<T> &g, cudaStream_t st) {
+    constexpr size_t smem = gen_smem<T, ROWS>();
+    if (smem > 48 * 1024 - 1024)
+        MXP_CUDA(cudaFuncSetAttribute(gen_kernel<T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gen_kernel<T, ROWS><<<(unsigned)cdiv(g.n, ROWS), kGenThreads, smem, st>>>(g);
+    MXP_LAUNCHED();
+    return MXP_OK;
+}
+
 template <typename T>
 mxp_status launch_gen(int n, uint64_t seed, int diag_rule, T *A, int64_t lda, double *d, double *rowsum,
                       double *rhs, cudaStream_t st) {
@@ -212,13 +222,16 @@ mxp_status launch_gen(int n, uint64_t seed, int diag_rule, T *A, int64_t lda, do
     g.rhs = rhs;
     if (!A && !d && !rowsum) {
         rhs_kernel<<<(unsigned)cdiv(n, 256), 256, 0, st>>>(n, g.s00, rhs);
-    } else {
-        constexpr size_t smem = gen_smem<T, kGenRows>();
-        static_assert(smem <= 48 * 1024, "no function attribute needed");
-        gen_kernel<T, kGenRows><<<(unsigned)cdiv(n, kGenRows), kGenThreads, smem, st>>>(g);
+        MXP_LAUNCHED();
+        return MXP_OK;
     }
-    MXP_LAUNCHED();
-    return MXP_OK;
+    // FP64 columns that do not all start on a sector (an odd pitch): a CTA's 64 bytes
+    // of a column then touch three sectors, two of them shared with the neighbours'.
+    // Twice the rows (one CTA per SM) make that five for 128: n = 8191 178 us (8
+    // rows 296), n = 8192 with a pitch of 8193 168 (271).
+    if (sizeof(T) == 8 && A && ((reinterpret_cast<uintptr_t>(A) | (uintptr_t)(lda * sizeof(T))) & 31))
+        return launch_gen_rows<T, 2 * kGenRows>(g, st);
+    return launch_gen_rows<T, kGenRows>(g, st);
 }
 
 }  // namespace

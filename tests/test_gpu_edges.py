@@ -23,6 +23,20 @@ def test_generation_rows_and_columns(mxp, orc, torch_cuda, n, pad):
         assert np.array_equal(got.cpu().numpy().view(np.uint64), want.view(np.uint64))
 
 
+@pytest.mark.parametrize("n,pad,shift", [(1, 0, 0), (15, 1, 0), (16, 1, 1), (17, 0, 0), (33, 2, 0), (256, 0, 1),
+                                         (512, 0, 0), (513, 2, 1), (1031, 0, 0)])
+def test_f64_generation_rows_and_pitches(mxp, orc, torch_cuda, n, pad, shift):
+    """8 or 16 rows per CTA by the columns' alignment; nothing past the rows."""
+    torch = torch_cuda
+    ld = n + pad
+    buf = torch.full((n * ld + shift + 2,), -3.0, dtype=torch.float64, device="cuda")
+    mxp.matgen_f64(n, 42, A=buf[shift:], lda=ld)
+    _, d, _, _ = orc.matgen(n, 42, with_matrix=False)
+    got = buf[shift:shift + n * ld].view(n, ld)
+    assert np.array_equal(got[:, :n].t().cpu().numpy().view(np.uint64), orc.matgen_f64(n, 42, d).view(np.uint64))
+    assert torch.all(got[:, n:] == -3.0) and torch.all(buf[:shift] == -3.0) and torch.all(buf[shift + n * ld:] == -3.0)
+
+
 def test_generation_of_single_outputs(mxp, orc, torch_cuda):
     """Any output may be skipped (NULL)."""
     torch = torch_cuda
