@@ -170,22 +170,26 @@ __device__ __forceinline__ void cast_right_block(int64_t blk, int m, int b, cons
 // Up to four casts of one form in one launch, side by side: a panel step casts
 // both panels and both inverses before its two products and both panels
 // after them, and for small blocks a launch costs more than its work.
+// A single cast (N = 1) has no job to look for and a quarter of the parameters.
+struct CastBlocks {
+    CastJob c;
+    bool vec, vec_in;
+    unsigned gx, blocks;  // left: tiles along the rows; blocks of the job
+};
+template <int N>
 struct CastJobs {
     int count;
-    struct Job {
-        CastJob c;
-        bool vec, vec_in;
-        unsigned gx, blocks;  // left: tiles along the rows; blocks of the job
-    } job[kMaxCastJobs];
+    CastBlocks job[N];
 };
 
-template <int FORM>
-__global__ void __launch_bounds__(kCastThreads) cast_jobs_kernel(const __grid_constant__ CastJobs jobs) {
+template <int FORM, int N>
+__global__ void __launch_bounds__(kCastThreads) cast_jobs_kernel(const __grid_constant__ CastJobs<N> jobs) {
     __shared__ float tile[kTile][kTile + 1];
     unsigned blk = blockIdx.x;
     int q = 0;
-    while (q + 1 < jobs.count && blk >= jobs.job[q].blocks) blk -= jobs.job[q++].blocks;
-    const CastJobs::Job &j = jobs.job[q];
+    if constexpr (N > 1)
+        while (q + 1 < jobs.count && blk >= jobs.job[q].blocks) blk -= jobs.job[q++].blocks;
+    const CastBlocks &j = jobs.job[q];
     if (j.c.right)
         cast_right_block<FORM>(blk, j.c.m, j.c.b, j.c.A, j.c.lda, j.c.out, j.c.ldk, j.vec, j.vec_in);
     else
@@ -366,9 +370,16 @@ static mxp_status check_cast_args(int form, int m, int b, int64_t lda, int64_t l
     return MXP_OK;
 }
 
+template <int N>
+static void launch_cast_jobs(int form, const CastJobs<N> &js, unsigned blocks, cudaStream_t st) {
+    if (form == MXP_FORM_FP16) cast_jobs_kernel<MXP_FORM_FP16, N><<<blocks, kCastThreads, 0, st>>>(js);
+    else if (form == kFormBf16) cast_jobs_kernel<kFormBf16, N><<<blocks, kCastThreads, 0, st>>>(js);
+    else cast_jobs_kernel<MXP_FORM_BF16X2, N><<<blocks, kCastThreads, 0, st>>>(js);
+}
+
 mxp_status launch_casts(int form, const CastJob *jobs, int count, cudaStream_t st) {
     if (form == MXP_FORM_FP8) return fail(MXP_UNSUPPORTED, "panel casts: FP8 panels are cast one by one");
-    CastJobs js;
+    CastJobs<kMaxCastJobs> js;
     js.count = 0;
     int64_t total = 0;
     for (int q = 0; q < count; ++q) {
@@ -376,7 +387,7 @@ mxp_status launch_casts(int form, const CastJob *jobs, int count, cudaStream_t s
         mxp_status s = check_cast_args(form, c.m, c.b, c.lda, c.ldk);
         if (s != MXP_OK) return s;
         if (c.m == 0) continue;
-        CastJobs::Job &j = js.job[js.count++];
+        CastBlocks &j = js.job[js.count++];
         j.c = c;
         j.vec = vec_ok(c.out, c.ldk, c.b);
         j.vec_in = (reinterpret_cast<uintptr_t>(c.A) % 16 == 0) && (c.lda % 4 == 0);
@@ -388,9 +399,8 @@ mxp_status launch_casts(int form, const CastJob *jobs, int count, cudaStream_t s
         j.blocks = (unsigned)blocks;
     }
     if (js.count == 0) return MXP_OK;
-    if (form == MXP_FORM_FP16) cast_jobs_kernel<MXP_FORM_FP16><<<(unsigned)total, kCastThreads, 0, st>>>(js);
-    else if (form == kFormBf16) cast_jobs_kernel<kFormBf16><<<(unsigned)total, kCastThreads, 0, st>>>(js);
-    else cast_jobs_kernel<MXP_FORM_BF16X2><<<(unsigned)total, kCastThreads, 0, st>>>(js);
+    if (js.count == 1) launch_cast_jobs(form, CastJobs<1>{1, {js.job[0]}}, (unsigned)total, st);
+    else launch_cast_jobs(form, js, (unsigned)total, st);
     MXP_LAUNCHED();
     return MXP_OK;
 }
