@@ -589,15 +589,24 @@ constexpr int kF8StageSF = 2048;  // SFA 512 B + SFB 1024 B, padded
 constexpr int kF8StageBytes = kF8StageA + kF8StageB + kF8StageSF;
 // Two forms.  Long K: four operand stages, C loaded by the epilogue into
 // registers (16 columns at a time: 16 KB in flight per SM, hidden by the
-// products).  Short K (kF8ShortK): the C read-modify-write bounds a tile (256 KB
-// against 128 KB of operands at K = 512), so one stage gives way to C: every
+// products).  Short K (up to kF8ShortK): the C read-modify-write bounds a tile
+// (256 KB against 192 KB of operands at K = 512), so one stage gives way to C: every
 // epilogue warp requests its 32 rows' next two 32-column pieces by cp.async
 // (64 KB in flight per SM), across tiles, while it stores the ones before.
+// Where the line lies, long / short, us, the first pass over a C that is not in
+// L2: 5003 x 4001, pitch 5004: K = 128 89 / 54, 640 88 / 56, 1024 89 / 57, 2048 90 /
+// 80; pitch 5006 (4-byte copies): 640 88 / 66, 1024 90 / 68, 2048 93 / 83; 12000 x
+// 12000: 512 403 / 253, 1024 406 / 248, 1536 413 / 320, 2048 420 / 387; 1500 x 1300:
+// 640 30 / 24 (over the same C again the ratios are the same or larger).  Update
+// phase of whole factorisations, ms: n = 18432, b = 384 (trailing K = 1536) 5.60 /
+// 4.21, n = 32768, b = 512 (K = 2048) 20.0 / 17.2, n = 61440, b = 2560 (K = 10240,
+// in a group 2560) 66.5 / 68.4, n = 32768, b = 1024 (K = 4096, in a group 1024): short
+// up to 1024 12.1, for all 12.9.
 constexpr int kF8StagesLong = 4, kF8StagesShort = 3;
 constexpr int kF8CStage = 2 * 32 * 32 * 4 * kEpiWarps;  // two pieces of 32 x 32 per epilogue warp
 constexpr int kF8SmemLong = 1024 + kF8StagesLong * kF8StageBytes + 512;
 constexpr int kF8SmemShort = 1024 + kF8StagesShort * kF8StageBytes + kF8CStage + 512;
-constexpr int kF8ShortK = 1024;
+constexpr int kF8ShortK = 2048;
 constexpr int kF8SfCol0 = 256;
 // Stages whose scale factors share one TMEM copy: a tile's scale is uniform
 // over its 128 x 128 block, so the four K blocks of a stage use one byte of

@@ -255,7 +255,8 @@ def test_which_solve_a_factor_takes(mxp, torch_cuda, n, b, chain):
 
 
 @pytest.mark.parametrize("m,n,k,ldc", [(129, 257, 4096, 132), (300, 260, 4224, 300), (640, 1000, 128, 643),
-                                       (4097, 300, 640, 4097), (127, 33, 256, 128)])
+                                       (4097, 300, 640, 4097), (127, 33, 256, 128), (257, 300, 2048, 260),
+                                       (300, 260, 2176, 301)])
 def test_fp8_update_short_and_long_k(mxp, orc, torch_cuda, m, n, k, ldc):
     """Both forms of the FP8 kernel, C with 16-byte and with scalar addresses.  FP32
     accumulation in another order: 1e-5 of the sum of the terms' sizes."""
