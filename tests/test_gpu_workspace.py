@@ -54,3 +54,26 @@ def test_memory_short_of_the_second_panel_copy(mxp, torch_cuda):
     mxp.panel_lu(p, b, ws)
     assert torch.equal(p.A.cpu(), want)
     ws.close()
+
+
+@pytest.mark.parametrize("form,tol", [(0, 1e-6), (2, 1e-4)])
+def test_panels_too_large_for_the_second_copy(mxp, torch_cuda, form, tol):
+    """A first panel of 10752 x 3584 (231 MB as split BF16) against 192 MB of second copy: its
+    U panel goes through the L panel's buffer, the later panels' through their own.
+    Factors against a 64-bit elimination of the same matrix: the forms' own rounding
+    of the panels, relative to the dominant diagonal, is 2e-7 (FP16) and 2e-5 (FP8)."""
+    torch = torch_cuda
+    n, b = 14336, 3584
+    p = mxp.panel_matgen(n, 9)
+    want, _ = torch.linalg.lu_factor(p.matrix().double(), pivot=False)
+    ws = mxp.Workspace(n, b, form)
+    mxp.panel_lu(p, b, ws)
+    got = p.matrix().double()
+    for part in (torch.tril, torch.triu):
+        err = torch.linalg.norm(part(got) - part(want)) / torch.linalg.norm(want)
+        assert float(err) < tol
+    # the panels of the first step by themselves: the U strip, and the L strip (its
+    # entries are smaller by the pivot)
+    for sl in ((slice(0, b), slice(b, n)), (slice(b, n), slice(0, b))):
+        assert float(torch.linalg.norm(got[sl] - want[sl]) / torch.linalg.norm(want[sl])) < 1e-4
+    ws.close()
