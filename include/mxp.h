@@ -140,8 +140,9 @@ typedef enum {
                                    product with its inverse, then one refinement step against
                                    the factor block, in FP64) where that is the faster way
                                    (b >= 340, or n (340 - b) < 1700 b); 0: always the chain of
-                                   64-row blocks, substituting exactly in FP64.  Setting the
-                                   option forgets the stored inverses. */
+                                   64-row blocks, each applying the FP64 inverse of its 64 x 64
+                                   diagonal block as a product.  Setting the option forgets the
+                                   stored inverses. */
     MXP_OPT_FP8_FUSED_CAST = 15, /* tensor-core TRSM, b % 256 == 0 (FP8 form) or b % 32 == 0 (FP16,
                                    BF16X2): 1 (default) the TRSM products that form the L and U
                                    panels also write their low-precision copies and FP8 scales
@@ -349,10 +350,11 @@ mxp_status mxp_workspace_set_matrix_higham(mxp_workspace *ws, double alpha, doub
  * When d_LU, n and lda are those of the last successful mxp_panel_lu on this
  * workspace (and MXP_OPT_TRSV_INV is on, and b >= 340 or n (340 - b) < 1700 b), the
  * diagonal blocks are solved with the inverses that LU kept (a product, then
- * one refinement step against the factor block); a factor written into that buffer by other means must be
- * solved after MXP_OPT_TRSV_INV is set again (setting it, to either value,
- * forgets the stored inverses) or from another buffer.  Otherwise 64-row
- * blocks substitute exactly in FP64 along a chain.  Blocking: reads the
+ * one refinement step against the factor block); a factor written into that
+ * buffer by other means must be solved after MXP_OPT_TRSV_INV is set again
+ * (setting it, to either value, forgets the stored inverses) or from another
+ * buffer.  Otherwise 64-row blocks run along a chain, each 64 x 64 diagonal
+ * block inverted in FP64 and applied as a product.  Blocking: reads the
  * workspace status word (MXP_TIMEOUT when a bounded wait between row blocks
  * gave up). */
 mxp_status mxp_lu_solve(int n, const float *d_LU, int64_t lda, double *d_x, mxp_workspace *ws,

@@ -666,8 +666,7 @@ extern "C" mxp_status mxp_schur_update(int form, int m, int n, int k, const void
 // ---------------------------------------------------------------------------
 namespace {
 // Phase marks on the solve stream, from the workspace's event pool (no event
-// is created once the pool has grown to a solve's number of marks); read
-// after the LU's final synchronisation.
+// is created once the pool has grown to a solve's number of marks).
 struct PhaseTimer {
     bool on = false;
     cudaStream_t st = 0;

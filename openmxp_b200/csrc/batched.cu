@@ -265,8 +265,9 @@ struct StripState {  // barrier positions, carried across tiles, steps and syste
     uint32_t mma_phase = 0, nb = 0;  // nb: W loads of the group so far
 };
 
-// x split into three BF16 terms: x = t0 + t1 + t2 exactly (24 bits), each term's
-// bits in the low half.
+// x split into three BF16 terms: x = t0 + t1 + t2 exactly (24 bits) for 2^-110 <= |x| <
+// 2^127 (below, the last terms meet BF16's smallest subnormal; infinity gives
+// NaN), each term's bits in the low half.
 __device__ __forceinline__ void split3(float x, uint32_t (&t)[3]) {
 #pragma unroll
     for (int p = 0; p < 3; ++p) {

@@ -211,7 +211,7 @@ mxp_status launch_tri_inv_upper(int n, const float *U, int64_t ldu, float *X, in
                                 float *tmp, cudaStream_t st);
 mxp_status launch_tri_inv_lower_unit(int n, const float *L, int64_t ldl, float *X, int64_t ldx,
                                      float *tmp, cudaStream_t st);
-// The same for a triangle of at most 64, a thread per row and a warp per column of B.
+// The panel solves of a triangle of at most 64: a thread per row, a warp per column of B.
 mxp_status launch_trsm_runn_small(int m, int nb, const float *U, int64_t ldu, float *B, int64_t ldb,
                                   cudaStream_t st);
 mxp_status launch_trsm_llnu_small(int nb, int n, const float *L, int64_t ldl, float *B, int64_t ldb,

@@ -953,7 +953,7 @@ schur_tc_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 __syncwarp();
                 tc_fence_after();
                 uint32_t r[4][32];
-    #pragma unroll
+#pragma unroll
                 for (int c = 0; c < 4; ++c)
                     tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + col_half * 128 + 32 * c, r[c]);
                 tc_fence_before();
@@ -961,23 +961,23 @@ schur_tc_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (lane == 0) mbar_arrive(smem_u32(tempty));  // accumulator free: next tile may start
                 const int64_t row = (int64_t)tm * kBM + quarter * 32 + lane;
                 if (row < M) {
-    #pragma unroll
+#pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const int64_t col0 = (int64_t)tn * kF8BN + col_half * 128 + 32 * c;
                         const int ncol = (int)imin64(32, (int64_t)N - col0);
                         float *cp = C + col0 * ldc + row;
                         if (ncol >= 32) {
-    #pragma unroll
+#pragma unroll
                             for (int h = 0; h < 2; ++h) {
                                 float cv[16];
-    #pragma unroll
+#pragma unroll
                                 for (int j = 0; j < 16; ++j) cv[j] = __ldcs(cp + (16 * h + j) * ldc);
-    #pragma unroll
+#pragma unroll
                                 for (int j = 0; j < 16; ++j)
                                     __stcs(cp + (16 * h + j) * ldc, cv[j] - __uint_as_float(r[c][16 * h + j]));
                             }
                         } else {
-    #pragma unroll
+#pragma unroll
                             for (int j = 0; j < 32; ++j)
                                 if (j < ncol) cp[j * ldc] = cp[j * ldc] - __uint_as_float(r[c][j]);
                         }
@@ -1055,7 +1055,7 @@ mxp_status launch_schur(int form, int m, int n, int k, const void *L, int64_t ld
                         int lsc_ld, int rsc_ld, int tri_mode, int pair, const SchurSched *sched,
                         const PanelCopy *copy_out) {
     if (pair) {
-        if (copy_out && copy_out->out) return fail(MXP_UNSUPPORTED, "schur: the FP8 copy is single-SM only");
+        if (copy_out && copy_out->out) return fail(MXP_UNSUPPORTED, "schur: panel copies are written by the single-SM kernel only");
         if (sched) return fail(MXP_UNSUPPORTED, "schur: tile schedules are single-SM only");
         return launch_schur2(form, m, n, k, L, ldl, lsc, R, ldr, rsc, C, ldc, dst, st, store, lsc_ld,
                              rsc_ld, tri_mode);
